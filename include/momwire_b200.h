@@ -354,8 +354,8 @@ size_t mw_getrf_workspace_size(int64_t n);
  * In-place LU with partial pivoting of a complex128 column-major matrix,
  * P A = L U, pivots 1-based as LAPACK zgetrf (ipiv device, length n).
  * Replaces LAPACK zgetrf inside scipy.linalg.solve (bspline.py:2979).
- * `info` (device, 1 int32) receives LAPACK's info (0, or j+1 for an exact
- * zero pivot U(j,j)).  `cancel` (host-mapped or device int32, may be NULL)
+ * `info` (device, 2 int32): info[0] receives LAPACK's info (0, or j+1 for an
+ * exact zero pivot U(j,j)), info[1] a device wait's timeout.  `cancel` (host-mapped or device int32, may be NULL)
  * is polled between panels; a raised flag returns MW_ERR_CANCELLED.
  */
 mw_status mw_zgetrf(int64_t n, double* A, int64_t lda, int32_t* ipiv,
@@ -369,6 +369,29 @@ mw_status mw_zgetrf(int64_t n, double* A, int64_t lda, int32_t* ipiv,
  */
 mw_status mw_zgetrs(int64_t n, int64_t nrhs, const double* LU, int64_t lda,
                     const int32_t* ipiv, double* B, int64_t ldb, void* stream);
+
+/*
+ * Factor A and solve A X = B in one call (LAPACK zgesv): A overwritten by
+ * its factors, ipiv and info as mw_zgetrf (info: 2 int32, info[1] a device
+ * wait's MW_ERR_TIMEOUT, else 0), B (n x nrhs, leading dimension ldb) by X.
+ * The right-hand sides ride through the factorisation, so only the back
+ * substitution follows it.  Workspace: mw_getrf_workspace_size(n).
+ */
+mw_status mw_zgesv(int64_t n, int64_t nrhs, double* A, int64_t lda, int32_t* ipiv, int32_t* info,
+                   double* B, int64_t ldb, void* workspace, size_t workspace_bytes,
+                   const volatile int32_t* cancel, void* stream);
+
+/*
+ * mw_zgesv on `batch` systems of one order: matrix b at A + 2 b a_stride,
+ * its right-hand sides at B + 2 b b_stride (strides in complex elements),
+ * its pivots at ipiv + b n, its two status words at info + 2 b.  Replaces
+ * the stacked numpy.linalg.solve of a swept solve (bspline.py:4181-4440).
+ * Workspace: mw_getrf_workspace_size(n).
+ */
+mw_status mw_zgesv_batched(int64_t n, int64_t nrhs, int32_t batch, double* A, int64_t lda, int64_t a_stride,
+                           int32_t* ipiv, int32_t* info, double* B, int64_t ldb, int64_t b_stride,
+                           void* workspace, size_t workspace_bytes, const volatile int32_t* cancel,
+                           void* stream);
 
 /*
  * complex64 LU with partial pivoting (same conventions as mw_zgetrf),

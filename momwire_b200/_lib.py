@@ -176,6 +176,8 @@ _SIGS = {
     "mw_getrf_workspace_size": (sz, [i64]),
     "mw_zgetrf": (i32, [i64, vp, i64, vp, vp, vp, sz, vp, vp]),
     "mw_zgetrs": (i32, [i64, i64, vp, i64, vp, vp, i64, vp]),
+    "mw_zgesv": (i32, [i64, i64, vp, i64, vp, vp, vp, i64, vp, sz, vp, vp]),
+    "mw_zgesv_batched": (i32, [i64, i64, i32, vp, i64, i64, vp, vp, vp, i64, i64, vp, sz, vp, vp]),
     "mw_scatter_c128": (i32, [i64, i64, i64, vp, vp, vp, vp, vp]),
     "mw_add_loading": (i32, [i64, i32, i64, vp, vp, vp, vp, vp, i32, vp, i64, i64, vp, i64, i64, vp, vp]),
     "mw_pad_identity": (i32, [i64, i64, i32, vp, i64, i64, vp, i64, i64, vp]),

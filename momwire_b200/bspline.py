@@ -975,17 +975,16 @@ class BSplineSolver:
         return master.view(self.k, self.omega, self.mu)
 
     def _lu_solve(self, A, n, ws, ipiv, info, rhs, nrhs, stream):
-        """zgetrf(A) in place then zgetrs on rhs (both column-major, ld n)."""
+        """Factor A in place and solve for rhs (both column-major, ld n) in
+        one native call: the right-hand sides ride through the factorisation."""
         cancel = C.c_void_p(self._cancel.ptr) if self._cancel is not None else None
         try:
-            _lib.call("mw_zgetrf", n, A.data_ptr(), n, ipiv.data_ptr(), info.data_ptr(), ws.data_ptr(),
-                      ws.numel(), cancel, stream)
+            _lib.call("mw_zgesv", n, nrhs, A.data_ptr(), n, ipiv.data_ptr(), info.data_ptr(), rhs.data_ptr(), n,
+                      ws.data_ptr(), ws.numel(), cancel, stream)
         except _lib.NativeError as e:
             if e.status == _lib.MW_ERR_CANCELLED:
                 raise SolveAborted() from e
             raise
-        if nrhs:
-            _lib.call("mw_zgetrs", n, nrhs, A.data_ptr(), n, ipiv.data_ptr(), rhs.data_ptr(), n, stream)
 
     def _device_solve(self, buf, stream):
         """The whole device pipeline of compute_port_solution: fill, LU,
@@ -1335,9 +1334,10 @@ class BSplineSolver:
 
     def _swept_fp64_batched(self, k_array, mem_budget_bytes=16 << 30):
         """FP64 sweep: per chunk of frequencies one batched complex128 fill,
-        then each matrix of the stack factorised and solved in complex128
-        (``mw_zgetrf`` / ``mw_zgetrs``) on the device, the right-hand sides
-        [B | A^T] uploaded once; Y_k from the Schur step on the host."""
+        then the stack factorised and solved in complex128 in one native
+        call (``mw_zgesv_batched``: a cluster of CTAs per matrix), the
+        right-hand sides [B | A^T] uploaded once; Y_k from the Schur step on
+        the host."""
         torch = _torch()
         dev = self._torch_device()
         dt = self._dev_tables()
@@ -1363,15 +1363,13 @@ class BSplineSolver:
             X = Rd.unsqueeze(0).repeat(nk, 1, 1)  # (nk, m, n): X_k^T, overwritten by the solves
             ipiv = torch.empty((nk, n), dtype=torch.int32, device=dev)
             info = torch.zeros((nk, 2), dtype=torch.int32, device=dev)
-            for b in range(nk):
-                try:
-                    _lib.call("mw_zgetrf", n, Z[b].data_ptr(), n, ipiv[b].data_ptr(), info[b].data_ptr(),
-                              ws.data_ptr(), wsb, cancel, st)
-                except _lib.NativeError as e:
-                    if e.status == _lib.MW_ERR_CANCELLED:
-                        raise SolveAborted() from e
-                    raise
-                _lib.call("mw_zgetrs", n, m, Z[b].data_ptr(), n, ipiv[b].data_ptr(), X[b].data_ptr(), n, st)
+            try:
+                _lib.call("mw_zgesv_batched", n, m, nk, Z.data_ptr(), n, n * n, ipiv.data_ptr(), info.data_ptr(),
+                          X.data_ptr(), n, m * n, ws.data_ptr(), wsb, cancel, st)
+            except _lib.NativeError as e:
+                if e.status == _lib.MW_ERR_CANCELLED:
+                    raise SolveAborted() from e
+                raise
             hinfo = info.cpu().numpy()
             if np.any(hinfo[:, 1] != 0):
                 raise RuntimeError("factorisation: a bounded device wait timed out")

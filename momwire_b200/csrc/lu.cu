@@ -4,6 +4,9 @@
 // momwire (bspline.py:2971-2989).  Right-looking blocked algorithm, generic
 // in the element type (complex128 for the plain path, complex64 for the
 // mixed-precision path):
+// The complex128 path takes the cluster factorisation of lu_cluster.cu up to
+// zlu_cluster_max_rows(); what follows serves the larger orders and the
+// complex64 path.
 //   panel   : one cooperative kernel per panel; rows split over the CTAs,
 //             each CTA's row slab kept in shared memory for the whole panel,
 //             one all-to-all pivot exchange per column -- complex128: a
@@ -24,6 +27,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "lu_cluster.cuh"
 #include "tc_layout.cuh"
 #include "waits.cuh"
 
@@ -1207,20 +1211,29 @@ __global__ void __launch_bounds__(256, 1) zgemm_dmma_kernel(int64_t m, int64_t n
                 }
         if (tid == 0) split.count[st] = 0u;
     }
+    // C in batches of eight values per thread: all eight loads are in flight
+    // before the first store (a load behind a store to the same array would
+    // wait for it, one round trip after the other)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int64_t gr = m0 + wm * 32 + i * 8 + gid;
-        if (gr >= m) continue;
+        cd old[4][2];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int64_t gc = n0 + wn * 32 + j * 8 + 2 * tig + h;
-                if (gc >= n) continue;
+                old[j][h] = !beta_zero && gr < m && gc < n ? C[gr + gc * ldc] : cd{0.0, 0.0};
+            }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int64_t gc = n0 + wn * 32 + j * 8 + 2 * tig + h;
+                if (gr >= m || gc >= n) continue;
                 cd v = alpha * cd{x[i][j][h], w[i][j][h]};
-                cd* cp = C + gr + gc * ldc;
-                if (!beta_zero) v = v + beta * (*cp);
-                *cp = v;
+                if (!beta_zero) v = v + beta * old[j][h];
+                C[gr + gc * ldc] = v;
             }
     }
     }  // units
@@ -2211,6 +2224,15 @@ static mw_status getrs(int64_t n, int64_t nrhs, const T* LU, int64_t lda, const 
     return trsm_sweep<T>(true, n, nrhs, LU, lda, B, ldb, up_main, up, st);
 }
 
+// Orders one cluster factors and solves by itself (lu_cluster.cu); beyond,
+// the blocked factorisation's update on every SM wins.  Measured on B200
+// with 17 right-hand sides: 0.54 ms at 300, 1.49 ms at 640 in one launch;
+// 1.63 against 2.17 ms at 656.
+static int64_t zlu_full_max() { return 640; }
+// A batch fills the device with clusters up to the order its back
+// substitution holds; a few matrices alone follow the rule of one.
+static int64_t zlu_batch_max(int32_t batch) { return batch >= 8 ? 1696 : zlu_full_max(); }
+
 static size_t panel_ws_bytes() {
     size_t a, b, c, d;
     return ws_layout(kMaxPanelGrid, &a, &b, &c, &d);
@@ -2273,9 +2295,53 @@ static Updater tc_updater_main(char* ws, int64_t n, int64_t nrhs_max) {
 
 using namespace mw;
 
+// The panel exchange slots, then the row orders of the blocked cluster
+// factorisation.
 extern "C" size_t mw_getrf_workspace_size(int64_t n) {
-    (void)n;
-    return panel_ws_bytes();
+    return panel_ws_bytes() + sizeof(int32_t) * ((size_t)(n > 0 ? n : 0) + 2 * kZluBlock);
+}
+
+// Factor A, carrying B (nrhs >= 0 columns) through it: B <- L^-1 P B, or with
+// `back` B <- A^-1 B.
+static mw_status zgetrf_any(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* info, void* workspace, cd* B,
+                            int64_t ldb, int64_t nrhs, bool back, const volatile int32_t* cancel, cudaStream_t st) {
+    if (cancel && *cancel) {
+        set_error("factorisation cancelled");
+        return MW_ERR_CANCELLED;
+    }
+    if (n <= zlu_full_max()) {
+        MW_CHECK_CUDA(cudaMemsetAsync(info, 0, 2 * sizeof(int32_t), st));
+        if (n == 0) return MW_OK;
+        const bool in_kernel = back && nrhs <= 64;  // (beyond, the block solves' products win)
+        ZluArgs P{};
+        P.A = A;
+        P.lda = lda;
+        P.n = P.jb = (int)n;
+        P.ipiv = ipiv;
+        P.info = info;
+        P.B = B;
+        P.ldb = ldb;
+        P.nrhs = (int)nrhs;
+        P.back = in_kernel ? 1 : 0;
+        mw_status s = zlu_cluster(P, 1, st);
+        if (s != MW_OK || in_kernel || !back || nrhs == 0) return s;
+        return zlu_upper(n, A, lda, B, ldb, nrhs, st);
+    }
+    if (n <= zlu_cluster_max_rows()) {
+        MW_CHECK_CUDA(cudaMemsetAsync(info, 0, 2 * sizeof(int32_t), st));
+        mw_status s = zlu_blocked(n, A, lda, ipiv, info, B, ldb, nrhs,
+                                  reinterpret_cast<int32_t*>(static_cast<char*>(workspace) + panel_ws_bytes()), cancel,
+                                  st);
+        if (s != MW_OK || !back || nrhs == 0) return s;
+        return zlu_upper(n, A, lda, B, ldb, nrhs, st);
+    }
+    Updater up_main, up_trail;
+    up_main.max_ctas = kLaPanelCtas;
+    up_trail.max_ctas = panel_sms<cd>() - kLaPanelCtas;
+    mw_status s = getrf_lookahead<cd>(n, A, lda, ipiv, info, static_cast<char*>(workspace), cancel, up_main, up_trail,
+                                      st, B, ldb, nrhs);
+    if (s != MW_OK || !back || nrhs == 0) return s;
+    return zlu_upper(n, A, lda, B, ldb, nrhs, st);
 }
 
 extern "C" mw_status mw_zgetrf(int64_t n, double* Ad, int64_t lda, int32_t* ipiv, int32_t* info, void* workspace,
@@ -2283,12 +2349,70 @@ extern "C" mw_status mw_zgetrf(int64_t n, double* Ad, int64_t lda, int32_t* ipiv
     MW_REQUIRE(n >= 0 && lda >= (n > 0 ? n : 1), "bad n/lda");
     MW_REQUIRE(Ad && ipiv && info && workspace, "NULL argument");
     MW_REQUIRE(workspace_bytes >= mw_getrf_workspace_size(n), "workspace too small");
-    Updater up_main, up_trail;
-    up_main.max_ctas = kLaPanelCtas;
-    up_trail.max_ctas = panel_sms<cd>() - kLaPanelCtas;
     ProfileScope ps(PC_FACTOR, as_stream(stream), 8.0 / 3.0 * (double)n * n * n, 0.0);
-    return getrf_lookahead<cd>(n, reinterpret_cast<cd*>(Ad), lda, ipiv, info, static_cast<char*>(workspace), cancel,
-                               up_main, up_trail, as_stream(stream));
+    return zgetrf_any(n, reinterpret_cast<cd*>(Ad), lda, ipiv, info, workspace, nullptr, 0, 0, false, cancel,
+                      as_stream(stream));
+}
+
+extern "C" mw_status mw_zgesv(int64_t n, int64_t nrhs, double* Ad, int64_t lda, int32_t* ipiv, int32_t* info,
+                              double* Bd, int64_t ldb, void* workspace, size_t workspace_bytes,
+                              const volatile int32_t* cancel, void* stream) {
+    MW_REQUIRE(n >= 0 && nrhs >= 0 && lda >= (n > 0 ? n : 1) && ldb >= (n > 0 ? n : 1), "bad sizes");
+    MW_REQUIRE(Ad && ipiv && info && workspace && (nrhs == 0 || Bd), "NULL argument");
+    MW_REQUIRE(workspace_bytes >= mw_getrf_workspace_size(n), "workspace too small");
+    ProfileScope ps(PC_FACTOR, as_stream(stream), 8.0 / 3.0 * (double)n * n * n + 8.0 * (double)n * n * nrhs, 0.0);
+    return zgetrf_any(n, reinterpret_cast<cd*>(Ad), lda, ipiv, info, workspace, reinterpret_cast<cd*>(Bd), ldb, nrhs,
+                      true, cancel, as_stream(stream));
+}
+
+// CTAs a batch's clusters may take each: together they should cover the
+// device once.
+static int zlu_batch_ctas(int32_t batch) {
+    int c = panel_sms<cd>() / batch;
+    return c < 1 ? 1 : c;
+}
+
+extern "C" mw_status mw_zgesv_batched(int64_t n, int64_t nrhs, int32_t batch, double* Ad, int64_t lda, int64_t a_stride,
+                                      int32_t* ipiv, int32_t* info, double* Bd, int64_t ldb, int64_t b_stride,
+                                      void* workspace, size_t workspace_bytes, const volatile int32_t* cancel,
+                                      void* stream) {
+    MW_REQUIRE(n >= 1 && nrhs >= 1 && batch >= 1 && lda >= n && ldb >= n, "bad sizes");
+    MW_REQUIRE(a_stride >= lda * n && b_stride >= ldb * nrhs, "strides overlap");
+    MW_REQUIRE(Ad && ipiv && info && Bd && workspace, "NULL argument");
+    MW_REQUIRE(workspace_bytes >= mw_getrf_workspace_size(n), "workspace too small");
+    cudaStream_t st = as_stream(stream);
+    cd* A = reinterpret_cast<cd*>(Ad);
+    cd* B = reinterpret_cast<cd*>(Bd);
+    if (n <= zlu_batch_max(batch) && nrhs <= 64) {
+        if (cancel && *cancel) {
+            set_error("factorisation cancelled");
+            return MW_ERR_CANCELLED;
+        }
+        ProfileScope ps(PC_FACTOR, st, batch * (8.0 / 3.0 * (double)n * n * n + 8.0 * (double)n * n * nrhs), 0.0);
+        MW_CHECK_CUDA(cudaMemsetAsync(info, 0, 2 * sizeof(int32_t) * batch, st));
+        ZluArgs P{};
+        P.A = A;
+        P.lda = lda;
+        P.a_stride = a_stride;
+        P.n = P.jb = (int)n;
+        P.ipiv = ipiv;
+        P.ipiv_stride = n;
+        P.info = info;
+        P.info_stride = 2;
+        P.B = B;
+        P.ldb = ldb;
+        P.b_stride = b_stride;
+        P.nrhs = (int)nrhs;
+        P.back = 1;
+        return zlu_cluster(P, batch, st, zlu_batch_ctas(batch));
+    }
+    for (int32_t b = 0; b < batch; ++b) {
+        mw_status s = mw_zgesv(n, nrhs, reinterpret_cast<double*>(A + b * a_stride), lda, ipiv + b * n, info + 2 * b,
+                               reinterpret_cast<double*>(B + b * b_stride), ldb, workspace, workspace_bytes, cancel,
+                               stream);
+        if (s != MW_OK) return s;
+    }
+    return MW_OK;
 }
 
 extern "C" mw_status mw_zgetrs(int64_t n, int64_t nrhs, const double* LUd, int64_t lda, const int32_t* ipiv,

@@ -1,0 +1,952 @@
+// Complex128 LU of a block of columns by one thread-block cluster (sm_100a).
+//
+// A partial-pivoting factorisation is a chain of n pivot searches, each of
+// which every row below the diagonal takes part in.  What bounds it at the
+// orders of an antenna solve is the time of one link of that chain, so this
+// kernel keeps the chain inside one cluster of at most 16 CTAs:
+//   panel   W = 16 columns at a time, each row of the panel in the registers
+//           of one thread (rows never move while the panel is factored: a
+//           thread tracks the position its row would hold after LAPACK's
+//           interchanges).  For every column each CTA sends its candidate's
+//           key and row to all CTAs with st.async, which signals
+//           the receiver's mbarrier: one one-way trip through distributed
+//           shared memory per column and no barrier round trip (a cluster
+//           barrier behind plain remote stores took 1,200 cycles of a
+//           4,500-cycle column).  The next column's search and send
+//           come before the bulk of the row update.  Up to 32 rows per CTA one
+//           warp does it all.
+//   rest    the panel's row interchanges and the W x W triangular solve of
+//           the columns to its right, four lanes per column (all gathered
+//           values in flight at once; every CTA already holds L11 and the
+//           row order from the exchange), then the rank-W update in 64 x 32
+//           tiles on FP64 tensor instructions, the next tile's operands
+//           loading meanwhile.
+//   B       right-hand sides ride along as further columns; with `back` the
+//           kernel also substitutes backwards, each CTA its own right-hand
+//           sides, so a small system is factored and solved by one launch.
+// The batch is on the grid: cluster b works on matrix b.
+//
+// Measured on B200 (order 306, one right-hand side): 2.0 ms as a sequence of
+// cooperative panels, swaps, leaves and products, 0.55 ms as one launch; 64
+// such systems 125 ms one after the other, 1.4 ms as one batch.  A column
+// costs about 2,000 cycles: the pivot's pick and reciprocal 600, the next
+// search 200, sending the row 350, the flight (hidden behind the update) 650.
+//
+// The panel slots rotate: column 0 of the register row is always the current
+// pivot column, a step shifts the row left by one and appends the multiplier
+// on the right, so the column loop is one copy of code (an unrolled panel
+// overflows the instruction cache).
+//
+// Pivot choice is LAPACK's izamax: largest |re| + |im|, smallest row on ties.
+#include "common.cuh"
+#include "lu_cluster.cuh"
+
+#include <cooperative_groups.h>
+
+namespace mw {
+namespace cg = cooperative_groups;
+
+mw_status zgemm_launch(bool ta, bool tb, int64_t m, int64_t n, int64_t k, cd alpha, const cd* A, int64_t lda,
+                       const cd* B, int64_t ldb, cd beta, cd* C, int64_t ldc, cudaStream_t st, int max_ctas,
+                       void* split_ws, size_t split_ws_bytes);
+
+namespace {
+
+constexpr int kW = 16;          // panel width
+constexpr int kCT = 256;        // threads per CTA
+constexpr int kCWarps = kCT / 32;
+constexpr int kMaxC = 16;       // CTAs per cluster
+constexpr int kTM = 64, kTN = 32;  // update tile
+constexpr int kBackRows = 1696;  // order times right-hand sides a CTA substitutes at once
+constexpr unsigned kNone = 0xffffffffu;
+constexpr int kXchBytes = (kW + 1) * 16;  // one CTA's share of a column's exchange
+constexpr int kSpinLimit = 1 << 21;       // polls of an exchange wait before it gives up (about two seconds)
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void group_barrier(int threads) {
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned map_rank(unsigned addr, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// 16 bytes to another CTA's shared memory, counted on that CTA's mbarrier
+// (predicated, not branched around: a branch per destination costs more than
+// the store)
+__device__ __forceinline__ void st_async16(bool on, unsigned dst, cd v, unsigned mbar) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+        " @p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];\n}" ::"r"(dst),
+        "d"(v.re), "d"(v.im), "r"(mbar), "r"((unsigned)on)
+        : "memory");
+}
+__device__ __forceinline__ void mbar_init(unsigned mbar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(bool on, unsigned mbar, unsigned bytes) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}" ::"r"(
+            mbar),
+        "r"(bytes), "r"((unsigned)on)
+        : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned mbar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity), "r"(1000u)  // suspended at most a microsecond a poll
+        : "memory");
+    return ok != 0;
+}
+
+// L2 loads: another CTA of the cluster may have written the line
+__device__ __forceinline__ cd ld2(const cd* p) {
+    const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
+    return cd{v.x, v.y};
+}
+__device__ __forceinline__ void st2(cd* p, cd v) { __stcg(reinterpret_cast<double2*>(p), make_double2(v.re, v.im)); }
+
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+__device__ __forceinline__ cd csub_mul(cd c, cd a, cd b) {  // c - a b
+    c.re = fma(-a.re, b.re, c.re);
+    c.im = fma(-a.re, b.im, c.im);
+    c.re = fma(a.im, b.im, c.re);
+    c.im = fma(-a.im, b.re, c.im);
+    return c;
+}
+
+// 1 / z with one reciprocal: z is first scaled by the power of two that
+// brings its larger part into [1, 2) (exact), so |z|^2 neither overflows nor
+// loses bits.  recip_special: zero, subnormal, infinite and NaN z, which take
+// the plain division instead.
+__device__ __forceinline__ int recip_exp(cd z) {
+    return (int)((__double_as_longlong(fmax(fabs(z.re), fabs(z.im))) >> 52) & 0x7ff);
+}
+__device__ __forceinline__ bool recip_special(cd z) {
+    const int ex = recip_exp(z);
+    return ex < 2 || ex > 2044;
+}
+// (the reciprocal by Newton's iteration from the single-precision one: |z|^2
+// is in [1, 8), two steps reach the last bits, and nothing branches)
+__device__ __forceinline__ cd recip_fast(cd z) {
+    const int ex = min(max(recip_exp(z), 2), 2044);
+    const double s = __longlong_as_double((long long)(2046 - ex) << 52);  // 2^(1023 - ex)
+    const double x = z.re * s, y = z.im * s;
+    const double d = fma(x, x, y * y);
+    float r0;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"((float)d));
+    double r = (double)r0;
+    r = fma(r, fma(-d, r, 1.0), r);
+    r = fma(r, fma(-d, r, 1.0), r);
+    const double t = s * r;
+    return cd{x * t, -(y * t)};
+}
+__device__ __forceinline__ cd crecip(cd z) { return recip_special(z) ? cdiv(cd{1.0, 0.0}, z) : recip_fast(z); }
+
+// Warp-wide best of (value bits hi:lo, larger wins; then smaller pos); lanes
+// without a candidate have pos = kNone.  Returns the lane that holds it (a
+// lane without a candidate if all do).  Values are non-negative doubles,
+// whose bits order like the values.  One reduction settles it unless two
+// lanes share the high word.
+__device__ __forceinline__ int warp_pick(unsigned mh, unsigned hi, unsigned lo, unsigned pos) {
+    const bool h = pos != kNone && hi == mh;
+    unsigned eq = __ballot_sync(0xffffffffu, h);
+    if (__popc(eq) != 1) {
+        const unsigned ml = __reduce_max_sync(0xffffffffu, h ? lo : 0u);
+        const bool l = h && lo == ml;
+        const unsigned mp = __reduce_min_sync(0xffffffffu, l ? pos : kNone);
+        eq = __ballot_sync(0xffffffffu, l && pos == mp);
+    }
+    return eq ? __ffs(eq) - 1 : 0;
+}
+__device__ __forceinline__ int warp_best(unsigned hi, unsigned lo, unsigned pos) {
+    return warp_pick(__reduce_max_sync(0xffffffffu, pos == kNone ? 0u : hi), hi, lo, pos);
+}
+
+struct Shared {
+    // every CTA's candidate row, by column mod 4: a warp may still apply the
+    // row of column t while the candidates of t + 1 and t + 2 arrive
+    cd rows[4][kMaxC][kW];
+    uint4 key[4][kMaxC];  // its key: value bits lo, hi, position, row
+    unsigned long long mbar[4];
+    cd pub[kW + 1];  // this CTA's candidate row and key on their way out
+    uint4 wkey[2][kCWarps];  // the warps' candidates, by column parity
+    int src[kW];             // row that ends in position c0 + i
+    int disp[kW];            // where row c0 + i went (-1: it stays within the top W)
+    cd tri[kW][kW + 1];      // W x W triangle of the solves
+    cd dinv[kW];
+    cd X[kW][4];  // a solved block of the back substitution
+    cd zero;
+    union {
+        struct {
+            cd L[kW][kTM + 2];  // (row strides that spread the fragment loads over the banks)
+            cd U[kTN][kW + 4];
+        } g;
+        cd y[kBackRows];
+    } u;
+};
+
+template <int RPT>
+__global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
+    extern __shared__ __align__(16) unsigned char zlu_smem[];
+    Shared& S = *reinterpret_cast<Shared*>(zlu_smem);
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t mat = blockIdx.x / C;
+    cd* const A = P.A + mat * P.a_stride;
+    cd* const B = P.B + mat * P.b_stride;
+    int32_t* const ipiv = P.ipiv + mat * P.ipiv_stride;
+    int32_t* const info = P.info + mat * P.info_stride;
+    const int64_t lda = P.lda, ldb = P.ldb;
+    const int n = P.n, jend = P.j0 + P.jb;
+
+    if (tid == 0) {
+        S.zero = cd{0.0, 0.0};
+        for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&S.mbar[i]), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (P.rid != nullptr)
+        for (int r = P.j0 + rank * kCT + tid; r < n; r += C * kCT) P.rid[r] = r;
+    __syncthreads();
+    cluster_barrier();
+    int step = 0;       // columns done: exchange buffer and mbarrier phase
+    bool dead = false;  // an exchange wait gave up: no further waits
+
+    for (int c0 = P.j0; c0 < jend; c0 += kW) {
+        const int w = min(kW, jend - c0);
+        // ---------------------------------------------------------- panel
+        const int per = (n - c0 + C - 1) / C;
+        const int base = c0 + rank * per;
+        const int cnt = max(0, min(per, n - base));
+        const int nw = RPT > 1 ? kCWarps : min(kCWarps, (per + 31) / 32);  // warps that hold rows
+        if (warp < nw) {
+            cd a[RPT][kW];
+            unsigned pos[RPT];  // the row's current position; kNone: no row, or a pivot already
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) {
+                const int lr = tid + kCT * i;
+                const bool ok = lr < cnt;
+                pos[i] = ok ? (unsigned)(base + lr) : kNone;
+#pragma unroll
+                for (int x = 0; x < kW; ++x)
+                    a[i][x] = ok && x < w ? ld2(A + (base + lr) + (int64_t)(c0 + x) * lda) : cd{0.0, 0.0};
+            }
+            unsigned tpos = (unsigned)(c0 + lane);  // lane i: position of row c0 + i
+            // this thread's candidate of the next column, and the lane that
+            // holds the warp's
+            unsigned bhi = 0, blo = 0, bp = kNone;
+            int bi = 0, wsrc = 0;
+            cd next[RPT], l[RPT];  // next: the rows' entries of the next pivot column
+            auto search = [&]() {
+                unsigned long long bb = 0;
+                bp = kNone;
+                bi = 0;
+#pragma unroll
+                for (int i = 0; i < RPT; ++i)
+                    if (pos[i] != kNone) {
+                        const unsigned long long v = (unsigned long long)__double_as_longlong(cabs1(next[i]));
+                        if (bp == kNone || v > bb || (v == bb && pos[i] < bp)) {
+                            bb = v;
+                            bp = pos[i];
+                            bi = i;
+                        }
+                    }
+                bhi = (unsigned)(bb >> 32);
+                blo = (unsigned)bb;
+                wsrc = warp_best(bhi, blo, bp);
+            };
+            // the other CTAs' shared memory: lanes 0-15 send to even, lanes
+            // 16-31 to odd ranks
+            const unsigned self = smem_u32(&S);
+            unsigned peer[kMaxC / 2];
+#pragma unroll
+            for (int u = 0; u < kMaxC / 2; ++u) peer[u] = map_rank(self, min(2 * u + (lane >> 4), C - 1));
+            const unsigned kpeer = map_rank(self, min(lane, C - 1));
+            // Sends this CTA's candidate for panel column jj.  Its row is
+            // raw (shifted by one slot from slot 1 on, the last pivot row
+            // `piv` not yet applied; first column: as it is): the sending
+            // lanes apply it, an element each.
+            auto publish = [&](int jj, int st, const cd* piv, bool apply) {
+                const int buf = st & 3;
+                const unsigned mbar = smem_u32(&S.mbar[buf]), omb = mbar - self;
+                bool mine = true;  // this warp holds the CTA's candidate
+                if (nw > 1) {
+                    if (lane == wsrc) S.wkey[st & 1][warp] = make_uint4(bhi, blo, bp, 0);
+                    group_barrier(nw * 32);
+                    const uint4 k = S.wkey[st & 1][lane & (kCWarps - 1)];
+                    mine = warp == warp_best(k.x, k.y, lane < nw ? k.z : kNone);
+                }
+                mbar_expect(tid == 0, mbar, (unsigned)(C * kXchBytes));
+                if (!mine) return;
+                if (lane == wsrc) {
+#pragma unroll
+                    for (int i = 0; i < RPT; ++i)
+                        if (RPT == 1 || i == bi) {
+                            if (jj == 0) {
+#pragma unroll
+                                for (int x = 0; x < kW; ++x) S.pub[x] = a[i][x];
+                            } else {
+#pragma unroll
+                                for (int x = 0; x + 1 < kW; ++x) S.pub[x] = a[i][x + 1];
+                                S.pub[kW - 1] = l[i];
+                            }
+                        }
+                    // key: value, position, row
+                    S.pub[kW] =
+                        cd{__longlong_as_double((long long)(((unsigned long long)bhi << 32) | blo)),
+                           __longlong_as_double(
+                               (long long)(((unsigned long long)(unsigned)(base + tid + kCT * bi) << 32) | bp))};
+                }
+                __syncwarp();
+                const int x = lane & 15;
+                cd v = S.pub[x];
+                const cd kv = S.pub[kW];
+                if (jj > 0 && apply && x < kW - jj) v = csub_mul(v, S.pub[kW - 1], piv[x + 1]);
+                const unsigned orow = smem_u32(&S.rows[buf][rank][x]) - self;
+                const unsigned okey = smem_u32(&S.key[buf][rank]) - self;
+#pragma unroll
+                for (int u = 0; u < kMaxC / 2; ++u)
+                    st_async16(2 * u + (lane >> 4) < C, peer[u] + orow, v, peer[u] + omb);
+                st_async16(lane < C, kpeer + okey, kv, kpeer + omb);
+                __syncwarp();
+            };
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) next[i] = a[i][0];
+            search();
+            publish(0, step, nullptr, false);
+            for (int jj = 0; jj < w; ++jj, ++step) {
+                const int buf = step & 3;
+                const unsigned c = (unsigned)(c0 + jj);
+                if (!dead) {
+                    int spins = 0;
+                    while (!mbar_try(smem_u32(&S.mbar[buf]), (unsigned)((step >> 2) & 1)))
+                        if (++spins > kSpinLimit) {
+                            dead = true;
+                            info[1] = MW_ERR_TIMEOUT;
+                            break;
+                        }
+                    dead = __any_sync(0xffffffffu, dead);
+                }
+                // the winner, from this CTA's own copies; each lane takes the
+                // reciprocal of one candidate in the reduction's shadow
+                const uint4 k = S.key[buf][lane & (kMaxC - 1)];
+                const unsigned kp = lane < C ? k.z : kNone;
+                const unsigned mh = __reduce_max_sync(0xffffffffu, kp == kNone ? 0u : k.y);
+                const cd z = S.rows[buf][lane & (kMaxC - 1)][0];
+                const cd iv = recip_fast(z);
+                const unsigned fl = ((k.x | k.y) != 0 ? 1u : 0u) | (recip_special(z) ? 2u : 0u);
+                const int g = warp_pick(mh, k.y, k.x, kp) & (kMaxC - 1);
+                const unsigned p = __shfl_sync(0xffffffffu, k.z, g), orig = __shfl_sync(0xffffffffu, k.w, g);
+                // LAPACK: an exact zero pivot is neither divided by nor applied
+                const unsigned flags = __shfl_sync(0xffffffffu, fl, g);
+                const bool apply = (flags & 1u) != 0;
+                const cd* piv = S.rows[buf][g];
+                cd inv{__shfl_sync(0xffffffffu, iv.re, g), __shfl_sync(0xffffffffu, iv.im, g)};
+                if (flags & 2u) inv = apply ? cdiv(cd{1.0, 0.0}, piv[0]) : cd{1.0, 0.0};
+                const int wj = apply ? kW - jj : 0;  // slots the pivot row updates
+                const cd p1 = *(1 < wj ? piv + 1 : &S.zero);
+                tpos = tpos == p ? c : (tpos == c ? p : tpos);
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) {
+                    pos[i] = pos[i] == p ? kNone : (pos[i] == c ? p : pos[i]);
+                    l[i] = a[i][0] * inv;
+                    next[i] = csub_mul(a[i][1], l[i], p1);
+                }
+                if (jj + 1 < w) {
+                    search();
+                    publish(jj + 1, step + 1, piv, apply);
+                }
+                // while the exchange is under way: the pivot row out, and the
+                // other columns (slots that hold multipliers meet a zero; a
+                // retired row's registers no longer matter)
+                if (warp == nw - 1) {
+                    if (rank == (jj & (C - 1)) && lane < w) {
+                        // slot s < W - jj holds column jj + s, then the multipliers
+                        const int sl = lane >= jj ? lane - jj : kW - jj + lane;
+                        st2(A + c + (int64_t)(c0 + lane) * lda, piv[sl]);
+                    }
+                    if (lane < jj) S.tri[jj][lane] = piv[kW - jj + lane];
+                    if (lane == 0) {
+                        // (clamped: after a wait that gave up the word is not a row)
+                        S.src[jj] = (int)min(max(orig, (unsigned)c0), (unsigned)(n - 1));
+                        if (rank == 0) {
+                            ipiv[c] = (int32_t)(p + 1);
+                            if (!apply && info[0] == 0) info[0] = (int32_t)(c + 1);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) a[i][0] = next[i];
+#pragma unroll
+                for (int x = 1; x + 1 < kW; ++x) {
+                    const cd px = *(x + 1 < wj ? piv + x + 1 : &S.zero);
+#pragma unroll
+                    for (int i = 0; i < RPT; ++i) a[i][x] = csub_mul(a[i][x + 1], l[i], px);
+                }
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) a[i][kW - 1] = l[i];
+            }
+            // the rows below to their positions: the last w slots hold their
+            // multipliers
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+                if (pos[i] != kNone) {
+                    cd* row = A + min(pos[i], (unsigned)(n - 1)) + (int64_t)c0 * lda;
+#pragma unroll
+                    for (int s = 0; s < kW; ++s)
+                        if (s >= kW - w) st2(row + (int64_t)(s - (kW - w)) * lda, a[i][s]);
+                }
+            if (warp == 0 && lane < kW)
+                S.disp[lane] = lane < w && tpos >= (unsigned)(c0 + w) ? (int)min(tpos, (unsigned)(n - 1)) : -1;
+        } else {
+            step += w;
+        }
+        __syncthreads();
+        // ------------------------------------- interchanges, triangular solve
+        const int left = c0 - P.j0, right = jend - c0 - w;
+        const int ncols = left + right + P.nrhs;
+        // four lanes a column (lane f of them holds rows f, f + 4, ...: a
+        // single thread's substitution is one long chain), eight columns a
+        // warp, to the warps of all CTAs in turn
+        const int f = lane & 3;
+        for (int qb = (warp * C + rank) * 8; qb < ncols; qb += kCWarps * C * 8) {
+            const int q = qb + (lane >> 2);
+            const bool ok = q < ncols;
+            cd* col = q < left ? A + (int64_t)(P.j0 + q) * lda
+                               : (q < left + right ? A + (int64_t)(c0 + w + q - left) * lda
+                                                   : B + (int64_t)(q - left - right) * ldb);
+            cd t[kW / 4], d[kW / 4];
+#pragma unroll
+            for (int u = 0; u < kW / 4; ++u) {
+                const int i = 4 * u + f;
+                t[u] = ok && i < w ? ld2(col + S.src[i]) : cd{0.0, 0.0};
+                d[u] = ok && S.disp[i] >= 0 ? ld2(col + c0 + i) : cd{0.0, 0.0};
+            }
+            __syncwarp();  // the column is read before it is written
+#pragma unroll
+            for (int u = 0; u < kW / 4; ++u)
+                if (ok && S.disp[4 * u + f] >= 0) st2(col + S.disp[4 * u + f], d[u]);
+            if (qb + 7 >= left) {
+#pragma unroll
+                for (int k = 0; k + 1 < kW; ++k) {
+                    const cd x{__shfl_sync(0xffffffffu, t[k / 4].re, (lane & ~3) | (k & 3)),
+                               __shfl_sync(0xffffffffu, t[k / 4].im, (lane & ~3) | (k & 3))};
+#pragma unroll
+                    for (int u = k / 4; u < kW / 4; ++u) {
+                        const int i = 4 * u + f;
+                        if (i > k && i < w && q >= left) t[u] = csub_mul(t[u], S.tri[i][k], x);
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kW / 4; ++u)
+                if (ok && 4 * u + f < w) st2(col + c0 + 4 * u + f, t[u]);
+        }
+        if (P.rid != nullptr && rank == C - 1 && warp == kCWarps - 1) {
+            // the rows' origins move like a column
+            const int t = lane < w ? __ldcg(P.rid + S.src[lane]) : 0;
+            const int dd = lane < w && S.disp[lane] >= 0 ? __ldcg(P.rid + c0 + lane) : 0;
+            __syncwarp();
+            if (lane < w) {
+                __stcg(P.rid + c0 + lane, t);
+                if (S.disp[lane] >= 0) __stcg(P.rid + S.disp[lane], dd);
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+        cluster_barrier();
+        // ---------------------------------------------------- rank-w update
+        const int r0 = c0 + w, m2 = n - r0, n2 = right + P.nrhs;
+        const int tm = (m2 + kTM - 1) / kTM, tn = (n2 + kTN - 1) / kTN;
+        auto colptr = [&](int q) { return q < right ? A + (int64_t)(r0 + q) * lda : B + (int64_t)(q - right) * ldb; };
+        // warp tile 16 x 16 of the 64 x 32: 2 x 2 blocks of 8 x 8, FP64
+        // tensor instructions with the four-product complex form
+        const int gid = lane >> 2, tig = lane & 3, wm = (warp & 3) * 16, wn = (warp >> 2) * 16;
+        cd acc[2][2][2], fl[kW * kTM / kCT], fu[kW * kTN / kCT];
+        auto fetch = [&](int i0, int q0) {  // C, L and U of a tile
+#pragma unroll
+            for (int u = 0; u < kW * kTM / kCT; ++u) {
+                const int e = tid + u * kCT, r = e % kTM, k = e / kTM;
+                fl[u] = k < w && i0 + r < m2 ? ld2(A + (r0 + i0 + r) + (int64_t)(c0 + k) * lda) : cd{0.0, 0.0};
+            }
+#pragma unroll
+            for (int u = 0; u < kW * kTN / kCT; ++u) {
+                const int e = tid + u * kCT, k = e % kW, q = e / kW;
+                fu[u] = k < w && q0 + q < n2 ? ld2(colptr(q0 + q) + c0 + k) : cd{0.0, 0.0};
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int q = q0 + wn + 8 * j + 2 * tig + h;
+                    const cd* col = colptr(q) + r0 + i0 + wm + gid;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+                        acc[i][j][h] = q < n2 && i0 + wm + gid + 8 * i < m2 ? ld2(col + 8 * i) : cd{0.0, 0.0};
+                }
+        };
+        // this CTA's tiles: row tiles fastest
+        int ti = rank % max(tm, 1), tq = tm > 0 ? rank / tm : tn;
+        const int di = C % max(tm, 1), dq = C / max(tm, 1);
+        if (tq < tn) fetch(ti * kTM, tq * kTN);
+        while (tq < tn) {
+            const int i0 = ti * kTM, q0 = tq * kTN;
+#pragma unroll
+            for (int u = 0; u < kW * kTM / kCT; ++u) {
+                const int e = tid + u * kCT;
+                S.u.g.L[e / kTM][e % kTM] = fl[u];
+            }
+#pragma unroll
+            for (int u = 0; u < kW * kTN / kCT; ++u) {
+                const int e = tid + u * kCT;
+                S.u.g.U[e / kW][e % kW] = fu[u];
+            }
+            double cr[2][2][2], ci[2][2][2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        cr[i][j][h] = acc[i][j][h].re;
+                        ci[i][j][h] = acc[i][j][h].im;
+                    }
+            __syncthreads();
+            ti += di;
+            tq += dq;
+            if (ti >= tm) {
+                ti -= tm;
+                ++tq;
+            }
+            if (tq < tn) fetch(ti * kTM, tq * kTN);
+#pragma unroll
+            for (int k4 = 0; k4 < kW; k4 += 4) {
+                cd la[2], ub[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) la[i] = S.u.g.L[k4 + tig][wm + 8 * i + gid];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) ub[j] = S.u.g.U[wn + 8 * j + gid][k4 + tig];
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        dmma(cr[i][j][0], cr[i][j][1], -la[i].re, ub[j].re);
+                        dmma(ci[i][j][0], ci[i][j][1], -la[i].re, ub[j].im);
+                    }
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        dmma(cr[i][j][0], cr[i][j][1], la[i].im, ub[j].im);
+                        dmma(ci[i][j][0], ci[i][j][1], -la[i].im, ub[j].re);
+                    }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int q = q0 + wn + 8 * j + 2 * tig + h;
+                    if (q < n2) {
+                        cd* col = colptr(q) + r0 + i0 + wm + gid;
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            if (i0 + wm + gid + 8 * i < m2) st2(col + 8 * i, cd{cr[i][j][h], ci[i][j][h]});
+                    }
+                }
+            __syncthreads();
+        }
+        __syncwarp();
+        cluster_barrier();
+    }
+    if (P.rid != nullptr) {
+        // the block's row order: src[i] the row that ends in position j0 + i,
+        // disp[i] where row j0 + i went (-1: it stays within the block)
+        int32_t* const src = P.rid + n;
+        int32_t* const disp = src + P.jb;
+        for (int r = P.j0 + rank * kCT + tid; r < n; r += C * kCT) {
+            const int o = __ldcg(P.rid + r);
+            if (r < jend) src[r - P.j0] = o;
+            if (o < jend) disp[o - P.j0] = r < jend ? -1 : r;
+        }
+    }
+    if (!P.back) return;
+    // ------------------------------------------------------ U X = L^-1 P B
+    // The right-hand sides are independent: CTA r takes columns r, r + C, ...
+    // up to four at a time, in shared memory, and needs no other CTA.  Per
+    // block of 16 rows: sixteen lanes a right-hand side substitute (lane i
+    // row i), then every thread updates its rows above; triangle, reciprocal
+    // diagonal and the rows' U entries are fetched a block ahead.
+    const int mine = P.nrhs > rank ? (P.nrhs - rank + C - 1) / C : 0;
+    const int at_once = min(4, kBackRows / n);
+    for (int q0 = 0; q0 < mine; q0 += at_once) {
+        const int nq = min(at_once, mine - q0);
+        cd* Bq = B + (int64_t)(rank + q0 * C) * ldb;
+        const int64_t bstep = (int64_t)C * ldb;
+        cd ft, fd, fu[kW];
+        auto fetch = [&](int b0) {
+            const int w = min(kW, n - b0), r = tid % kW, k = tid / kW;
+            ft = r < k && k < w ? ld2(A + (b0 + r) + (int64_t)(b0 + k) * lda) : cd{0.0, 0.0};
+            fd = tid < w ? ld2(A + (b0 + tid) + (int64_t)(b0 + tid) * lda) : cd{1.0, 0.0};
+#pragma unroll
+            for (int c = 0; c < kW; ++c)
+                fu[c] = tid < b0 && c < w ? ld2(A + tid + (int64_t)(b0 + c) * lda) : cd{0.0, 0.0};
+        };
+        static_assert(kCT == kW * kW, "one triangle entry per thread");
+        cd* y = S.u.y;  // [n][at_once]
+        for (int e = tid; e < n * nq; e += kCT) y[(e % n) * at_once + e / n] = ld2(Bq + e % n + (e / n) * bstep);
+        const int last = ((n - 1) / kW) * kW;
+        fetch(last);
+        for (int b0 = last; b0 >= 0; b0 -= kW) {
+            const int w = min(kW, n - b0);
+            S.tri[tid % kW][tid / kW] = ft;
+            if (tid < kW) S.dinv[tid] = crecip(fd);
+            cd u[kW];
+#pragma unroll
+            for (int c = 0; c < kW; ++c) u[c] = fu[c];
+            if (b0 > 0) fetch(b0 - kW);
+            __syncthreads();
+            const int q = tid >> 4, i = tid & 15;
+            if (warp < 2) {
+                const bool ok = q < nq && i < w;
+                cd t = ok ? y[(b0 + i) * at_once + q] : cd{0.0, 0.0};
+                const cd di = S.dinv[i];
+#pragma unroll
+                for (int k = kW - 1; k >= 0; --k) {
+                    if (i == k) t = t * di;
+                    const cd x{__shfl_sync(0xffffffffu, t.re, (lane & 16) | k),
+                               __shfl_sync(0xffffffffu, t.im, (lane & 16) | k)};
+                    if (i < k) t = csub_mul(t, S.tri[i][k], x);
+                }
+                S.X[i][q] = t;
+                if (ok) st2(Bq + b0 + i + q * bstep, t);
+            }
+            __syncthreads();
+            for (int r = tid; r < b0; r += kCT) {
+                if (r != tid)
+#pragma unroll
+                    for (int c = 0; c < kW; ++c)
+                        u[c] = c < w ? ld2(A + r + (int64_t)(b0 + c) * lda) : cd{0.0, 0.0};
+                for (int p = 0; p < nq; ++p) {
+                    cd v = y[r * at_once + p], v2{0.0, 0.0};
+#pragma unroll
+                    for (int c = 0; c < kW; c += 2) {
+                        v = csub_mul(v, u[c], S.X[c][p]);
+                        v2 = csub_mul(v2, u[c + 1], S.X[c + 1][p]);
+                    }
+                    y[r * at_once + p] = v + v2;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// ------------------------------------------------------------ block solves
+// X <- T^-1 P X for the jb <= 128 rows [j0, j0 + jb) of many columns, T the
+// unit lower (or, UPPER, the upper) triangle of the diagonal block and P the
+// block's row order (src / disp of the panel; null: the rows stay).  A CTA
+// holds 32 columns of X in shared memory and takes the triangle in strips of
+// 16 columns: one warp solves the strip's 16 rows (a column per lane, in
+// registers), all warps apply it to the rest.  The columns left of the block
+// only take the interchanges: `left` of them from Aleft on, in CTAs of their
+// own.  A gather of all rows at once replaces LAPACK's sequential swaps.
+constexpr int kSN = 32, kSMax = 128;
+constexpr int kSPitch = kSN + 1;
+constexpr size_t kSolveSmem = sizeof(cd) * (kSMax * kSPitch + kW * kSMax + kW) + sizeof(int) * 2 * kSMax;
+
+struct SolveArgs {
+    const cd* T;  // the diagonal block
+    int64_t ldt;
+    int j0, jb;
+    const int32_t *src, *disp;
+    cd* Aleft;
+    int64_t ldleft;
+    int left;
+    cd* X;  // column 0, row 0 of the right columns
+    int64_t ldx;
+    int ncols;
+    cd* B;  // further right columns
+    int64_t ldb;
+    int nrhs;
+};
+
+template <bool UPPER>
+__global__ void __launch_bounds__(kCT) zblock_solve_kernel(SolveArgs P) {
+    extern __shared__ __align__(16) unsigned char zs_smem[];
+    cd* X = reinterpret_cast<cd*>(zs_smem);  // [kSMax][kSPitch]
+    cd* Ls = X + kSMax * kSPitch;            // [kW][kSMax]
+    cd* dinv = Ls + kW * kSMax;
+    int* src = reinterpret_cast<int*>(dinv + kW);
+    int* disp = src + kSMax;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nleft = (P.left + kSN - 1) / kSN;
+    const bool isleft = (int)blockIdx.x < nleft;
+    const int q0 = ((int)blockIdx.x - (isleft ? 0 : nleft)) * kSN;
+    const int total = isleft ? P.left : P.ncols + P.nrhs;
+    const int j0 = P.j0, jb = P.jb;
+    auto colptr = [&](int q) {
+        return isleft ? P.Aleft + (int64_t)q * P.ldleft
+                      : (q < P.ncols ? P.X + (int64_t)q * P.ldx : P.B + (int64_t)(q - P.ncols) * P.ldb);
+    };
+    for (int i = tid; i < jb; i += kCT) {
+        src[i] = P.src ? P.src[i] : j0 + i;
+        disp[i] = P.src ? P.disp[i] : -1;
+    }
+    __syncthreads();
+    constexpr int U = kSMax * kSN / kCT;
+    {
+        cd d[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int e = tid + u * kCT, r = e % kSMax, c = e / kSMax;
+            const bool ok = r < jb && q0 + c < total;
+            const cd* col = colptr(q0 + c);
+            X[r * kSPitch + c] = ok ? ld2(col + src[r]) : cd{0.0, 0.0};
+            d[u] = ok && disp[r] >= 0 ? ld2(col + j0 + r) : cd{0.0, 0.0};
+        }
+        __syncthreads();  // every row read before any is overwritten
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int e = tid + u * kCT, r = e % kSMax, c = e / kSMax;
+            if (r < jb && q0 + c < total && disp[r] >= 0) st2(colptr(q0 + c) + disp[r], d[u]);
+        }
+    }
+    const int nstrip = isleft ? 0 : (jb + kW - 1) / kW;
+    for (int s = 0; s < nstrip; ++s) {
+        const int k0 = (UPPER ? nstrip - 1 - s : s) * kW, w = min(kW, jb - k0);
+        // the strip's rows: k0 .. jb (lower), 0 .. k0 + w (upper)
+        const int f0 = UPPER ? 0 : k0, f1 = UPPER ? k0 + w : jb;
+        for (int e = tid; e < kW * kSMax; e += kCT) {
+            const int r = f0 + e % kSMax, k = e / kSMax;
+            if (r < f1) Ls[k * kSMax + r] = k < w ? ld2(P.T + r + (int64_t)(k0 + k) * P.ldt) : cd{0.0, 0.0};
+        }
+        if (UPPER && tid < w) dinv[tid] = cdiv(cd{1.0, 0.0}, ld2(P.T + (k0 + tid) + (int64_t)(k0 + tid) * P.ldt));
+        __syncthreads();
+        if (warp == 0) {
+            cd t[kW];
+#pragma unroll
+            for (int i = 0; i < kW; ++i) t[i] = i < w ? X[(k0 + i) * kSPitch + lane] : cd{0.0, 0.0};
+            if (UPPER) {
+#pragma unroll
+                for (int i = kW - 1; i >= 0; --i)
+                    if (i < w) {
+                        t[i] = t[i] * dinv[i];
+#pragma unroll
+                        for (int r = 0; r < i; ++r) t[r] = csub_mul(t[r], Ls[i * kSMax + k0 + r], t[i]);
+                    }
+            } else {
+#pragma unroll
+                for (int k = 0; k + 1 < kW; ++k)
+#pragma unroll
+                    for (int i = k + 1; i < kW; ++i)
+                        if (i < w) t[i] = csub_mul(t[i], Ls[k * kSMax + k0 + i], t[k]);
+            }
+#pragma unroll
+            for (int i = 0; i < kW; ++i)
+                if (i < w) X[(k0 + i) * kSPitch + lane] = t[i];
+        }
+        __syncthreads();
+        const int g0 = UPPER ? 0 : k0 + w, g1 = UPPER ? k0 : jb;
+        if (g0 < g1) {
+            cd xk[kW];
+#pragma unroll
+            for (int k = 0; k < kW; ++k) xk[k] = k < w ? X[(k0 + k) * kSPitch + lane] : cd{0.0, 0.0};
+            for (int r = g0 + warp; r < g1; r += kCWarps) {
+                cd y = X[r * kSPitch + lane], z{0.0, 0.0};
+#pragma unroll
+                for (int k = 0; k < kW; k += 2) {  // two chains
+                    y = csub_mul(y, Ls[k * kSMax + r], xk[k]);
+                    z = csub_mul(z, Ls[(k + 1) * kSMax + r], xk[k + 1]);
+                }
+                X[r * kSPitch + lane] = y + z;
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll 4
+    for (int u = 0; u < U; ++u) {
+        const int e = tid + u * kCT, r = e % kSMax, c = e / kSMax;
+        if (r < jb && q0 + c < total) st2(colptr(q0 + c) + j0 + r, X[r * kSPitch + c]);
+    }
+}
+
+template <bool UPPER>
+mw_status block_solve(const SolveArgs& P, cudaStream_t st) {
+    static const cudaError_t attr = cudaFuncSetAttribute(
+        zblock_solve_kernel<UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveSmem);
+    MW_CHECK_CUDA(attr);
+    const int ctas = (P.left + kSN - 1) / kSN + (P.ncols + P.nrhs + kSN - 1) / kSN;
+    if (ctas == 0) return MW_OK;
+    ProfileScope ps(PC_TRSM, st, 4.0 * (double)P.jb * P.jb * (P.ncols + P.nrhs),
+                    32.0 * (double)P.jb * (P.left + P.ncols + P.nrhs));
+    zblock_solve_kernel<UPPER><<<(unsigned)ctas, kCT, kSolveSmem, st>>>(P);
+    MW_CHECK_CUDA(cudaGetLastError());
+    count_launch();
+    return MW_OK;
+}
+
+// Largest cluster this device can hold of the kernel: 16 CTAs (a
+// non-portable size) where it fits, else 8.
+template <int RPT>
+int max_cluster() {
+    static const int v = [] {
+        auto kern = zlu_cluster_kernel<RPT>;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared)) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return 8;
+        }
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kMaxC);
+        cfg.blockDim = dim3(kCT);
+        cfg.dynamicSmemBytes = sizeof(Shared);
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kMaxC;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int num = 0;
+        if (cudaOccupancyMaxActiveClusters(&num, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return 8;
+        }
+        return num >= 1 ? kMaxC : 8;
+    }();
+    return v;
+}
+
+template <int RPT>
+mw_status launch(const ZluArgs& P, int C, int batch, cudaStream_t st) {
+    MW_REQUIRE(C <= max_cluster<RPT>(), "cluster too large");  // (sets the kernel's attributes)
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(batch * C));
+    cfg.blockDim = dim3(kCT);
+    cfg.dynamicSmemBytes = sizeof(Shared);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    ProfileScope ps(PC_PANEL, st, 4.0 * (double)(P.n - P.j0) * P.jb * P.jb * batch,
+                    32.0 * (double)(P.n - P.j0) * P.jb * batch);
+    MW_CHECK_CUDA(cudaLaunchKernelEx(&cfg, zlu_cluster_kernel<RPT>, P));
+    count_launch();
+    return MW_OK;
+}
+
+}  // namespace
+
+int zlu_cluster_max_rows() { return max_cluster<3>() * kCT * 3; }
+
+mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas) {
+    MW_REQUIRE(batch >= 1 && P.jb >= 1 && P.j0 >= 0 && P.j0 + P.jb <= P.n, "bad block");
+    MW_REQUIRE(!P.back || (P.j0 == 0 && P.jb == P.n && P.n <= kBackRows), "back substitution needs the whole matrix");
+    const int m = P.n - P.j0;
+    const int cap = max_ctas > 0 && max_ctas < kMaxC ? max_ctas : kMaxC;
+    int C = 1;
+    while (C < cap && C < max_cluster<1>() && C * 32 < m) C *= 2;
+    // enough rows per thread for the panel
+    while (C < kMaxC && (m + C - 1) / C > 3 * kCT) C *= 2;
+    const int per = (m + C - 1) / C;
+    if (per <= kCT) return launch<1>(P, C, batch, st);
+    if (per <= 2 * kCT) return launch<2>(P, C, batch, st);
+    MW_REQUIRE(per <= 3 * kCT, "block of %d rows too large for one cluster", m);
+    return launch<3>(P, C, batch, st);
+}
+
+// ------------------------------------------------------------------ driver
+// Blocked factorisation of the whole matrix with nrhs carried columns (B <-
+// L^-1 P B).  `rid`: n + 2 kZluBlock ints of workspace.  One stream: the
+// block's cluster leaves 132 SMs idle, but its chain is short beside the
+// update, which in return has every SM (a second stream's update would keep
+// a cluster from finding its SMs together).
+mw_status zlu_blocked(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* info, cd* B, int64_t ldb, int64_t nrhs,
+                      int32_t* rid, const volatile int32_t* cancel, cudaStream_t st) {
+    const int nb = kZluBlock;
+    for (int64_t j0 = 0; j0 < n; j0 += nb) {
+        if (cancel && *cancel) {
+            MW_CHECK_CUDA(cudaStreamSynchronize(st));
+            set_error("factorisation cancelled");
+            return MW_ERR_CANCELLED;
+        }
+        const int jb = (int)(n - j0 < nb ? n - j0 : nb);
+        const int64_t c1 = j0 + jb, right = n - c1;
+        ZluArgs P{};
+        P.A = A;
+        P.lda = lda;
+        P.n = (int)n;
+        P.j0 = (int)j0;
+        P.jb = jb;
+        P.ipiv = ipiv;
+        P.info = info;
+        P.rid = rid;
+        mw_status s = zlu_cluster(P, 1, st);
+        if (s != MW_OK) return s;
+        SolveArgs Q{};
+        Q.T = A + j0 + j0 * lda;
+        Q.ldt = lda;
+        Q.j0 = (int)j0;
+        Q.jb = jb;
+        Q.src = rid + n;
+        Q.disp = rid + n + jb;
+        Q.Aleft = A;
+        Q.ldleft = lda;
+        Q.left = (int)j0;
+        Q.X = A + c1 * lda;
+        Q.ldx = lda;
+        Q.ncols = (int)right;
+        Q.B = B;
+        Q.ldb = ldb;
+        Q.nrhs = (int)nrhs;
+        s = block_solve<false>(Q, st);
+        if (s != MW_OK) return s;
+        if (right > 0) {
+            const cd m1{-1.0, 0.0}, p1{1.0, 0.0};
+            s = zgemm_launch(false, false, right, right, jb, m1, A + c1 + j0 * lda, lda, A + j0 + c1 * lda, lda, p1,
+                             A + c1 + c1 * lda, lda, st, 0, nullptr, 0);
+            if (s == MW_OK && nrhs > 0)
+                s = zgemm_launch(false, false, right, nrhs, jb, m1, A + c1 + j0 * lda, lda, B + j0, ldb, p1, B + c1,
+                                 ldb, st, 0, nullptr, 0);
+            if (s != MW_OK) return s;
+        }
+    }
+    return MW_OK;
+}
+
+// B <- U^-1 B, 128 rows at a time.
+mw_status zlu_upper(int64_t n, const cd* LU, int64_t lda, cd* B, int64_t ldb, int64_t nrhs, cudaStream_t st) {
+    for (int64_t j0 = (n - 1) / kSMax * kSMax; j0 >= 0; j0 -= kSMax) {
+        SolveArgs Q{};
+        Q.T = LU + j0 + j0 * lda;
+        Q.ldt = lda;
+        Q.j0 = (int)j0;
+        Q.jb = (int)(n - j0 < kSMax ? n - j0 : kSMax);
+        Q.X = B;
+        Q.ldx = ldb;
+        Q.ncols = (int)nrhs;
+        mw_status s = block_solve<true>(Q, st);
+        if (s == MW_OK && j0 > 0)
+            s = zgemm_launch(false, false, j0, nrhs, Q.jb, cd{-1.0, 0.0}, LU + j0 * lda, lda, B + j0, ldb,
+                             cd{1.0, 0.0}, B, ldb, st, 0, nullptr, 0);
+        if (s != MW_OK) return s;
+    }
+    return MW_OK;
+}
+
+}  // namespace mw

@@ -1,0 +1,40 @@
+// Complex128 LU of a block of columns by one thread-block cluster per matrix
+// (lu_cluster.cu).
+#pragma once
+
+#include "common.cuh"
+
+namespace mw {
+
+struct ZluArgs {
+    cd* A;  // column-major
+    int64_t lda, a_stride;
+    int n;       // order: rows [j0, n) take part
+    int j0, jb;  // columns factored
+    int32_t* ipiv;  // 1-based, whole matrix
+    int64_t ipiv_stride;
+    int32_t* info;  // info[0]: first exact zero pivot (1-based), untouched otherwise
+    int64_t info_stride;
+    cd* B;  // nrhs further columns of n rows (may be null with nrhs = 0)
+    int64_t ldb, b_stride;
+    int nrhs;
+    int back;  // also B <- U^-1 B (whole matrix, nrhs <= 64)
+    // n + 2 jb ints (single matrix), or null: on return rid[n + i] is the
+    // row that ends in position j0 + i and rid[n + jb + i] the position row
+    // j0 + i went to (-1: it stays within the block)
+    int32_t* rid;
+};
+
+// Rows one cluster can hold.
+int zlu_cluster_max_rows();
+mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas = 0);
+
+// Columns of a block of the blocked factorisation.
+constexpr int kZluBlock = 128;
+// Whole factorisation of an order within zlu_cluster_max_rows() by blocks;
+// rid: n + 2 kZluBlock ints.
+mw_status zlu_blocked(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* info, cd* B, int64_t ldb, int64_t nrhs,
+                      int32_t* rid, const volatile int32_t* cancel, cudaStream_t st);
+mw_status zlu_upper(int64_t n, const cd* LU, int64_t lda, cd* B, int64_t ldb, int64_t nrhs, cudaStream_t st);
+
+}  // namespace mw
