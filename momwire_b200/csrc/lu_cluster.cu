@@ -871,6 +871,37 @@ mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas
 }
 
 // ------------------------------------------------------------------ driver
+// Keeps the host at most kDepth blocks ahead of the device, so that a
+// cancellation flag polled before each block is seen while the device still
+// works (the whole factorisation is enqueued in about two milliseconds).
+class Pace {
+  public:
+    static constexpr int kDepth = 4;
+    mw_status start(cudaStream_t st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        MW_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
+        if (cap != cudaStreamCaptureStatusNone) return MW_OK;  // nothing runs yet
+        for (auto& e : ev_) MW_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        on_ = true;
+        return MW_OK;
+    }
+    mw_status step(int64_t j, cudaStream_t st) {
+        if (!on_) return MW_OK;
+        cudaEvent_t e = ev_[j % kDepth];
+        if (j >= kDepth) MW_CHECK_CUDA(cudaEventSynchronize(e));
+        MW_CHECK_CUDA(cudaEventRecord(e, st));
+        return MW_OK;
+    }
+    ~Pace() {
+        for (auto e : ev_)
+            if (e) cudaEventDestroy(e);
+    }
+
+  private:
+    cudaEvent_t ev_[kDepth] = {};
+    bool on_ = false;
+};
+
 // Blocked factorisation of the whole matrix with nrhs carried columns (B <-
 // L^-1 P B).  `rid`: n + 2 kZluBlock ints of workspace.  One stream: the
 // block's cluster leaves 132 SMs idle, but its chain is short beside the
@@ -879,7 +910,16 @@ mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas
 mw_status zlu_blocked(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* info, cd* B, int64_t ldb, int64_t nrhs,
                       int32_t* rid, const volatile int32_t* cancel, cudaStream_t st) {
     const int nb = kZluBlock;
+    Pace pace;
+    if (cancel) {
+        mw_status s = pace.start(st);
+        if (s != MW_OK) return s;
+    }
     for (int64_t j0 = 0; j0 < n; j0 += nb) {
+        if (cancel) {
+            mw_status s = pace.step(j0 / nb, st);
+            if (s != MW_OK) return s;
+        }
         if (cancel && *cancel) {
             MW_CHECK_CUDA(cudaStreamSynchronize(st));
             set_error("factorisation cancelled");
