@@ -4,20 +4,20 @@
 // _bspline_kernels.py's moment integrals and _accelerators.cpp's assembly.
 // Design (B200-first, not a port):
 //   * one CTA owns a tile of up to 16 x 16 basis pairs; the segments its
-//     bases touch (<= 24 per side) are staged in shared memory together with
-//     their Gauss points and weight-folded monomials;
-//   * phase A computes the (d+1)^2 moments of every touched segment pair
-//     straight into shared memory -- four lanes per pair, one source-side
-//     quadrature row each, reduced with warp shuffles; same-edge pairs read
-//     the analytic static + smooth Toeplitz table instead;
-//   * phase B contracts moments with the basis polynomials into Z and
-//     writes the tile column-major with coalesced stores (optionally a
-//     complex64 copy for the mixed-precision factorisation).
+//     bases touch (<= 24 per side) are staged in shared memory as their Gauss
+//     points with weight-folded monomials;
+//   * phase A computes the (d+1)^2 moments of every touched segment pair, one
+//     thread each, straight into shared memory; same-edge pairs read the
+//     analytic static + smooth Toeplitz table instead;
+//   * phase B contracts moments with the basis polynomials into Z (source
+//     side, then observer side) and writes the tile column-major (optionally
+//     a complex64 copy for the mixed-precision factorisation).
+// The arithmetic of both phases is in pair_moments.cuh.
 // The (d+1)^2 x N^2 moment tensor of the reference never exists.
 #include <cstdio>
 
 #include "common.cuh"
-#include "ground_weights.cuh"
+#include "pair_moments.cuh"
 
 namespace mw {
 
@@ -267,163 +267,6 @@ __global__ void __launch_bounds__(kTableThreads) same_edge_table_kernel(
 }
 
 // --------------------------------------------------------------------------
-// Pair moments (shared by the fused fill and the standalone moment kernel)
-// --------------------------------------------------------------------------
-
-// Per-segment staged data: Gauss points (3 nq), weight-folded powers
-// w_q L (u_q)^p (nq*(D+1)), tangent, centre, radius.
-template <int D>
-struct SegStage {
-    static constexpr int NM = D + 1;
-    __device__ static int stride(int nq) { return nq * 3 + nq * NM + 7; }
-};
-
-template <int D>
-__device__ __forceinline__ void stage_segment(double* dst, int nq, const GLParams& gl,
-                                              const double* sl, const double* sr, const double* tg,
-                                              double a, bool mirror, double gz) {
-    constexpr int NM = D + 1;
-    double l0 = sl[0], l1 = sl[1], l2 = sl[2];
-    double r0 = sr[0], r1 = sr[1], r2 = sr[2];
-    double dx = r0 - l0, dy = r1 - l1, dz = r2 - l2;
-    double L = sqrt(dx * dx + dy * dy + dz * dz);
-    for (int q = 0; q < nq; ++q) {
-        double t = gl.t[q];
-        double px = (1.0 - t) * l0 + t * r0;
-        double py = (1.0 - t) * l1 + t * r1;
-        double pz = (1.0 - t) * l2 + t * r2;
-        if (mirror) pz = 2.0 * gz - pz;
-        dst[q * 3 + 0] = px;
-        dst[q * 3 + 1] = py;
-        dst[q * 3 + 2] = pz;
-        double u = t * L, wp = gl.w[q] * L;
-        for (int p = 0; p < NM; ++p) {
-            dst[nq * 3 + q * NM + p] = wp;
-            wp *= u;
-        }
-    }
-    int o = nq * 3 + nq * NM;
-    dst[o + 0] = tg[0];
-    dst[o + 1] = tg[1];
-    dst[o + 2] = mirror ? -tg[2] : tg[2];
-    double cz = 0.5 * (l2 + r2);
-    dst[o + 3] = 0.5 * (l0 + r0);
-    dst[o + 4] = 0.5 * (l1 + r1);
-    dst[o + 5] = mirror ? 2.0 * gz - cz : cz;
-    dst[o + 6] = a;
-}
-
-// sin x and cos x for |x| <= kPhaseStepMax from their Taylor series through
-// x^17 and x^16 (Horner in x^2; coefficients 1/n!).  At |x| = 0.75 the first
-// omitted terms, x^19/19! and x^18/18!, are below 1e-18: full double
-// precision.
-constexpr double kPhaseStepMax = 0.75;
-__device__ __forceinline__ void phase_step(double x, double* sx, double* cx) {
-    const double t = x * x;
-    double c = 1.0 / 20922789888000.0;  // 1/16!
-    c = fma(c, t, -1.0 / 87178291200.0);
-    c = fma(c, t, 1.0 / 479001600.0);
-    c = fma(c, t, -1.0 / 3628800.0);
-    c = fma(c, t, 1.0 / 40320.0);
-    c = fma(c, t, -1.0 / 720.0);
-    c = fma(c, t, 1.0 / 24.0);
-    c = fma(c, t, -0.5);
-    *cx = fma(c, t, 1.0);
-    double s = 1.0 / 355687428096000.0;  // 1/17!
-    s = fma(s, t, -1.0 / 1307674368000.0);
-    s = fma(s, t, 1.0 / 6227020800.0);
-    s = fma(s, t, -1.0 / 39916800.0);
-    s = fma(s, t, 1.0 / 362880.0);
-    s = fma(s, t, -1.0 / 5040.0);
-    s = fma(s, t, 1.0 / 120.0);
-    s = fma(s, t, -1.0 / 6.0);
-    *sx = fma(s * t, x, x);
-}
-
-// Lane `qi` of a pair computes its observer quadrature row and returns its
-// share of all (D+1)^2 moments; the caller reduces the shares over lanes.
-// NQ > 0: the quadrature order is known at compile time (nq == NQ), so the
-// source-point loop unrolls and its independent samples interleave.
-template <int D, bool EK, int NQ = 0>
-__device__ __forceinline__ void pair_row(const double* si, const double* sj, int nq_rt, int qi,
-                                         double k, bool ek_on, cd Jp[D + 1][D + 1]) {
-    constexpr int NM = D + 1;
-    const int nq = NQ > 0 ? NQ : nq_rt;
-#pragma unroll
-    for (int p = 0; p < NM; ++p)
-#pragma unroll
-        for (int P = 0; P < NM; ++P) Jp[p][P] = cd{0.0, 0.0};
-    if (qi >= nq) return;
-    double a = si[nq * 3 + nq * NM + 6];
-    double a2 = a * a;
-    double xi = si[qi * 3 + 0], yi = si[qi * 3 + 1], zi = si[qi * 3 + 2];
-    cd accP[NM];
-#pragma unroll
-    for (int P = 0; P < NM; ++P) accP[P] = cd{0.0, 0.0};
-    const double* wv = sj + nq * 3;
-    double R0 = 0.0, s0 = 0.0, c0 = 1.0;
-#pragma unroll
-    for (int r = 0; r < (NQ > 0 ? NQ : 8); ++r) {
-        if (NQ == 0 && r >= nq) break;
-        double dx = xi - sj[r * 3 + 0];
-        double dy = yi - sj[r * 3 + 1];
-        double dz = zi - sj[r * 3 + 2];
-        double R2 = dx * dx + dy * dy + dz * dz + a2;
-        // one reciprocal square root serves both R and 1/R
-        double iR = rsqrt(R2);
-        double R = R2 * iR;
-        double s, c;
-        // the first source point's phase in full; the others rotate it by
-        // k (R - R0), at most k times a segment length, through that angle's
-        // Taylor series (phase_step) -- a full sincos where it is wider
-        const double x = k * (R - R0);
-        if (r == 0 || fabs(x) > kPhaseStepMax) {
-            sincos(k * R, &s, &c);
-            if (r == 0) {
-                R0 = R;
-                s0 = s;
-                c0 = c;
-            }
-        } else {
-            double sx, cx;
-            phase_step(x, &sx, &cx);
-            s = s0 * cx + c0 * sx;
-            c = c0 * cx - s0 * sx;
-        }
-        double g = kInv4Pi * iR;
-        cd G = cd{c * g, -s * g};
-        if (EK && ek_on) G = G * ek_factor(R, a, k);
-#pragma unroll
-        for (int P = 0; P < NM; ++P) {
-            double w = wv[r * NM + P];
-            accP[P].re += w * G.re;
-            accP[P].im += w * G.im;
-        }
-    }
-    const double* wu = si + nq * 3 + qi * NM;
-#pragma unroll
-    for (int p = 0; p < NM; ++p) {
-        double w = wu[p];
-#pragma unroll
-        for (int P = 0; P < NM; ++P) Jp[p][P] = cd{w * accP[P].re, w * accP[P].im};
-    }
-}
-
-template <int D>
-__device__ __forceinline__ void reduce4(cd Jp[D + 1][D + 1]) {
-#pragma unroll
-    for (int p = 0; p <= D; ++p)
-#pragma unroll
-        for (int P = 0; P <= D; ++P) {
-#pragma unroll
-            for (int off = 1; off < 4; off <<= 1) {
-                Jp[p][P].re += __shfl_xor_sync(0xffffffffu, Jp[p][P].re, off);
-                Jp[p][P].im += __shfl_xor_sync(0xffffffffu, Jp[p][P].im, off);
-            }
-        }
-}
-
-// --------------------------------------------------------------------------
 // Fused fill kernel
 // --------------------------------------------------------------------------
 
@@ -447,17 +290,37 @@ struct FillArgs {
     int nbatch;
 };
 
+// Column bases per contraction round: half a tile, so that three blocks'
+// shared memory fits an SM.
+constexpr int kFillCols = MW_MAX_TILE_BASIS / 2;
+
+// Shared memory of a tile pair, in elements.
+template <int D, bool IMAGE>
+struct FillSmem {
+    static constexpr int NM = D + 1;
+    size_t nJ, nT, nW, bytes;
+    __host__ __device__ FillSmem(int nq, int smax, int tb) {
+        const size_t pairs = (size_t)smax * smax;
+        nJ = pairs * NM * NM;
+        nT = (size_t)(NM + D) * smax * (kFillCols + 1);
+        nW = IMAGE ? pairs * 2 : 0;
+        bytes = (nJ + nT + nW) * sizeof(cd) +
+                ((size_t)2 * smax * seg_stride<D>(nq) + (size_t)2 * tb * NM * NM) * sizeof(double) +
+                ((size_t)6 * smax + (size_t)2 * tb * NM) * sizeof(int);
+    }
+};
+
 // One (row tile, column tile) block of Z.  With allow_mirror the tile pair
 // is checked for symmetry (every staged segment of both tiles has the same
 // radius: the thin-wire kernel uses the observer radius, so only then is the
 // Galerkin block of (tc, tr) the transpose of that of (tr, tc)); a symmetric
 // pair also writes the transposed block.  Returns whether it did.
-template <int D, bool IMAGE, bool EK>
+template <int D, bool IMAGE, bool EK, int NT>
 __device__ __forceinline__ bool fill_tile(const FillArgs& A, const GLParams& gl, double* smem, const int tr,
                                           const int tc, const bool allow_mirror) {
     constexpr int NM = D + 1, NMM = NM * NM;
     const int nq = gl.nq;
-    const int SD = SegStage<D>::stride(nq);
+    const int SD = seg_stride<D>(nq);
     const int SMAX = A.basis.max_tile_seg;
     const int TB = A.basis.max_tile_basis;
     const int ns_r = A.basis.tile_ns[tr], ns_c = A.basis.tile_ns[tc];
@@ -471,17 +334,15 @@ __device__ __forceinline__ bool fill_tile(const FillArgs& A, const GLParams& gl,
     double* Zb = A.Z + 2 * bz * A.z_stride;
     float* Z32b = A.Z32 ? A.Z32 + 2 * bz * A.z32_stride : nullptr;
 
-    double* s_row = smem;                               // SMAX * SD
-    double* s_col = s_row + SMAX * SD;                  // SMAX * SD
-    double* s_J = s_col + SMAX * SD;                    // SMAX*SMAX*NMM*2
-    double* s_W = s_J + (size_t)SMAX * SMAX * NMM * 2;  // image: SMAX*SMAX*4
-    double* s_pr = s_W + (IMAGE ? (size_t)SMAX * SMAX * 4 : 0);  // TB*NMM
-    double* s_pc = s_pr + TB * NMM;                     // TB*NMM
-    double* s_out = s_pc + TB * NMM;                    // TB*TB*2 (mirrored block)
-    int* s_int = reinterpret_cast<int*>(s_out + TB * TB * 2);
-    int* s_seg_r = s_int;               // SMAX
-    int* s_seg_c = s_seg_r + SMAX;      // SMAX
-    int* s_edge_r = s_seg_c + SMAX;     // SMAX
+    const FillSmem<D, IMAGE> lay(nq, SMAX, TB);
+    cd* s_J = reinterpret_cast<cd*>(smem);            // SMAX*SMAX*NMM moments
+    cd* s_T = s_J + lay.nJ;                           // stage 1: (NM + D) planes of SMAX x (kFillCols + 1)
+    cd* s_W = s_T + lay.nT;                           // image: the pairs' weights, 2 each
+    double* s_row = reinterpret_cast<double*>(s_W + lay.nW);  // SMAX * SD
+    double* s_col = s_row + SMAX * SD;                // SMAX * SD
+    double* s_pr = s_col + SMAX * SD;                 // TB*NMM
+    double* s_pc = s_pr + TB * NMM;                   // TB*NMM
+    int* s_edge_r = reinterpret_cast<int*>(s_pc + TB * NMM);  // SMAX each
     int* s_edge_c = s_edge_r + SMAX;
     int* s_pos_r = s_edge_c + SMAX;
     int* s_pos_c = s_pos_r + SMAX;
@@ -493,101 +354,66 @@ __device__ __forceinline__ bool fill_tile(const FillArgs& A, const GLParams& gl,
     const int tid = threadIdx.x;
     const double gz = A.ground.ground_z;
 
-    // ---- staging: segment lists, Gauss points, basis polynomials
+    // ---- staging: a thread per segment node, basis tables
     const double r_ref = A.seg.radius[A.basis.tile_seg[(size_t)tr * SMAX]];
     int odd_radius = 0;
-    for (int i = tid; i < ns_r; i += blockDim.x) {
-        int s = A.basis.tile_seg[(size_t)tr * SMAX + i];
-        odd_radius |= A.seg.radius[s] != r_ref;
-        s_seg_r[i] = s;
-        s_edge_r[i] = A.seg.edge[s];
-        s_pos_r[i] = A.seg.pos_in_edge[s];
-        s_grp_r[i] = EK ? A.seg.ek_group[s] : 0;
-        stage_segment<D>(s_row + i * SD, nq, gl, A.seg.seg_l + 3 * s, A.seg.seg_r + 3 * s,
-                         A.seg.tangent + 3 * s, A.seg.radius[s], false, 0.0);
+    for (int e = tid; e < (ns_r + ns_c) * nq; e += NT) {
+        const int g = e / nq, q = e - g * nq;
+        const bool c = g >= ns_r;
+        const int i = c ? g - ns_r : g;
+        const int s = A.basis.tile_seg[(size_t)(c ? tc : tr) * SMAX + i];
+        const double a = A.seg.radius[s];
+        stage_node<D>((c ? s_col : s_row) + i * SD, nq, q, gl.t, gl.w, A.seg.seg_l + 3 * s, A.seg.seg_r + 3 * s,
+                      A.seg.tangent + 3 * s, a, IMAGE && c, gz);
+        if (q == 0) {
+            odd_radius |= a != r_ref;
+            (c ? s_edge_c : s_edge_r)[i] = A.seg.edge[s];
+            (c ? s_pos_c : s_pos_r)[i] = A.seg.pos_in_edge[s];
+            (c ? s_grp_c : s_grp_r)[i] = EK ? (IMAGE && c ? A.seg.ek_group_img[s] : A.seg.ek_group[s]) : 0;
+        }
     }
-    for (int i = tid; i < ns_c; i += blockDim.x) {
-        int s = A.basis.tile_seg[(size_t)tc * SMAX + i];
-        odd_radius |= A.seg.radius[s] != r_ref;
-        s_seg_c[i] = s;
-        s_edge_c[i] = A.seg.edge[s];
-        s_pos_c[i] = A.seg.pos_in_edge[s];
-        s_grp_c[i] = EK ? (IMAGE ? A.seg.ek_group_img[s] : A.seg.ek_group[s]) : 0;
-        stage_segment<D>(s_col + i * SD, nq, gl, A.seg.seg_l + 3 * s, A.seg.seg_r + 3 * s,
-                         A.seg.tangent + 3 * s, A.seg.radius[s], IMAGE, gz);
-    }
-    for (int i = tid; i < nb_r * NMM; i += blockDim.x)
+    for (int i = tid; i < nb_r * NMM; i += NT)
         s_pr[i] = A.basis.polys[(size_t)fb_r * NMM + i];
-    for (int i = tid; i < nb_c * NMM; i += blockDim.x)
+    for (int i = tid; i < nb_c * NMM; i += NT)
         s_pc[i] = A.basis.polys[(size_t)fb_c * NMM + i];
-    for (int i = tid; i < nb_r * NM; i += blockDim.x) s_loc_r[i] = A.basis.loc[(size_t)fb_r * NM + i];
-    for (int i = tid; i < nb_c * NM; i += blockDim.x) s_loc_c[i] = A.basis.loc[(size_t)fb_c * NM + i];
+    for (int i = tid; i < nb_r * NM; i += NT) s_loc_r[i] = A.basis.loc[(size_t)fb_r * NM + i];
+    for (int i = tid; i < nb_c * NM; i += NT) s_loc_c[i] = A.basis.loc[(size_t)fb_c * NM + i];
     const bool mirror = __syncthreads_or(odd_radius) == 0 && allow_mirror;
 
-    // ---- phase A: moments of every staged segment pair (4 lanes per pair)
+    // ---- phase A: moments of every staged segment pair, one thread each
     const int npair = ns_r * ns_c;
-    const int lane4 = tid & 3;
-    const int ngroups = blockDim.x >> 2;
-    const int rounds = (npair + ngroups - 1) / ngroups;
-    for (int rd = 0; rd < rounds; ++rd) {
-        int pidx = rd * ngroups + (tid >> 2);
-        bool valid = pidx < npair;
-        int li = valid ? pidx / ns_c : 0;
-        int lj = valid ? pidx - li * ns_c : 0;
-        bool same_edge = !IMAGE && valid && s_edge_r[li] == s_edge_c[lj];
-        cd Jp[NM][NM];
-        // every lane of the warp joins the shuffles; invalid/same-edge
-        // groups contribute zeros
-        if (valid && !same_edge) {
-            bool ek_on = EK && (s_grp_r[li] == s_grp_c[lj]);
-            if (nq == 4) {
-                // the default rule: one observer point per lane
-                pair_row<D, EK, 4>(s_row + li * SD, s_col + lj * SD, 4, lane4, kz, ek_on, Jp);
-            } else {
-                cd Jt[NM][NM];
-                pair_row<D, EK>(s_row + li * SD, s_col + lj * SD, nq, lane4, kz, ek_on, Jt);
-                cd Jt2[NM][NM];
-                pair_row<D, EK>(s_row + li * SD, s_col + lj * SD, nq, lane4 + 4, kz, ek_on, Jt2);
-#pragma unroll
-                for (int p = 0; p < NM; ++p)
-#pragma unroll
-                    for (int P = 0; P < NM; ++P) Jp[p][P] = Jt[p][P] + Jt2[p][P];
-            }
-        } else {
-#pragma unroll
-            for (int p = 0; p < NM; ++p)
-#pragma unroll
-                for (int P = 0; P < NM; ++P) Jp[p][P] = cd{0.0, 0.0};
-        }
-        reduce4<D>(Jp);
+    for (int p0 = 0; p0 < npair; p0 += NT) {
+        const int pidx = p0 + tid;
+        const bool valid = pidx < npair;
+        const int li = valid ? pidx / ns_c : 0;
+        const int lj = valid ? pidx - li * ns_c : 0;
+        const bool same_edge = !IMAGE && valid && s_edge_r[li] == s_edge_c[lj];
+        const double* si = s_row + li * SD;
+        const double* sj = s_col + lj * SD;
+        const double* ti = seg_tail<D>(si, nq);
+        const double a2 = ti[6];
+        const double ek_a = EK && s_grp_r[li] == s_grp_c[lj] ? sqrt(a2) : 0.0;
+        cd* dst = s_J + (size_t)(valid ? pidx : 0) * NMM;
+        pair_moments_any<D, EK>(si, sj, nq, kz, a2, ek_a, valid && !same_edge, dst);
         if (valid) {
-            double* dst = s_J + (size_t)pidx * NMM * 2;
             if (same_edge) {
-                if (lane4 == 0) {
-                    int e = s_edge_r[li];
-                    int64_t row = A.e_off[e] + (s_pos_c[lj] - s_pos_r[li]) + A.e_n[e] - 1;
-                    const double* src = table + row * NMM * 2;
+                const int e = s_edge_r[li];
+                const int64_t row = A.e_off[e] + (s_pos_c[lj] - s_pos_r[li]) + A.e_n[e] - 1;
+                const double2* src = reinterpret_cast<const double2*>(table) + row * NMM;
 #pragma unroll
-                    for (int x = 0; x < NMM * 2; ++x) dst[x] = src[x];
+                for (int x = 0; x < NMM; ++x) {
+                    const double2 v = src[x];
+                    dst[x] = cd{v.x, v.y};
                 }
-            } else if (lane4 == 0) {
-#pragma unroll
-                for (int p = 0; p < NM; ++p)
-#pragma unroll
-                    for (int P = 0; P < NM; ++P) {
-                        dst[(p * NM + P) * 2 + 0] = Jp[p][P].re;
-                        dst[(p * NM + P) * 2 + 1] = Jp[p][P].im;
-                    }
             }
-            if (IMAGE && lane4 == 1) {
+            if (IMAGE) {
                 // per-pair image weights
-                const double* si = s_row + li * SD + nq * 3 + nq * NM;
-                const double* sj = s_col + lj * SD + nq * 3 + nq * NM;
+                const double* tj = seg_tail<D>(sj, nq);
                 cd wA, wP;
                 if (A.ground.model == MW_GROUND_REFL) {
-                    refl_weights(si + 3, si, sj + 3, sj, A.ground, &wA, &wP);
+                    refl_weights(ti + 3, ti, tj + 3, tj, A.ground, &wA, &wP);
                 } else {
-                    double td = si[0] * sj[0] + si[1] * sj[1] + si[2] * sj[2];
+                    const double td = ti[0] * tj[0] + ti[1] * tj[1] + ti[2] * tj[2];
                     if (A.ground.model == MW_GROUND_SOMM_IMAGE) {
                         cd et{A.ground.eps_re, A.ground.eps_im};
                         cd c2 = cdiv(cd{et.re - 1.0, et.im}, cd{et.re + 1.0, et.im});
@@ -598,114 +424,74 @@ __device__ __forceinline__ bool fill_tile(const FillArgs& A, const GLParams& gl,
                         wP = cd{1.0, 0.0};
                     }
                 }
-                double* w = s_W + (size_t)pidx * 4;
-                w[0] = wA.re; w[1] = wA.im; w[2] = wP.re; w[3] = wP.im;
+                s_W[2 * pidx] = wA;
+                s_W[2 * pidx + 1] = wP;
             }
         }
     }
     __syncthreads();
 
-    // ---- phase B: Galerkin contraction into the Z tile
+    // ---- phase B: Galerkin contraction, source side then observer side,
+    // kFillCols column bases at a time
+    constexpr int pitch = kFillCols + 1;
+    const int plane = SMAX * pitch;
+    cd* TQ = s_T + NM * plane;
     const double wmu = omz * A.mu0;
     const double inv_weps = 1.0 / (omz * A.eps0);
-    for (int pp = tid; pp < TB * TB; pp += blockDim.x) {
-        int mi = pp % TB, ni = pp / TB;
-        if (mi >= nb_r || ni >= nb_c) continue;
-        cd zA{0.0, 0.0}, zP{0.0, 0.0};
-        const double* Cm = s_pr + mi * NMM;
-        const double* Cn = s_pc + ni * NMM;
-        for (int a = 0; a < NM; ++a) {
-            int la = s_loc_r[mi * NM + a];
-            if (la < 0) continue;
-            for (int b = 0; b < NM; ++b) {
-                int lb = s_loc_c[ni * NM + b];
-                if (lb < 0) continue;
-                const double* J = s_J + ((size_t)la * ns_c + lb) * NMM * 2;
-                cd inA{0.0, 0.0}, inP{0.0, 0.0};
-#pragma unroll
-                for (int p = 0; p < NM; ++p) {
-                    cd rowA{0.0, 0.0};
-#pragma unroll
-                    for (int P = 0; P < NM; ++P) {
-                        double c = Cn[b * NM + P];
-                        rowA.re += c * J[(p * NM + P) * 2 + 0];
-                        rowA.im += c * J[(p * NM + P) * 2 + 1];
-                    }
-                    double cm = Cm[a * NM + p];
-                    inA.re += cm * rowA.re;
-                    inA.im += cm * rowA.im;
-                }
-#pragma unroll
-                for (int p = 1; p < NM; ++p) {
-                    cd rowP{0.0, 0.0};
-#pragma unroll
-                    for (int P = 1; P < NM; ++P) {
-                        double c = P * Cn[b * NM + P];
-                        rowP.re += c * J[((p - 1) * NM + (P - 1)) * 2 + 0];
-                        rowP.im += c * J[((p - 1) * NM + (P - 1)) * 2 + 1];
-                    }
-                    double cm = p * Cm[a * NM + p];
-                    inP.re += cm * rowP.re;
-                    inP.im += cm * rowP.im;
-                }
-                if (IMAGE) {
-                    const double* w = s_W + ((size_t)la * ns_c + lb) * 4;
-                    zA = zA + cd{w[0], w[1]} * inA;
-                    zP = zP + cd{w[2], w[3]} * inP;
-                } else {
-                    const double* ti = s_row + la * SD + nq * 3 + nq * NM;
-                    const double* tj = s_col + lb * SD + nq * 3 + nq * NM;
-                    double td = ti[0] * tj[0] + ti[1] * tj[1] + ti[2] * tj[2];
-                    zA.re += td * inA.re;
-                    zA.im += td * inA.im;
-                    zP = zP + inP;
-                }
+    // into Z[m, n]: the value, or under a ground what the image term leaves
+    auto put = [&](int64_t m, int64_t n, double zre, double zim) {
+        double2* zp = reinterpret_cast<double2*>(Zb + m * 2 + n * A.ldz * 2);
+        if (IMAGE) {
+            const double2 z = *zp;
+            zre = z.x - zre;
+            zim = z.y - zim;
+        }
+        *zp = make_double2(zre, zim);
+        if (Z32b) *reinterpret_cast<float2*>(Z32b + m * 2 + n * A.ldz32 * 2) = make_float2((float)zre, (float)zim);
+    };
+    for (int n0 = 0; n0 < nb_c; n0 += kFillCols) {
+        const int nc = min(kFillCols, nb_c - n0);
+        for (int it = tid; it < ns_r * kFillCols; it += NT) {
+            const int la = it / kFillCols, nl = it % kFillCols, ni = n0 + nl;
+            if (nl >= nc) continue;
+            const double* ti = seg_tail<D>(s_row + la * SD, nq);
+            cd a[NM], q[D];
+            const cd* J0 = s_J + (size_t)la * ns_c * NMM;
+            if constexpr (IMAGE) {
+                contract_source<D>(J0, s_loc_c + ni * NM, s_pc + ni * NMM,
+                                   [&](int lb) {
+                                       return ComplexWeight{s_W[2 * (la * ns_c + lb)], s_W[2 * (la * ns_c + lb) + 1]};
+                                   },
+                                   a, q);
+            } else {
+                contract_source<D>(J0, s_loc_c + ni * NM, s_pc + ni * NMM,
+                                   [&](int lb) {
+                                       const double* tj = seg_tail<D>(s_col + lb * SD, nq);
+                                       return RealWeight{ti[0] * tj[0] + ti[1] * tj[1] + ti[2] * tj[2]};
+                                   },
+                                   a, q);
             }
+#pragma unroll
+            for (int p = 0; p < NM; ++p) s_T[p * plane + la * pitch + nl] = a[p];
+#pragma unroll
+            for (int p = 0; p < D; ++p) TQ[p * plane + la * pitch + nl] = q[p];
         }
-        // j w mu zA + zP / (j w eps)
-        double zre = -wmu * zA.im + inv_weps * zP.im;
-        double zim = wmu * zA.re - inv_weps * zP.re;
-        if (mirror) {
-            s_out[(mi * TB + ni) * 2 + 0] = zre;
-            s_out[(mi * TB + ni) * 2 + 1] = zim;
+        __syncthreads();
+        // column-major Z: the row basis fastest
+        for (int pp = tid; pp < TB * kFillCols; pp += NT) {
+            const int mi = pp % TB, nl = pp / TB;
+            if (mi >= nb_r || nl >= nc) continue;
+            cd zA, zP;
+            contract_observer<D>(s_T + nl, TQ + nl, pitch, plane, s_loc_r + mi * NM, s_pr + mi * NMM, &zA, &zP);
+            // j w mu zA + zP / (j w eps)
+            const double zre = -wmu * zA.im + inv_weps * zP.im, zim = wmu * zA.re - inv_weps * zP.re;
+            put(fb_r + mi, fb_c + n0 + nl, zre, zim);
+            // the transposed block: 128-byte runs of the column bases
+            if (mirror) put(fb_c + n0 + nl, fb_r + mi, zre, zim);
         }
-        int64_t m = fb_r + mi, n = fb_c + ni;
-        double* zp = Zb + m * 2 + n * A.ldz * 2;
-        if (IMAGE) {
-            zre = zp[0] - zre;
-            zim = zp[1] - zim;
-        }
-        zp[0] = zre;
-        zp[1] = zim;
-        if (Z32b) {
-            float* z32 = Z32b + m * 2 + n * A.ldz32 * 2;
-            z32[0] = (float)zre;
-            z32[1] = (float)zim;
-        }
+        if (n0 + kFillCols < nb_c) __syncthreads();
     }
-    if (!mirror) return false;
-    __syncthreads();
-    // the transposed block Z[n, m], column tile index fastest (coalesced)
-    for (int pp = tid; pp < TB * TB; pp += blockDim.x) {
-        int ni = pp % TB, mi = pp / TB;
-        if (mi >= nb_r || ni >= nb_c) continue;
-        double zre = s_out[(mi * TB + ni) * 2 + 0];
-        double zim = s_out[(mi * TB + ni) * 2 + 1];
-        int64_t m = fb_r + mi, n = fb_c + ni;
-        double* zp = Zb + n * 2 + m * A.ldz * 2;
-        if (IMAGE) {
-            zre = zp[0] - zre;
-            zim = zp[1] - zim;
-        }
-        zp[0] = zre;
-        zp[1] = zim;
-        if (Z32b) {
-            float* z32 = Z32b + n * 2 + m * A.ldz32 * 2;
-            z32[0] = (float)zre;
-            z32[1] = (float)zim;
-        }
-    }
-    return true;
+    return mirror;
 }
 
 // Upper-triangle tile pair of block b: tc(tc+1)/2 <= b < (tc+1)(tc+2)/2,
@@ -722,20 +508,26 @@ __device__ __forceinline__ void tri_pair(int64_t b, int& tr, int& tc) {
 // computed once and written to both blocks of Z; otherwise the block also
 // computes (tc, tr) itself.  The EK image fill labels direct and mirrored
 // segments separately, so it always computes both.
-#ifndef MW_FILL_MIN_BLOCKS
-#define MW_FILL_MIN_BLOCKS 3  // resident CTAs per SM the register allocation must allow
-#endif
-
-template <int D, bool IMAGE, bool EK>
-__global__ void __launch_bounds__(256, MW_FILL_MIN_BLOCKS) fill_kernel(FillArgs A, GLParams gl) {
-    extern __shared__ double smem[];
+//
+// What bounds it: the FP64 pipe in phase A, latency in staging and phase B,
+// so the blocks of an SM must be in different phases.  A block is NT threads,
+// as many blocks as shared memory lets share an SM, and twelve (or eleven)
+// warps at 168 registers in all: the samples need those, and spilling them
+// for more warps loses more than it hides (18 warps at 96: 9.7 ms).
+// Measured on B200, fill of the 16 x 16 array with its complex64 copy: 13.3
+// ms with four lanes per pair and 256 threads, 7.6 with one thread per pair
+// and two blocks of 176, 6.7 with three blocks of 128 -- the
+// samples' FP64 operations alone take about 4.
+template <int D, bool IMAGE, bool EK, int NT>
+__global__ void __launch_bounds__(NT, NT == 128 ? 3 : (NT == 192 ? 2 : 1)) fill_kernel(FillArgs A, GLParams gl) {
+    extern __shared__ __align__(16) double smem[];
     int tr, tc;
     tri_pair((int64_t)blockIdx.x, tr, tc);
     const bool off_diag = tr != tc;
-    const bool mirrored = fill_tile<D, IMAGE, EK>(A, gl, smem, tr, tc, off_diag && !(IMAGE && EK));
+    const bool mirrored = fill_tile<D, IMAGE, EK, NT>(A, gl, smem, tr, tc, off_diag && !(IMAGE && EK));
     if (off_diag && !mirrored) {
         __syncthreads();
-        fill_tile<D, IMAGE, EK>(A, gl, smem, tc, tr, false);
+        fill_tile<D, IMAGE, EK, NT>(A, gl, smem, tc, tr, false);
     }
 }
 
@@ -744,68 +536,43 @@ __global__ void __launch_bounds__(256, MW_FILL_MIN_BLOCKS) fill_kernel(FillArgs 
 // --------------------------------------------------------------------------
 
 template <int D>
-__global__ void offedge_moments_kernel(mw_segments si, mw_segments sj, double k, int mirror, double gz,
-                                       const int32_t* gi, const int32_t* gj, GLParams gl,
-                                       double* __restrict__ out) {
+__global__ void __launch_bounds__(128) offedge_moments_kernel(mw_segments si, mw_segments sj, double k, int mirror,
+                                                              double gz, const int32_t* gi, const int32_t* gj,
+                                                              GLParams gl, double* __restrict__ out) {
     constexpr int NM = D + 1;
-    int nq = gl.nq;
-    int64_t pair = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 2;
-    int lane4 = threadIdx.x & 3;
-    int64_t npair = (int64_t)si.n_seg * sj.n_seg;
-    bool valid = pair < npair;
-    int i = valid ? (int)(pair / sj.n_seg) : 0;
-    int j = valid ? (int)(pair - (int64_t)i * sj.n_seg) : 0;
-    double bi[8 * 3 + 8 * NM + 7], bj[8 * 3 + 8 * NM + 7];
-    cd Jp[NM][NM];
-    if (valid) {
-        stage_segment<D>(bi, nq, gl, si.seg_l + 3 * i, si.seg_r + 3 * i, si.tangent + 3 * i,
-                         si.radius[i], false, 0.0);
-        stage_segment<D>(bj, nq, gl, sj.seg_l + 3 * j, sj.seg_r + 3 * j, sj.tangent + 3 * j,
-                         sj.radius[j], mirror != 0, gz);
-        bool ek_on = gi && gj && gi[i] == gj[j];
-        cd J1[NM][NM], J2[NM][NM];
-        if (gi && gj) {
-            pair_row<D, true>(bi, bj, nq, lane4, k, ek_on, J1);
-            pair_row<D, true>(bi, bj, nq, lane4 + 4, k, ek_on, J2);
-        } else {
-            pair_row<D, false>(bi, bj, nq, lane4, k, false, J1);
-            pair_row<D, false>(bi, bj, nq, lane4 + 4, k, false, J2);
+    const int nq = gl.nq;
+    const int64_t pair = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t npair = (int64_t)si.n_seg * sj.n_seg;
+    const bool valid = pair < npair;
+    const int i = valid ? (int)(pair / sj.n_seg) : 0;
+    const int j = valid ? (int)(pair - (int64_t)i * sj.n_seg) : 0;
+    __align__(16) double bi[seg_stride<D>(8)], bj[seg_stride<D>(8)];
+    for (int q = 0; q < nq; ++q) {
+        stage_node<D>(bi, nq, q, gl.t, gl.w, si.seg_l + 3 * i, si.seg_r + 3 * i, si.tangent + 3 * i, si.radius[i],
+                      false, 0.0);
+        stage_node<D>(bj, nq, q, gl.t, gl.w, sj.seg_l + 3 * j, sj.seg_r + 3 * j, sj.tangent + 3 * j, sj.radius[j],
+                      mirror != 0, gz);
+    }
+    const double a2 = seg_tail<D>(bi, nq)[6];
+    cd J[NM * NM];
+    if (gi && gj)
+        pair_moments_any<D, true>(bi, bj, nq, k, a2, valid && gi[i] == gj[j] ? sqrt(a2) : 0.0, valid, J);
+    else
+        pair_moments_any<D, false>(bi, bj, nq, k, a2, 0.0, valid, J);
+    if (!valid) return;
+#pragma unroll
+    for (int p = 0; p < NM; ++p)
+#pragma unroll
+        for (int P = 0; P < NM; ++P) {
+            const size_t o = (((size_t)p * NM + P) * si.n_seg + i) * sj.n_seg + j;
+            out[2 * o + 0] = J[p * NM + P].re;
+            out[2 * o + 1] = J[p * NM + P].im;
         }
-#pragma unroll
-        for (int p = 0; p < NM; ++p)
-#pragma unroll
-            for (int P = 0; P < NM; ++P) Jp[p][P] = J1[p][P] + J2[p][P];
-    } else {
-#pragma unroll
-        for (int p = 0; p < NM; ++p)
-#pragma unroll
-            for (int P = 0; P < NM; ++P) Jp[p][P] = cd{0.0, 0.0};
-    }
-    reduce4<D>(Jp);
-    if (valid && lane4 == 0) {
-#pragma unroll
-        for (int p = 0; p < NM; ++p)
-#pragma unroll
-            for (int P = 0; P < NM; ++P) {
-                size_t o = (((size_t)p * NM + P) * si.n_seg + i) * sj.n_seg + j;
-                out[2 * o + 0] = Jp[p][P].re;
-                out[2 * o + 1] = Jp[p][P].im;
-            }
-    }
 }
 
 // --------------------------------------------------------------------------
 // Host launchers
 // --------------------------------------------------------------------------
-
-static size_t fill_smem_bytes(int D, bool image, int nq, int smax, int tb) {
-    int NM = D + 1, NMM = NM * NM;
-    int SD = nq * 3 + nq * NM + 7;
-    size_t dbl = (size_t)2 * smax * SD + (size_t)smax * smax * NMM * 2 + (image ? (size_t)smax * smax * 4 : 0) +
-                 (size_t)2 * tb * NMM + (size_t)tb * tb * 2;
-    size_t ints = (size_t)8 * smax + (size_t)2 * tb * NM;
-    return dbl * 8 + ints * 4;
-}
 
 // Algorithmic flops of one fill: q^2 * 20 per kernel sample group plus the
 // (d+1)^2 moment FMAs per segment pair, and the Galerkin contraction per
@@ -817,10 +584,19 @@ static double fill_flops(int D, int nq, double n_seg, double n_basis) {
     return n_seg * n_seg * f_pair + n_basis * n_basis * f_basis;
 }
 
+// The block size by the blocks whose shared memory an SM holds (it grows with
+// the square of the largest tile's segment count, 18 for a solver's tiles and
+// at most 24): three blocks of 128 threads, two of 192 (the image fill at
+// degree 2), or one of 352.
+constexpr size_t kFillSmemSM = 227 * 1024;
+
 template <int D, bool IMAGE, bool EK>
 static mw_status launch_fill(const FillArgs& A, const GLParams& gl, cudaStream_t st) {
-    size_t smem = fill_smem_bytes(D, IMAGE, gl.nq, A.basis.max_tile_seg, A.basis.max_tile_basis);
-    auto kern = fill_kernel<D, IMAGE, EK>;
+    const size_t smem = FillSmem<D, IMAGE>(gl.nq, A.basis.max_tile_seg, A.basis.max_tile_basis).bytes;
+    const size_t fit = kFillSmemSM / (smem + 1024);
+    auto kern = fit >= 3 ? fill_kernel<D, IMAGE, EK, 128>
+                         : (fit == 2 ? fill_kernel<D, IMAGE, EK, 192> : fill_kernel<D, IMAGE, EK, 352>);
+    const int threads = fit >= 3 ? 128 : (fit == 2 ? 192 : 352);
     MW_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int nbz = A.nbatch > 0 ? A.nbatch : 1;
     const int64_t nt = A.basis.n_tile;
@@ -831,7 +607,7 @@ static mw_status launch_fill(const FillArgs& A, const GLParams& gl, cudaStream_t
     const double tri = (double)(nt + 1) / (2.0 * (double)nt);
     ProfileScope ps(IMAGE ? PC_FILL_IMAGE : PC_FILL, st, tri * nbz * fill_flops(D, gl.nq, A.seg.n_seg, nb),
                     nbz * nb * nb * (16.0 + (A.Z32 ? 8.0 : 0.0)) * (IMAGE ? 2.0 : 1.0));
-    kern<<<grid, 256, smem, st>>>(A, gl);
+    kern<<<grid, threads, smem, st>>>(A, gl);
     MW_CHECK_CUDA(cudaGetLastError());
     count_launch();
     return MW_OK;
@@ -886,8 +662,8 @@ extern "C" mw_status mw_offedge_moments(const mw_segments* seg_i, const mw_segme
     int64_t npair = (int64_t)seg_i->n_seg * seg_j->n_seg;
     if (npair == 0) return MW_OK;
     GLParams gl = make_gl(n_qp);
-    int threads = 256;
-    int64_t blocks = (npair * 4 + threads - 1) / threads;
+    int threads = 128;
+    int64_t blocks = (npair + threads - 1) / threads;
     cudaStream_t st = as_stream(stream);
     if (degree == 1)
         offedge_moments_kernel<1><<<(unsigned)blocks, threads, 0, st>>>(*seg_i, *seg_j, k, mirror, ground_z,
