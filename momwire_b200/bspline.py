@@ -31,6 +31,7 @@ import numpy as np
 import scipy.sparse
 
 from . import _lib
+from . import _staging
 from . import _tables as T
 from . import _topology as topo
 from . import _validate as V
@@ -170,6 +171,24 @@ class _PackedTables:
         self.rows = rows
         self.meta = (geom.n, len(geom.edge_n), int(geom.edge_n.max()), basis.degree, basis.n, len(tiles.first),
                      tiles.max_basis, tiles.max_seg)
+
+
+class _PortPlan:
+    """The ports and KCL rows of a solver as the device reads them, packed
+    for one upload: the nonzeros of the right-hand sides [B | kcl_con^T]
+    (rows, columns, values), then B^T and kcl_con by rows (row pointers,
+    columns, values each)."""
+
+    def __init__(self, solver):
+        pr, pc, pv, self.n_p = solver._port_entries()
+        kcl = solver._split_kcl_ports(solver._basis().kcl_A)[0].tocoo()
+        self.n_c = kcl.shape[0]
+        kr, kc = kcl.row.astype(np.int64), kcl.col.astype(np.int64)
+        kv = kcl.data.astype(np.complex128)
+        rr, rc, rv = np.concatenate([pr, kc]), np.concatenate([pc, kr + self.n_p]), np.concatenate([pv, kv])
+        self.n_rhs = int(rr.size)
+        self.tables = _staging.Packed(
+            _torch(), [rr, rc, rv, *_csr(pc, pr, pv, self.n_p), *_csr(kr, kc, kv, self.n_c)])
 
 
 class _DeviceTables:
@@ -381,6 +400,7 @@ class BSplineSolver:
         self._cached_dev = None
         self._cached_packed = None
         self._cached_ek = None
+        self._cached_ports = None
         self.last_stats = {}
 
     # ------------------------------------------------------------------ misc
@@ -603,6 +623,16 @@ class BSplineSolver:
         n_p = len(self.feeds) + port_A.shape[0] + gap.shape[1]
         return np.concatenate(rs), np.concatenate(cs), np.concatenate(vs), n_p
 
+    def _port_plan(self) -> _PortPlan:
+        """The packed port tables, built again only when the ports have
+        changed: they depend on the geometry and on these settings, not on
+        the frequency, and building them took longer than a small solve."""
+        key = (tuple(map(tuple, self.feeds)), self.feed_model, self.feed_smoothing_factor, self.n_qp_source,
+               tuple(map(tuple, self.junction_ports)), tuple(map(tuple, self.node_gaps)))
+        if self._cached_ports is None or self._cached_ports[0] != key:
+            self._cached_ports = (key, _PortPlan(self))
+        return self._cached_ports[1]
+
     def _port_count(self):
         return len(self.feeds) + len(self.junction_ports) + len(self.node_gaps)
 
@@ -637,43 +667,14 @@ class BSplineSolver:
         n_poly = self._basis().n
         n = n_poly + (len(enrich) if enrich else 0)
         nm = self.degree + 1
-        # port columns and KCL rows are a few nonzeros each: upload them in
-        # coordinate form and scatter [B | kcl_con^T], B and kcl_con on the
-        # device
-        pr, pc, pv, n_p = self._port_entries()
-        kcl_con = self._split_kcl_ports(self._basis().kcl_A)[0].tocoo()
-        n_c = kcl_con.shape[0]
-        kr, kc = kcl_con.row.astype(np.int64), kcl_con.col.astype(np.int64)
-        kv = kcl_con.data.astype(np.complex128)
-        rr, rc, rv = np.concatenate([pr, kc]), np.concatenate([pc, kr + n_p]), np.concatenate([pv, kv])
-        # CSR of B^T (one row per port) and of kcl_con for the sparse
-        # products Y = B^T X, A Xc and A W
-        bt_ptr, bt_col, bt_val = _csr(pc, pr, pv, n_p)
-        a_ptr, a_col, a_val = _csr(kr, kc, kv, n_c)
-        host = [pr, pc, np.ascontiguousarray(pv).view(np.float64), kr, kc, np.ascontiguousarray(kv).view(np.float64),
-                rr, rc, np.ascontiguousarray(rv).view(np.float64), bt_ptr, bt_col, bt_val.view(np.float64), a_ptr,
-                a_col, a_val.view(np.float64)]
-        # one page-locked staging buffer and one stream-ordered copy for all
-        # of them (each array 256-byte aligned), device views by offset
-        host = [np.ascontiguousarray(a) for a in host]
-        offs, tot = [], 0
-        for a in host:
-            offs.append(tot)
-            tot += (a.nbytes + 255) & ~255
-        stage = torch.empty(max(tot, 256), dtype=torch.uint8, pin_memory=True)
-        sv = stage.numpy()
-        for a, o in zip(host, offs):
-            sv[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
-        dbytes = torch.empty(stage.numel(), dtype=torch.uint8, device=dev)
-        dbytes.copy_(stage, non_blocking=True)
-        tdt = {np.dtype(np.int64): torch.int64, np.dtype(np.float64): torch.float64}
-        ent = [dbytes[o:o + a.nbytes].view(tdt[a.dtype]) for a, o in zip(host, offs)]
+        plan = self._port_plan()
+        n_p, n_c, n_rhs = plan.n_p, plan.n_c, plan.n_rhs
+        dbytes, ent = plan.tables.upload(dev)
         lib = _lib.load()
         st = torch.cuda.current_stream(dev).cuda_stream
         m = n_p + n_c
         rhs0 = torch.empty((max(m, 1), n), dtype=torch.complex128, device=dev)
-        _lib.call("mw_scatter_c128", n, m, rr.size, ent[6].data_ptr(), ent[7].data_ptr(), ent[8].data_ptr(),
-                  rhs0.data_ptr(), st)
+        _lib.call("mw_scatter_c128", n, m, n_rhs, ent[0], ent[1], ent[2], rhs0.data_ptr(), st)
         buf = {
             "n": n,
             "n_poly": n_poly,
@@ -684,13 +685,13 @@ class BSplineSolver:
             "table": torch.empty((max(dt.table_rows, 1), nm, nm), dtype=torch.complex128, device=dev),
             # column-major (n x m) right-hand sides live in an (m, n) tensor
             "RHS0": rhs0,
-            "entries": ent,
+            "entries": ent,  # addresses within ent_buf: see _PortPlan
+            "ent_buf": dbytes,
             "ws": torch.empty(lib.mw_getrf_workspace_size(n), dtype=torch.uint8, device=dev),
             "ipiv": torch.empty(max(n, 1), dtype=torch.int32, device=dev),
             "info": torch.zeros(2, dtype=torch.int32, device=dev),
             "Y": torch.empty((max(n_p, 1), max(n_p, 1)), dtype=torch.complex128, device=dev),
-            "kcl": kcl_con,
-            "_stage": stage,  # the staging buffer lives until the copy has run
+            "plan": plan,
         }
         buf["RHS"] = torch.empty_like(buf["RHS0"])
         if self.precision == "mixed":
@@ -704,7 +705,7 @@ class BSplineSolver:
             buf["ipiv_c"] = torch.empty(n_c, dtype=torch.int32, device=dev)
             buf["info_c"] = torch.zeros(2, dtype=torch.int32, device=dev)
             buf["W"] = torch.empty((max(n_p, 1), n), dtype=torch.complex128, device=dev)
-        buf["h2d_bytes"] = int(sum(a.nbytes for a in host) + dt.h2d_bytes)
+        buf["h2d_bytes"] = int(plan.tables.nbytes + dt.h2d_bytes)
         return buf
 
     def _fill_device(self, buf, stream):
@@ -1017,10 +1018,10 @@ class BSplineSolver:
             # A (the KCL rows, a few +-1 each) applied as a sparse gather
             S, AW = buf["S"], buf["AW"]
             Wd, Xc = X[:n_p], X[n_p:]
-            _lib.call("mw_csr_mm_c128", n_c, n_c, ent[12].data_ptr(), ent[13].data_ptr(), ent[14].data_ptr(),
+            _lib.call("mw_csr_mm_c128", n_c, n_c, ent[6], ent[7], ent[8],
                       Xc.data_ptr(), n, S.data_ptr(), n_c, stream)
             if n_p:
-                _lib.call("mw_csr_mm_c128", n_c, n_p, ent[12].data_ptr(), ent[13].data_ptr(), ent[14].data_ptr(),
+                _lib.call("mw_csr_mm_c128", n_c, n_p, ent[6], ent[7], ent[8],
                           Wd.data_ptr(), n, AW.data_ptr(), n_c, stream)
             self._lu_solve(S, n_c, buf["ws_c"], buf["ipiv_c"], buf["info_c"], AW, n_p, stream)
             W = buf["W"][:n_p]
@@ -1031,7 +1032,7 @@ class BSplineSolver:
             X = W
         if n_p:
             # Y = B^T X with B's few nonzeros per port column
-            _lib.call("mw_csr_mm_c128", n_p, n_p, ent[9].data_ptr(), ent[10].data_ptr(), ent[11].data_ptr(),
+            _lib.call("mw_csr_mm_c128", n_p, n_p, ent[3], ent[4], ent[5],
                       X.data_ptr(), n, buf["Y"].data_ptr(), n_p, stream)
         return X
 
@@ -1103,21 +1104,10 @@ class BSplineSolver:
         # one stream-ordered read-back into page-locked host memory: the
         # coefficients stay column-major (Xh is the transposed view), Y and
         # the status words ride along, then a single stream synchronise
-        dev_stream = torch.cuda.current_stream(buf["Z"].device)
-        hx = torch.empty(X.shape, dtype=X.dtype, pin_memory=True)
-        hx.copy_(X, non_blocking=True)
-        hy = torch.empty((n_p, n_p), dtype=X.dtype, pin_memory=True)
-        if n_p:
-            hy.copy_(buf["Y"][:n_p, :n_p], non_blocking=True)
-        hinfo = [torch.empty(2, dtype=torch.int32, pin_memory=True)
-                 for _ in range(2 if buf["n_c"] else 1)]
-        hinfo[0].copy_(buf["info"][:2], non_blocking=True)
-        if buf["n_c"]:
-            hinfo[1].copy_(buf["info_c"][:2], non_blocking=True)
-        dev_stream.synchronize()
-        Xh = hx.numpy().T
-        Yh = hy.numpy().T
-        self._check_info(buf, [h.numpy() for h in hinfo])
+        want = [X, buf["Y"][:n_p, :n_p], buf["info"]] + ([buf["info_c"]] if buf["n_c"] else [])
+        hx, hy, *hinfo = _staging.read_back(torch, torch.cuda.current_stream(buf["Z"].device), want)
+        Xh, Yh = hx.T, hy.T
+        self._check_info(buf, hinfo)
         self.last_stats = {"h2d_bytes": buf["h2d_bytes"], "d2h_bytes": int(Xh.nbytes + Yh.nbytes + 16)}
         return PortSolution(
             y=Yh,
