@@ -2226,8 +2226,8 @@ static mw_status getrs(int64_t n, int64_t nrhs, const T* LU, int64_t lda, const 
 
 // Orders one cluster factors and solves by itself (lu_cluster.cu); beyond,
 // the blocked factorisation's update on every SM wins.  Measured on B200
-// with 17 right-hand sides: 0.54 ms at 300, 1.49 ms at 640 in one launch;
-// 1.63 against 2.17 ms at 656.
+// with 17 right-hand sides: 0.52 ms at 300, 1.48 ms at 640 in one launch,
+// 2.12 ms at 656 by blocks.
 static int64_t zlu_full_max() { return 640; }
 // A batch fills the device with clusters up to the order its back
 // substitution holds; a few matrices alone follow the rule of one.

@@ -26,11 +26,17 @@
 //           sides, so a small system is factored and solved by one launch.
 // The batch is on the grid: cluster b works on matrix b.
 //
+// Once 256 rows or fewer are left, one CTA factors the panel alone
+// (panel_solo): two CTA barriers a column beat the exchange.
+//
 // Measured on B200 (order 306, one right-hand side): 2.0 ms as a sequence of
-// cooperative panels, swaps, leaves and products, 0.55 ms as one launch; 64
-// such systems 125 ms one after the other, 1.4 ms as one batch.  A column
-// costs about 2,000 cycles: the pivot's pick and reciprocal 600, the next
-// search 200, sending the row 350, the flight (hidden behind the update) 650.
+// cooperative panels, swaps, leaves and products, 0.52 ms as one launch; 64
+// such systems 125 ms one after the other, 0.88 ms as one batch.  A column
+// of the exchange costs about 2,000 cycles, latencies all: the pivot's pick
+// and reciprocal 600, the next search 200, sending the row 400, the flight
+// (the other columns' update runs under it) 650.  512 threads a CTA with one
+// row each measured slower (635 against 522 us at order 300: the update's
+// registers spill), and so did two rows a thread in one CTA (646).
 //
 // The panel slots rotate: column 0 of the register row is always the current
 // pivot column, a step shifts the row left by one and appends the multiplier
@@ -187,6 +193,7 @@ struct Shared {
     cd tri[kW][kW + 1];      // W x W triangle of the solves
     cd dinv[kW];
     cd X[kW][4];  // a solved block of the back substitution
+    cd inv[2];    // one-CTA panel: the pivot's reciprocal
     cd zero;
     union {
         struct {
@@ -196,6 +203,82 @@ struct Shared {
         cd y[kBackRows];
     } u;
 };
+
+// The panel rows [c0, n) x columns [c0, c0 + w) by one CTA (n - c0 <= kCT):
+// ipiv, the factored panel in A at its final positions, S.src, S.disp and
+// S.tri.  As in the exchange below, rows stay in their threads and the
+// register slots rotate.
+__device__ __forceinline__ void panel_solo(Shared& S, cd* A, int64_t lda, int32_t* ipiv, int32_t* info, int n, int c0,
+                                           int w) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cnt = n - c0, nw = min(kCWarps, (cnt + 31) / 32);  // warps that hold rows
+    if (warp >= nw) return;
+    cd a[kW];
+    unsigned pos = tid < cnt ? (unsigned)(c0 + tid) : kNone;  // the row's position; kNone: none, or a pivot already
+#pragma unroll
+    for (int x = 0; x < kW; ++x)
+        a[x] = tid < cnt && x < w ? ld2(A + (c0 + tid) + (int64_t)(c0 + x) * lda) : cd{0.0, 0.0};
+    unsigned tpos = (unsigned)(c0 + lane);  // lane i: position of row c0 + i
+    for (int jj = 0; jj < w; ++jj) {
+        const int par = jj & 1;
+        const unsigned c = (unsigned)(c0 + jj);
+        // the lane that holds the warp's candidate, then the pivot
+        const cd z = a[0];
+        const unsigned long long bb = (unsigned long long)__double_as_longlong(cabs1(z));
+        const unsigned bhi = (unsigned)(bb >> 32), blo = (unsigned)bb;
+        const unsigned mh = __reduce_max_sync(0xffffffffu, pos == kNone ? 0u : bhi);
+        const cd binv = recip_fast(z);  // (in the shadow of the reduction)
+        const int wsrc = warp_pick(mh, bhi, blo, pos);
+        int g = wsrc;
+        uint4 k = make_uint4(bhi, blo, pos, (unsigned)(c0 + tid));
+        bool mine = lane == wsrc;
+        if (nw > 1) {
+            if (mine) S.wkey[par][warp] = k;
+            group_barrier(nw * 32);
+            k = S.wkey[par][lane & (kCWarps - 1)];
+            g = warp_best(k.x, k.y, lane < nw ? k.z : kNone);
+            mine = mine && warp == g;
+        }
+        const unsigned p = __shfl_sync(0xffffffffu, k.z, g), orig = __shfl_sync(0xffffffffu, k.w, g);
+        // LAPACK: an exact zero pivot is neither divided by nor applied
+        const bool apply = __shfl_sync(0xffffffffu, k.x | k.y, g) != 0;
+        if (mine) {
+            cd* row = S.rows[par][0];
+#pragma unroll
+            for (int x = 0; x < kW; ++x) row[x] = a[x];
+            S.inv[par] = !apply ? cd{1.0, 0.0} : (recip_special(z) ? cdiv(cd{1.0, 0.0}, z) : binv);
+        }
+        if (nw > 1) group_barrier(nw * 32);
+        else __syncwarp();
+        const cd* piv = S.rows[par][0];
+        const cd l = a[0] * S.inv[par];
+        const int wj = apply ? kW - jj : 0;  // slots the pivot row updates; multipliers meet a zero
+        tpos = tpos == p ? c : (tpos == c ? p : tpos);
+        pos = pos == p ? kNone : (pos == c ? p : pos);
+#pragma unroll
+        for (int x = 0; x + 1 < kW; ++x) a[x] = csub_mul(a[x + 1], l, *(x + 1 < wj ? piv + x + 1 : &S.zero));
+        a[kW - 1] = l;
+        if (warp == nw - 1) {
+            // the pivot row out: slot s < W - jj holds column jj + s, then
+            // the multipliers
+            if (lane < w) st2(A + c + (int64_t)(c0 + lane) * lda, piv[lane >= jj ? lane - jj : kW - jj + lane]);
+            if (lane < jj) S.tri[jj][lane] = piv[kW - jj + lane];
+            if (lane == 0) {
+                S.src[jj] = (int)orig;
+                ipiv[c] = (int32_t)(p + 1);
+                if (!apply && info[0] == 0) info[0] = (int32_t)(c + 1);
+            }
+        }
+    }
+    // the rows below to their positions: the last w slots hold their multipliers
+    if (pos != kNone) {
+        cd* row = A + pos + (int64_t)c0 * lda;
+#pragma unroll
+        for (int s = 0; s < kW; ++s)
+            if (s >= kW - w) st2(row + (int64_t)(s - (kW - w)) * lda, a[s]);
+    }
+    if (warp == 0 && lane < kW) S.disp[lane] = lane < w && tpos >= (unsigned)(c0 + w) ? (int)tpos : -1;
+}
 
 template <int RPT>
 __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
@@ -227,10 +310,28 @@ __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
     for (int c0 = P.j0; c0 < jend; c0 += kW) {
         const int w = min(kW, jend - c0);
         // ---------------------------------------------------------- panel
+        const bool solo = RPT == 1 && n - c0 <= kCT;
+        if (solo) {
+            // The rows fit one CTA: rank 0 factors the panel alone, two CTA
+            // barriers a column instead of an exchange, and the others take
+            // the row order and L11 from its shared memory: 104 against 118
+            // us at order 64, 355 against 372 at 200.  (Two rows a thread are
+            // the slower choice: 646 against 543 us at 300.)
+            if (rank == 0) panel_solo(S, A, lda, ipiv, info, n, c0, w);
+            __syncwarp();
+            cluster_barrier();
+            if (rank != 0) {
+                if (tid < kW) {
+                    S.src[tid] = *cl.map_shared_rank(&S.src[tid], 0);
+                    S.disp[tid] = *cl.map_shared_rank(&S.disp[tid], 0);
+                }
+                if (tid < kW * kW) S.tri[tid / kW][tid % kW] = *cl.map_shared_rank(&S.tri[tid / kW][tid % kW], 0);
+            }
+        } else {
         const int per = (n - c0 + C - 1) / C;
         const int base = c0 + rank * per;
         const int cnt = max(0, min(per, n - base));
-        const int nw = RPT > 1 ? kCWarps : min(kCWarps, (per + 31) / 32);  // warps that hold rows
+        const int nw = min(kCWarps, (per + 31) / 32);  // warps that hold rows
         if (warp < nw) {
             cd a[RPT][kW];
             unsigned pos[RPT];  // the row's current position; kNone: no row, or a pivot already
@@ -412,6 +513,7 @@ __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
                 S.disp[lane] = lane < w && tpos >= (unsigned)(c0 + w) ? (int)min(tpos, (unsigned)(n - 1)) : -1;
         } else {
             step += w;
+        }
         }
         __syncthreads();
         // ------------------------------------- interchanges, triangular solve
@@ -859,8 +961,13 @@ mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas
     MW_REQUIRE(!P.back || (P.j0 == 0 && P.jb == P.n && P.n <= kBackRows), "back substitution needs the whole matrix");
     const int m = P.n - P.j0;
     const int cap = max_ctas > 0 && max_ctas < kMaxC ? max_ctas : kMaxC;
+    // CTAs per cluster: one up to a single panel, eight up to 256 rows (the
+    // panel is one CTA's, the rest of the work still spreads: 49 us at order
+    // 21 against 66 with one CTA, 355 at 200 against 408 with four and 362
+    // with sixteen), sixteen beyond (549 against 601 us at 300)
+    const int want = m <= kW ? 1 : (m <= kCT ? 8 : kMaxC);
     int C = 1;
-    while (C < cap && C < max_cluster<1>() && C * 32 < m) C *= 2;
+    while (2 * C <= cap && C < want && C < max_cluster<1>()) C *= 2;
     // enough rows per thread for the panel
     while (C < kMaxC && (m + C - 1) / C > 3 * kCT) C *= 2;
     const int per = (m + C - 1) / C;
