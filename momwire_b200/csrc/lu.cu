@@ -1296,6 +1296,7 @@ mw_status zgemm_launch(bool ta, bool tb, int64_t m, int64_t n, int64_t k, cd alp
         const int64_t tiles = ((m + DM_M - 1) / DM_M) * ((n + DM_N - 1) / DM_N);
         int64_t ctas = dmma_sms();
         if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
+        if (max_ctas < 0) ctas = tiles;  // a CTA per tile: SMs free up while the product runs
         DmSplit split{nullptr, nullptr, tiles, 1};
         const int64_t tail = tiles % ctas;
         if (split_ws && tail > 0 && split_ws_bytes > kDmSplitCountBytes) {
@@ -1636,6 +1637,14 @@ static mw_status aux_streams(AuxStreams** out) {
         MW_CHECK_CUDA(cudaEventCreateWithFlags(&a.ev_back, cudaEventDisableTiming));
     }
     *out = &a;
+    return MW_OK;
+}
+
+mw_status zlu_streams(ZluStreams* out) {
+    AuxStreams* a = nullptr;
+    mw_status s = aux_streams(&a);
+    if (s != MW_OK) return s;
+    *out = ZluStreams{a->trail, a->critical, a->ev_main, a->ev_handover, {a->ev_trail[0], a->ev_trail[1]}};
     return MW_OK;
 }
 
@@ -2298,7 +2307,7 @@ using namespace mw;
 // The panel exchange slots, then the row orders of the blocked cluster
 // factorisation.
 extern "C" size_t mw_getrf_workspace_size(int64_t n) {
-    return panel_ws_bytes() + sizeof(int32_t) * ((size_t)(n > 0 ? n : 0) + 2 * kZluBlock);
+    return panel_ws_bytes() + sizeof(int32_t) * ((size_t)(n > 0 ? n : 0) + 4 * kZluBlock);
 }
 
 // Factor A, carrying B (nrhs >= 0 columns) through it: B <- L^-1 P B, or with

@@ -55,6 +55,7 @@ namespace cg = cooperative_groups;
 mw_status zgemm_launch(bool ta, bool tb, int64_t m, int64_t n, int64_t k, cd alpha, const cd* A, int64_t lda,
                        const cd* B, int64_t ldb, cd beta, cd* C, int64_t ldc, cudaStream_t st, int max_ctas,
                        void* split_ws, size_t split_ws_bytes);
+constexpr int kCtaPerTile = -1;  // max_ctas: a CTA per tile instead of persistent ones
 
 namespace {
 
@@ -675,7 +676,7 @@ __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
     if (P.rid != nullptr) {
         // the block's row order: src[i] the row that ends in position j0 + i,
         // disp[i] where row j0 + i went (-1: it stays within the block)
-        int32_t* const src = P.rid + n;
+        int32_t* const src = P.order;
         int32_t* const disp = src + P.jb;
         for (int r = P.j0 + rank * kCT + tid; r < n; r += C * kCT) {
             const int o = __ldcg(P.rid + r);
@@ -1010,30 +1011,43 @@ class Pace {
 };
 
 // Blocked factorisation of the whole matrix with nrhs carried columns (B <-
-// L^-1 P B).  `rid`: n + 2 kZluBlock ints of workspace.  One stream: the
-// block's cluster leaves 132 SMs idle, but its chain is short beside the
-// update, which in return has every SM (a second stream's update would keep
-// a cluster from finding its SMs together).
+// L^-1 P B).  `rid`: n + 4 kZluBlock ints of workspace.  A look-ahead of one
+// block on two streams: the critical one (highest priority) updates the next
+// block's columns and factors them while the other applies the block to the
+// rest of the matrix.  Panel j waits for that stream's step j - 2 only.  The
+// rest's product is one block per tile, so that SMs free up in between and
+// the next panel's cluster finds its sixteen together.  Measured on B200,
+// factorisation and solve with 64 right-hand sides, one stream against two:
+// 11.2 -> 9.5 ms at order 2,624, 32.9 -> 25.2 at 5,000, 162 -> 133 at 10,496.
 mw_status zlu_blocked(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* info, cd* B, int64_t ldb, int64_t nrhs,
-                      int32_t* rid, const volatile int32_t* cancel, cudaStream_t st) {
+                      int32_t* rid, const volatile int32_t* cancel, cudaStream_t caller) {
     const int nb = kZluBlock;
+    ZluStreams zs;
+    if (mw_status s = zlu_streams(&zs); s != MW_OK) return s;
+    const cudaStream_t st = zs.critical, tr = zs.trail;
+    MW_CHECK_CUDA(cudaEventRecord(zs.ev_handover, caller));
+    MW_CHECK_CUDA(cudaStreamWaitEvent(st, zs.ev_handover, 0));
+    MW_CHECK_CUDA(cudaStreamWaitEvent(tr, zs.ev_handover, 0));
     Pace pace;
     if (cancel) {
         mw_status s = pace.start(st);
         if (s != MW_OK) return s;
     }
-    for (int64_t j0 = 0; j0 < n; j0 += nb) {
+    const cd m1{-1.0, 0.0}, p1{1.0, 0.0};
+    for (int64_t j = 0, j0 = 0; j0 < n; ++j, j0 += nb) {
         if (cancel) {
-            mw_status s = pace.step(j0 / nb, st);
+            mw_status s = pace.step(j, st);
             if (s != MW_OK) return s;
         }
         if (cancel && *cancel) {
+            // let both streams finish what they were given
+            MW_CHECK_CUDA(cudaStreamSynchronize(tr));
             MW_CHECK_CUDA(cudaStreamSynchronize(st));
             set_error("factorisation cancelled");
             return MW_ERR_CANCELLED;
         }
         const int jb = (int)(n - j0 < nb ? n - j0 : nb);
-        const int64_t c1 = j0 + jb, right = n - c1;
+        const int64_t c1 = j0 + jb, cn = n - c1 < nb ? n - c1 : nb, c2 = c1 + cn;
         ZluArgs P{};
         P.A = A;
         P.lda = lda;
@@ -1043,6 +1057,7 @@ mw_status zlu_blocked(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* inf
         P.ipiv = ipiv;
         P.info = info;
         P.rid = rid;
+        P.order = rid + n + (j & 1) * 2 * kZluBlock;  // (the other stream may still read the last block's)
         mw_status s = zlu_cluster(P, 1, st);
         if (s != MW_OK) return s;
         SolveArgs Q{};
@@ -1050,29 +1065,47 @@ mw_status zlu_blocked(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* inf
         Q.ldt = lda;
         Q.j0 = (int)j0;
         Q.jb = jb;
-        Q.src = rid + n;
-        Q.disp = rid + n + jb;
+        Q.src = P.order;
+        Q.disp = P.order + jb;
+        MW_CHECK_CUDA(cudaEventRecord(zs.ev_main, st));
+        MW_CHECK_CUDA(cudaStreamWaitEvent(tr, zs.ev_main, 0));
+        if (cn > 0) {  // the next block's columns
+            if (j > 0) MW_CHECK_CUDA(cudaStreamWaitEvent(st, zs.ev_trail[(j - 1) & 1], 0));
+            SolveArgs N = Q;
+            N.X = A + c1 * lda;
+            N.ldx = lda;
+            N.ncols = (int)cn;
+            s = block_solve<false>(N, st);
+            if (s == MW_OK)
+                s = zgemm_launch(false, false, n - c1, cn, jb, m1, A + c1 + j0 * lda, lda, A + j0 + c1 * lda, lda, p1,
+                                 A + c1 + c1 * lda, lda, st, 0, nullptr, 0);
+            if (s != MW_OK) return s;
+        }
+        // everything else: the columns left of the block take its row order,
+        // those right of the next block and the right-hand sides the rest too
         Q.Aleft = A;
         Q.ldleft = lda;
         Q.left = (int)j0;
-        Q.X = A + c1 * lda;
+        Q.X = A + c2 * lda;
         Q.ldx = lda;
-        Q.ncols = (int)right;
+        Q.ncols = (int)(n - c2);
         Q.B = B;
         Q.ldb = ldb;
         Q.nrhs = (int)nrhs;
-        s = block_solve<false>(Q, st);
+        s = block_solve<false>(Q, tr);
+        if (s == MW_OK && n - c2 > 0)
+            s = zgemm_launch(false, false, n - c1, n - c2, jb, m1, A + c1 + j0 * lda, lda, A + j0 + c2 * lda, lda, p1,
+                             A + c1 + c2 * lda, lda, tr, kCtaPerTile, nullptr, 0);
+        if (s == MW_OK && nrhs > 0 && n - c1 > 0)
+            s = zgemm_launch(false, false, n - c1, nrhs, jb, m1, A + c1 + j0 * lda, lda, B + j0, ldb, p1, B + c1, ldb,
+                             tr, kCtaPerTile, nullptr, 0);
         if (s != MW_OK) return s;
-        if (right > 0) {
-            const cd m1{-1.0, 0.0}, p1{1.0, 0.0};
-            s = zgemm_launch(false, false, right, right, jb, m1, A + c1 + j0 * lda, lda, A + j0 + c1 * lda, lda, p1,
-                             A + c1 + c1 * lda, lda, st, 0, nullptr, 0);
-            if (s == MW_OK && nrhs > 0)
-                s = zgemm_launch(false, false, right, nrhs, jb, m1, A + c1 + j0 * lda, lda, B + j0, ldb, p1, B + c1,
-                                 ldb, st, 0, nullptr, 0);
-            if (s != MW_OK) return s;
-        }
+        MW_CHECK_CUDA(cudaEventRecord(zs.ev_trail[j & 1], tr));
     }
+    MW_CHECK_CUDA(cudaEventRecord(zs.ev_handover, st));
+    MW_CHECK_CUDA(cudaStreamWaitEvent(caller, zs.ev_handover, 0));
+    MW_CHECK_CUDA(cudaEventRecord(zs.ev_main, tr));
+    MW_CHECK_CUDA(cudaStreamWaitEvent(caller, zs.ev_main, 0));
     return MW_OK;
 }
 

@@ -19,11 +19,22 @@ struct ZluArgs {
     int64_t ldb, b_stride;
     int nrhs;
     int back;  // also B <- U^-1 B (whole matrix, nrhs <= 64)
-    // n + 2 jb ints (single matrix), or null: on return rid[n + i] is the
-    // row that ends in position j0 + i and rid[n + jb + i] the position row
-    // j0 + i went to (-1: it stays within the block)
+    // single matrix, or null: n ints of scratch, and 2 jb ints that return
+    // the block's row order -- order[i] the row that ends in position j0 + i,
+    // order[jb + i] the position row j0 + i went to (-1: it stays within the
+    // block)
     int32_t* rid;
+    int32_t* order;
 };
+
+// The two streams and events of a look-ahead factorisation, one set per host
+// thread and device (lu.cu).
+struct ZluStreams {
+    cudaStream_t trail, critical;
+    cudaEvent_t ev_main, ev_handover;
+    cudaEvent_t ev_trail[2];
+};
+mw_status zlu_streams(ZluStreams* out);
 
 // Rows one cluster can hold.
 int zlu_cluster_max_rows();
@@ -32,7 +43,7 @@ mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas
 // Columns of a block of the blocked factorisation.
 constexpr int kZluBlock = 128;
 // Whole factorisation of an order within zlu_cluster_max_rows() by blocks;
-// rid: n + 2 kZluBlock ints.
+// rid: n + 4 kZluBlock ints.
 mw_status zlu_blocked(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* info, cd* B, int64_t ldb, int64_t nrhs,
                       int32_t* rid, const volatile int32_t* cancel, cudaStream_t st);
 mw_status zlu_upper(int64_t n, const cd* LU, int64_t lda, cd* B, int64_t ldb, int64_t nrhs, cudaStream_t st);
