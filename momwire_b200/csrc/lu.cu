@@ -1023,10 +1023,15 @@ __global__ void __launch_bounds__(256) zgemm_kernel(int64_t m, int64_t n, int64_
 // time through a three-slot shared-memory ring filled by cp.async (no
 // staging registers: the three accumulator sets need them).
 constexpr int DM_M = 128, DM_N = 64, DM_K = 16, DM_STAGES = 3;
-constexpr int DM_PA = DM_M + 2;   // sA[kk][row] row stride (complex): the 4 kk rows of a load fall on distinct banks
 constexpr int DM_PB = DM_K + 4;   // sB[col][kk] stride (complex): 8 columns x 4 kk of a load on distinct banks
-constexpr int DM_SA = DM_K * DM_PA, DM_SB = DM_N * DM_PB;  // per slot
-constexpr size_t kDmmaSmem = sizeof(cd) * DM_STAGES * (DM_SA + DM_SB);
+constexpr int DM_SB = DM_N * DM_PB;  // per slot
+// A tile of TM rows: 2 TM threads, sA[kk][row] rows of TM + 2 (complex: the 4
+// kk rows of a load fall on distinct banks).
+template <int TM>
+struct DmTile {
+    static constexpr int threads = 2 * TM, PA = TM + 2, SA = DM_K * PA;
+    static constexpr size_t smem = sizeof(cd) * DM_STAGES * (SA + DM_SB);
+};
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -1062,22 +1067,23 @@ struct DmSplit {
 constexpr int kDmSplitMaxUnits = 256;
 constexpr size_t kDmSplitCountBytes = sizeof(unsigned int) * kDmSplitMaxUnits;
 
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256, 1) zgemm_dmma_kernel(int64_t m, int64_t n, int64_t k, cd alpha,
+template <bool TA, bool TB, int TM>
+__global__ void __launch_bounds__(2 * TM, 128 / TM) zgemm_dmma_kernel(int64_t m, int64_t n, int64_t k, cd alpha,
                                                             const cd* __restrict__ A, int64_t lda,
                                                             const cd* __restrict__ B, int64_t ldb, cd beta,
                                                             cd* __restrict__ C, int64_t ldc, DmSplit split) {
+    constexpr int NT = DmTile<TM>::threads, DM_PA = DmTile<TM>::PA, DM_SA = DmTile<TM>::SA;
     extern __shared__ __align__(16) unsigned char dm_smem[];
     __shared__ int s_last;
     cd* sA0 = reinterpret_cast<cd*>(dm_smem);  // [DM_STAGES][DM_K][DM_PA]
     cd* sB0 = sA0 + DM_STAGES * DM_SA;         // [DM_STAGES][DM_N][DM_PB]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp & 3, wn = warp >> 2;
+    const int wm = warp % (TM / 32), wn = warp / (TM / 32);
     const int gid = lane >> 2, tig = lane & 3;
-    constexpr int LA = DM_M * DM_K / 256, LB = DM_K * DM_N / 256;
+    constexpr int LA = TM * DM_K / NT, LB = DM_K * DM_N / NT;
     // persistent over the work units (the grid may be capped to leave SMs
     // to a concurrent kernel)
-    const int64_t n_mt = (m + DM_M - 1) / DM_M;
+    const int64_t n_mt = (m + TM - 1) / TM;
     const int64_t n_tiles = n_mt * ((n + DM_N - 1) / DM_N);
     const int64_t n_units = split.full + (n_tiles - split.full) * split.splits;
     const int64_t kchunk = ((k + DM_K - 1) / DM_K + split.splits - 1) / split.splits * DM_K;
@@ -1091,7 +1097,7 @@ __global__ void __launch_bounds__(256, 1) zgemm_dmma_kernel(int64_t m, int64_t n
         kb = chunk * kchunk;
         ke = kb + kchunk < k ? kb + kchunk : k;
     }
-    const int64_t m0 = (tile % n_mt) * DM_M, n0 = (tile / n_mt) * DM_N;
+    const int64_t m0 = (tile % n_mt) * TM, n0 = (tile / n_mt) * DM_N;
     double x[4][4][2], y[4][4][2], w[4][4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -1106,16 +1112,16 @@ __global__ void __launch_bounds__(256, 1) zgemm_dmma_kernel(int64_t m, int64_t n
         cd* sB = sB0 + slot * DM_SB;
 #pragma unroll
         for (int u = 0; u < LA; ++u) {
-            const int i = tid + u * 256;
-            const int r = TA ? i / DM_K : i % DM_M;
-            const int kk = TA ? i % DM_K : i / DM_M;
+            const int i = tid + u * NT;
+            const int r = TA ? i / DM_K : i % TM;
+            const int kk = TA ? i % DM_K : i / TM;
             const int64_t gr = m0 + r, gk = k0 + kk;
             const bool ok = gr < m && gk < ke;
             cp_async16(sA + kk * DM_PA + r, ok ? (TA ? A + gk + gr * lda : A + gr + gk * lda) : A, ok);
         }
 #pragma unroll
         for (int u = 0; u < LB; ++u) {
-            const int i = tid + u * 256;
+            const int i = tid + u * NT;
             const int kk = TB ? i / DM_N : i % DM_K;
             const int cc = TB ? i % DM_N : i / DM_K;
             const int64_t gk = k0 + kk, gc = n0 + cc;
@@ -1177,22 +1183,22 @@ __global__ void __launch_bounds__(256, 1) zgemm_dmma_kernel(int64_t m, int64_t n
             }
     const bool beta_zero = (beta.re == 0.0 && beta.im == 0.0);
     if (chunk >= 0) {
-        // partial sum of a split tile: element e of this thread at e * 256 + tid
+        // partial sum of a split tile: element e of this thread at e * NT + tid
         const int64_t st = tile - split.full;
-        cd* P = split.part + (st * split.splits + chunk) * (DM_M * DM_N);
+        cd* P = split.part + (st * split.splits + chunk) * (TM * DM_N);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int h = 0; h < 2; ++h) P[((i * 4 + j) * 2 + h) * 256 + tid] = cd{x[i][j][h], w[i][j][h]};
+                for (int h = 0; h < 2; ++h) P[((i * 4 + j) * 2 + h) * NT + tid] = cd{x[i][j][h], w[i][j][h]};
         __threadfence();
         __syncthreads();
         if (tid == 0) s_last = atomicAdd(split.count + st, 1u) == (unsigned)split.splits - 1;
         __syncthreads();
         if (!s_last) continue;
         __threadfence();
-        const cd* P0 = split.part + st * split.splits * (DM_M * DM_N);
+        const cd* P0 = split.part + st * split.splits * (TM * DM_N);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -1202,7 +1208,7 @@ __global__ void __launch_bounds__(256, 1) zgemm_dmma_kernel(int64_t m, int64_t n
                     double sr = 0.0, si = 0.0;
                     for (int c = 0; c < split.splits; ++c) {
                         const double2 v = __ldcg(reinterpret_cast<const double2*>(
-                            P0 + (int64_t)c * (DM_M * DM_N) + ((i * 4 + j) * 2 + h) * 256 + tid));
+                            P0 + (int64_t)c * (TM * DM_N) + ((i * 4 + j) * 2 + h) * NT + tid));
                         sr += v.x;
                         si += v.y;
                     }
@@ -1266,6 +1272,51 @@ static int dmma_sms() {
     return sms;
 }
 
+template <bool TA, bool TB, int TM>
+static mw_status dmma_launch(int64_t m, int64_t n, int64_t k, cd alpha, const cd* A, int64_t lda, const cd* B,
+                             int64_t ldb, cd beta, cd* C, int64_t ldc, cudaStream_t st, int max_ctas, void* split_ws,
+                             size_t split_ws_bytes) {
+    static const cudaError_t attr = cudaFuncSetAttribute(
+        zgemm_dmma_kernel<TA, TB, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DmTile<TM>::smem);
+    MW_CHECK_CUDA(attr);
+    // the CTAs an SM holds (register-bound); a cap leaves SMs to other work
+    const int64_t tiles = ((m + TM - 1) / TM) * ((n + DM_N - 1) / DM_N);
+    int64_t ctas = dmma_sms();
+    if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
+    ctas *= DM_M / TM;
+    if (max_ctas < 0) ctas = tiles;  // a CTA per tile: SMs free up while the product runs
+    DmSplit split{nullptr, nullptr, tiles, 1};
+    const int64_t tail = tiles % ctas;
+    if (split_ws && tail > 0 && split_ws_bytes > kDmSplitCountBytes) {
+        const int64_t room = (int64_t)((split_ws_bytes - kDmSplitCountBytes) / (TM * DM_N * sizeof(cd)));
+        int64_t s = ctas / tail;
+        const int64_t ksteps = (k + DM_K - 1) / DM_K;
+        if (s > ksteps) s = ksteps;
+        if (tail * s > room) s = room / tail;
+        if (tail * s > kDmSplitMaxUnits) s = kDmSplitMaxUnits / tail;
+        if (s >= 2) s = (ksteps + (ksteps + s - 1) / s - 1) / ((ksteps + s - 1) / s);  // no empty chunk
+        if (s >= 2) {
+            split.count = static_cast<unsigned int*>(split_ws);
+            split.part = reinterpret_cast<cd*>(static_cast<char*>(split_ws) + kDmSplitCountBytes);
+            split.full = tiles - tail;
+            split.splits = (int)s;
+        }
+    }
+    const int64_t units = split.full + (tiles - split.full) * split.splits;
+    dim3 grid((unsigned)(units < ctas ? units : ctas));
+    ProfileScope ps(PC_ZGEMM, st, 8.0 * (double)m * n * k, 16.0 * ((double)m * k + (double)k * n + 2.0 * m * n));
+    zgemm_dmma_kernel<TA, TB, TM><<<grid, DmTile<TM>::threads, DmTile<TM>::smem, st>>>(m, n, k, alpha, A, lda, B, ldb,
+                                                                                         beta, C, ldc, split);
+    MW_CHECK_CUDA(cudaGetLastError());
+    count_launch();
+    return MW_OK;
+}
+
+// Inner dimensions up to which a product takes 64-row tiles, two CTAs an SM:
+// the LU's updates (k = 128) spend as long in a tile's prologue and epilogue
+// as in its products, so another CTA has to compute meanwhile.
+constexpr int64_t kDmShortK = 256;
+
 // Shape dispatch (measured on B200, 16x16 dipole array): the register-tiled
 // DFMA kernel wins on the LU's rank-64 updates (16.4 vs 13.8 TFLOP/s: short
 // K, epilogue-bound), the DMMA kernel on long-K products such as the
@@ -1279,60 +1330,23 @@ mw_status zgemm_launch(bool ta, bool tb, int64_t m, int64_t n, int64_t k, cd alp
                        void* split_ws, size_t split_ws_bytes) {
     if (m <= 0 || n <= 0) return MW_OK;
     if (k < 128) return zgemm_launch_simt(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st);
-    {
-        static bool attr = false;
-        if (!attr) {
-            MW_CHECK_CUDA(cudaFuncSetAttribute(zgemm_dmma_kernel<false, false>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDmmaSmem));
-            MW_CHECK_CUDA(cudaFuncSetAttribute(zgemm_dmma_kernel<true, false>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDmmaSmem));
-            MW_CHECK_CUDA(cudaFuncSetAttribute(zgemm_dmma_kernel<false, true>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDmmaSmem));
-            MW_CHECK_CUDA(cudaFuncSetAttribute(zgemm_dmma_kernel<true, true>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDmmaSmem));
-            attr = true;
-        }
-        // one CTA per SM (register-bound); a cap leaves SMs to other work
-        const int64_t tiles = ((m + DM_M - 1) / DM_M) * ((n + DM_N - 1) / DM_N);
-        int64_t ctas = dmma_sms();
-        if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
-        if (max_ctas < 0) ctas = tiles;  // a CTA per tile: SMs free up while the product runs
-        DmSplit split{nullptr, nullptr, tiles, 1};
-        const int64_t tail = tiles % ctas;
-        if (split_ws && tail > 0 && split_ws_bytes > kDmSplitCountBytes) {
-            const int64_t room = (int64_t)((split_ws_bytes - kDmSplitCountBytes) / (DM_M * DM_N * sizeof(cd)));
-            int64_t s = ctas / tail;
-            const int64_t ksteps = (k + DM_K - 1) / DM_K;
-            if (s > ksteps) s = ksteps;
-            if (tail * s > room) s = room / tail;
-            if (tail * s > kDmSplitMaxUnits) s = kDmSplitMaxUnits / tail;
-            if (s >= 2) s = (ksteps + (ksteps + s - 1) / s - 1) / ((ksteps + s - 1) / s);  // no empty chunk
-            if (s >= 2) {
-                split.count = static_cast<unsigned int*>(split_ws);
-                split.part = reinterpret_cast<cd*>(static_cast<char*>(split_ws) + kDmSplitCountBytes);
-                split.full = tiles - tail;
-                split.splits = (int)s;
-            }
-        }
-        const int64_t units = split.full + (tiles - split.full) * split.splits;
-        dim3 grid((unsigned)(units < ctas ? units : ctas));
-        ProfileScope ps(PC_ZGEMM, st, 8.0 * (double)m * n * k, 16.0 * ((double)m * k + (double)k * n + 2.0 * m * n));
-        if (!ta && !tb)
-            zgemm_dmma_kernel<false, false><<<grid, 256, kDmmaSmem, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
-                                                                             split);
-        else if (ta && !tb)
-            zgemm_dmma_kernel<true, false><<<grid, 256, kDmmaSmem, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
-                                                                             split);
-        else if (!ta && tb)
-            zgemm_dmma_kernel<false, true><<<grid, 256, kDmmaSmem, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
-                                                                             split);
-        else
-            zgemm_dmma_kernel<true, true><<<grid, 256, kDmmaSmem, st>>>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc,
-                                                                             split);
-        MW_CHECK_CUDA(cudaGetLastError());
-        count_launch();
-        return MW_OK;
+    if (k <= kDmShortK && !split_ws) {
+        if (!ta) return tb ? dmma_launch<false, true, 64>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st, max_ctas,
+                                                          nullptr, 0)
+                           : dmma_launch<false, false, 64>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st, max_ctas,
+                                                           nullptr, 0);
+        return tb ? dmma_launch<true, true, 64>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st, max_ctas, nullptr, 0)
+                  : dmma_launch<true, false, 64>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st, max_ctas, nullptr,
+                                                 0);
     }
+    if (!ta) return tb ? dmma_launch<false, true, 128>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st, max_ctas,
+                                                       split_ws, split_ws_bytes)
+                       : dmma_launch<false, false, 128>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st, max_ctas,
+                                                        split_ws, split_ws_bytes);
+    return tb ? dmma_launch<true, true, 128>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st, max_ctas, split_ws,
+                                             split_ws_bytes)
+              : dmma_launch<true, false, 128>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st, max_ctas, split_ws,
+                                              split_ws_bytes);
 }
 
 // The register-tiled DFMA kernel: the products with k < 128 (the FP64

@@ -761,8 +761,8 @@ __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
 // unit lower (or, UPPER, the upper) triangle of the diagonal block and P the
 // block's row order (src / disp of the panel; null: the rows stay).  A CTA
 // holds 32 columns of X in shared memory and takes the triangle in strips of
-// 16 columns: one warp solves the strip's 16 rows (a column per lane, in
-// registers), all warps apply it to the rest.  The columns left of the block
+// 16 columns, fetched a strip ahead: four warps solve the strip's 16 rows
+// (four lanes a column), all warps apply it to the rest.  The columns left of the block
 // only take the interchanges: `left` of them from Aleft on, in CTAs of their
 // own.  A gather of all rows at once replaces LAPACK's sequential swaps.
 constexpr int kSN = 32, kSMax = 128;
@@ -827,38 +827,54 @@ __global__ void __launch_bounds__(kCT) zblock_solve_kernel(SolveArgs P) {
         }
     }
     const int nstrip = isleft ? 0 : (jb + kW - 1) / kW;
+    // strip s: columns k0 .. k0 + w of the triangle, its rows from k0 down
+    // (lower) or down to k0 + w (upper); fetched a strip ahead
+    constexpr int F = kW * kSMax / kCT;
+    cd fs[F], fd{1.0, 0.0};
+    auto fetch = [&](int st) {
+        const int k0 = (UPPER ? nstrip - 1 - st : st) * kW, w = min(kW, jb - k0);
+        const int f0 = UPPER ? 0 : k0, f1 = UPPER ? k0 + w : jb;
+#pragma unroll
+        for (int u = 0; u < F; ++u) {
+            const int e = tid + u * kCT, r = e % kSMax, k = e / kSMax;
+            fs[u] = r >= f0 && r < f1 && k < w ? ld2(P.T + r + (int64_t)(k0 + k) * P.ldt) : cd{0.0, 0.0};
+        }
+        if (UPPER) fd = tid < w ? ld2(P.T + (k0 + tid) + (int64_t)(k0 + tid) * P.ldt) : cd{1.0, 0.0};
+    };
+    if (nstrip > 0) fetch(0);
     for (int s = 0; s < nstrip; ++s) {
         const int k0 = (UPPER ? nstrip - 1 - s : s) * kW, w = min(kW, jb - k0);
-        // the strip's rows: k0 .. jb (lower), 0 .. k0 + w (upper)
-        const int f0 = UPPER ? 0 : k0, f1 = UPPER ? k0 + w : jb;
-        for (int e = tid; e < kW * kSMax; e += kCT) {
-            const int r = f0 + e % kSMax, k = e / kSMax;
-            if (r < f1) Ls[k * kSMax + r] = k < w ? ld2(P.T + r + (int64_t)(k0 + k) * P.ldt) : cd{0.0, 0.0};
+#pragma unroll
+        for (int u = 0; u < F; ++u) {
+            const int e = tid + u * kCT;
+            Ls[(e / kSMax) * kSMax + e % kSMax] = fs[u];
         }
-        if (UPPER && tid < w) dinv[tid] = cdiv(cd{1.0, 0.0}, ld2(P.T + (k0 + tid) + (int64_t)(k0 + tid) * P.ldt));
+        if (UPPER && tid < kW) dinv[tid] = crecip(fd);
         __syncthreads();
-        if (warp == 0) {
-            cd t[kW];
+        if (s + 1 < nstrip) fetch(s + 1);
+        if (warp < kSN / 8) {
+            // the strip's rows: four lanes a column (lane f of them rows f,
+            // f + 4, ...), eight columns a warp
+            const int f = lane & 3, c = warp * 8 + (lane >> 2);
+            cd t[kW / 4];
 #pragma unroll
-            for (int i = 0; i < kW; ++i) t[i] = i < w ? X[(k0 + i) * kSPitch + lane] : cd{0.0, 0.0};
-            if (UPPER) {
+            for (int u = 0; u < kW / 4; ++u)
+                t[u] = 4 * u + f < w ? X[(k0 + 4 * u + f) * kSPitch + c] : cd{0.0, 0.0};
 #pragma unroll
-                for (int i = kW - 1; i >= 0; --i)
-                    if (i < w) {
-                        t[i] = t[i] * dinv[i];
+            for (int kk = 0; kk < kW; ++kk) {
+                const int k = UPPER ? kW - 1 - kk : kk;
+                if (UPPER && f == (k & 3)) t[k / 4] = t[k / 4] * dinv[k];
+                const cd x{__shfl_sync(0xffffffffu, t[k / 4].re, (lane & ~3) | (k & 3)),
+                           __shfl_sync(0xffffffffu, t[k / 4].im, (lane & ~3) | (k & 3))};
 #pragma unroll
-                        for (int r = 0; r < i; ++r) t[r] = csub_mul(t[r], Ls[i * kSMax + k0 + r], t[i]);
-                    }
-            } else {
-#pragma unroll
-                for (int k = 0; k + 1 < kW; ++k)
-#pragma unroll
-                    for (int i = k + 1; i < kW; ++i)
-                        if (i < w) t[i] = csub_mul(t[i], Ls[k * kSMax + k0 + i], t[k]);
+                for (int u = 0; u < kW / 4; ++u) {
+                    const int i = 4 * u + f;
+                    if ((UPPER ? i < k : i > k) && i < w) t[u] = csub_mul(t[u], Ls[k * kSMax + k0 + i], x);
+                }
             }
 #pragma unroll
-            for (int i = 0; i < kW; ++i)
-                if (i < w) X[(k0 + i) * kSPitch + lane] = t[i];
+            for (int u = 0; u < kW / 4; ++u)
+                if (4 * u + f < w) X[(k0 + 4 * u + f) * kSPitch + c] = t[u];
         }
         __syncthreads();
         const int g0 = UPPER ? 0 : k0 + w, g1 = UPPER ? k0 : jb;
