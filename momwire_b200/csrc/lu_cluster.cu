@@ -18,9 +18,8 @@
 //   rest    the panel's row interchanges and the W x W triangular solve of
 //           the columns to its right, four lanes per column (all gathered
 //           values in flight at once; every CTA already holds L11 and the
-//           row order from the exchange), then the rank-W update in 64 x 32
-//           tiles on FP64 tensor instructions, the next tile's operands
-//           loading meanwhile.
+//           row order from the exchange), then the rank-W update on FP64
+//           tensor instructions, 16 x 32 entries a warp.
 //   B       right-hand sides ride along as further columns; with `back` the
 //           kernel also substitutes backwards, each CTA its own right-hand
 //           sides, so a small system is factored and solved by one launch.
@@ -63,7 +62,7 @@ constexpr int kW = 16;          // panel width
 constexpr int kCT = 256;        // threads per CTA
 constexpr int kCWarps = kCT / 32;
 constexpr int kMaxC = 16;       // CTAs per cluster
-constexpr int kTM = 64, kTN = 32;  // update tile
+constexpr int kTM = 16, kTN = 32;  // a warp's update task
 constexpr int kBackRows = 1696;  // order times right-hand sides a CTA substitutes at once
 constexpr unsigned kNone = 0xffffffffu;
 constexpr int kXchBytes = (kW + 1) * 16;  // one CTA's share of a column's exchange
@@ -196,13 +195,7 @@ struct Shared {
     cd X[kW][4];  // a solved block of the back substitution
     cd inv[2];    // one-CTA panel: the pivot's reciprocal
     cd zero;
-    union {
-        struct {
-            cd L[kW][kTM + 2];  // (row strides that spread the fragment loads over the banks)
-            cd U[kTN][kW + 4];
-        } g;
-        cd y[kBackRows];
-    } u;
+    cd y[kBackRows];  // the back substitution's right-hand sides
 };
 
 // The panel rows [c0, n) x columns [c0, c0 + w) by one CTA (n - c0 <= kCT):
@@ -571,104 +564,78 @@ __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
         __syncwarp();
         cluster_barrier();
         // ---------------------------------------------------- rank-w update
+        // A warp takes 16 x 32 entries: 2 x 4 blocks of 8 x 8 for the FP64
+        // tensor instruction, in the four-product complex form.  C, L and U
+        // come straight from L2 in the instruction's fragment layout -- whole
+        // 64- and 128-byte runs -- all loads in flight at once; no staging and
+        // no barrier (64 x 32 tiles through shared memory took 4,600 cycles
+        // for what 2,050 of products need).
         const int r0 = c0 + w, m2 = n - r0, n2 = right + P.nrhs;
         const int tm = (m2 + kTM - 1) / kTM, tn = (n2 + kTN - 1) / kTN;
-        auto colptr = [&](int q) { return q < right ? A + (int64_t)(r0 + q) * lda : B + (int64_t)(q - right) * ldb; };
-        // warp tile 16 x 16 of the 64 x 32: 2 x 2 blocks of 8 x 8, FP64
-        // tensor instructions with the four-product complex form
-        const int gid = lane >> 2, tig = lane & 3, wm = (warp & 3) * 16, wn = (warp >> 2) * 16;
-        cd acc[2][2][2], fl[kW * kTM / kCT], fu[kW * kTN / kCT];
-        auto fetch = [&](int i0, int q0) {  // C, L and U of a tile
+        const int gid = lane >> 2, tig = lane & 3;
+        for (int task = warp * C + rank; task < tm * tn; task += kCWarps * C) {
+            const int i0 = (task % tm) * kTM, q0 = (task / tm) * kTN;
+            auto colptr = [&](int q) {
+                return q < right ? A + (int64_t)(r0 + q) * lda : B + (int64_t)(q - right) * ldb;
+            };
+            double cr[2][4][2], ci[2][4][2];
 #pragma unroll
-            for (int u = 0; u < kW * kTM / kCT; ++u) {
-                const int e = tid + u * kCT, r = e % kTM, k = e / kTM;
-                fl[u] = k < w && i0 + r < m2 ? ld2(A + (r0 + i0 + r) + (int64_t)(c0 + k) * lda) : cd{0.0, 0.0};
-            }
-#pragma unroll
-            for (int u = 0; u < kW * kTN / kCT; ++u) {
-                const int e = tid + u * kCT, k = e % kW, q = e / kW;
-                fu[u] = k < w && q0 + q < n2 ? ld2(colptr(q0 + q) + c0 + k) : cd{0.0, 0.0};
-            }
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int q = q0 + wn + 8 * j + 2 * tig + h;
-                    const cd* col = colptr(q) + r0 + i0 + wm + gid;
+                    const int q = q0 + 8 * j + 2 * tig + h;
+                    const cd* col = colptr(q) + r0 + i0 + gid;
 #pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        acc[i][j][h] = q < n2 && i0 + wm + gid + 8 * i < m2 ? ld2(col + 8 * i) : cd{0.0, 0.0};
+                    for (int i = 0; i < 2; ++i) {
+                        const cd v = q < n2 && i0 + gid + 8 * i < m2 ? ld2(col + 8 * i) : cd{0.0, 0.0};
+                        cr[i][j][h] = v.re;
+                        ci[i][j][h] = v.im;
+                    }
                 }
-        };
-        // this CTA's tiles: row tiles fastest
-        int ti = rank % max(tm, 1), tq = tm > 0 ? rank / tm : tn;
-        const int di = C % max(tm, 1), dq = C / max(tm, 1);
-        if (tq < tn) fetch(ti * kTM, tq * kTN);
-        while (tq < tn) {
-            const int i0 = ti * kTM, q0 = tq * kTN;
+            cd la[kW / 4][2], ub[kW / 4][4];
 #pragma unroll
-            for (int u = 0; u < kW * kTM / kCT; ++u) {
-                const int e = tid + u * kCT;
-                S.u.g.L[e / kTM][e % kTM] = fl[u];
+            for (int k4 = 0; k4 < kW / 4; ++k4) {
+                const int k = 4 * k4 + tig;
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                    la[k4][i] = k < w && i0 + gid + 8 * i < m2
+                                    ? ld2(A + (r0 + i0 + gid + 8 * i) + (int64_t)(c0 + k) * lda)
+                                    : cd{0.0, 0.0};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int q = q0 + 8 * j + gid;
+                    ub[k4][j] = k < w && q < n2 ? ld2(colptr(q) + c0 + k) : cd{0.0, 0.0};
+                }
             }
 #pragma unroll
-            for (int u = 0; u < kW * kTN / kCT; ++u) {
-                const int e = tid + u * kCT;
-                S.u.g.U[e / kW][e % kW] = fu[u];
-            }
-            double cr[2][2][2], ci[2][2][2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        cr[i][j][h] = acc[i][j][h].re;
-                        ci[i][j][h] = acc[i][j][h].im;
-                    }
-            __syncthreads();
-            ti += di;
-            tq += dq;
-            if (ti >= tm) {
-                ti -= tm;
-                ++tq;
-            }
-            if (tq < tn) fetch(ti * kTM, tq * kTN);
-#pragma unroll
-            for (int k4 = 0; k4 < kW; k4 += 4) {
-                cd la[2], ub[2];
-#pragma unroll
-                for (int i = 0; i < 2; ++i) la[i] = S.u.g.L[k4 + tig][wm + 8 * i + gid];
-#pragma unroll
-                for (int j = 0; j < 2; ++j) ub[j] = S.u.g.U[wn + 8 * j + gid][k4 + tig];
+            for (int k4 = 0; k4 < kW / 4; ++k4) {
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        dmma(cr[i][j][0], cr[i][j][1], -la[i].re, ub[j].re);
-                        dmma(ci[i][j][0], ci[i][j][1], -la[i].re, ub[j].im);
+                    for (int j = 0; j < 4; ++j) {
+                        dmma(cr[i][j][0], cr[i][j][1], -la[k4][i].re, ub[k4][j].re);
+                        dmma(ci[i][j][0], ci[i][j][1], -la[k4][i].re, ub[k4][j].im);
                     }
 #pragma unroll
                 for (int i = 0; i < 2; ++i)
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        dmma(cr[i][j][0], cr[i][j][1], la[i].im, ub[j].im);
-                        dmma(ci[i][j][0], ci[i][j][1], -la[i].im, ub[j].re);
+                    for (int j = 0; j < 4; ++j) {
+                        dmma(cr[i][j][0], cr[i][j][1], la[k4][i].im, ub[k4][j].im);
+                        dmma(ci[i][j][0], ci[i][j][1], -la[k4][i].im, ub[k4][j].re);
                     }
             }
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const int q = q0 + wn + 8 * j + 2 * tig + h;
+                    const int q = q0 + 8 * j + 2 * tig + h;
                     if (q < n2) {
-                        cd* col = colptr(q) + r0 + i0 + wm + gid;
+                        cd* col = colptr(q) + r0 + i0 + gid;
 #pragma unroll
                         for (int i = 0; i < 2; ++i)
-                            if (i0 + wm + gid + 8 * i < m2) st2(col + 8 * i, cd{cr[i][j][h], ci[i][j][h]});
+                            if (i0 + gid + 8 * i < m2) st2(col + 8 * i, cd{cr[i][j][h], ci[i][j][h]});
                     }
                 }
-            __syncthreads();
         }
         __syncwarp();
         cluster_barrier();
@@ -707,7 +674,7 @@ __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
                 fu[c] = tid < b0 && c < w ? ld2(A + tid + (int64_t)(b0 + c) * lda) : cd{0.0, 0.0};
         };
         static_assert(kCT == kW * kW, "one triangle entry per thread");
-        cd* y = S.u.y;  // [n][at_once]
+        cd* y = S.y;  // [n][at_once]
         for (int e = tid; e < n * nq; e += kCT) y[(e % n) * at_once + e / n] = ld2(Bq + e % n + (e / n) * bstep);
         const int last = ((n - 1) / kW) * kW;
         fetch(last);
