@@ -494,16 +494,6 @@ __device__ __forceinline__ bool fill_tile(const FillArgs& A, const GLParams& gl,
     return mirror;
 }
 
-// Upper-triangle tile pair of block b: tc(tc+1)/2 <= b < (tc+1)(tc+2)/2,
-// tr = b - tc(tc+1)/2 <= tc.
-__device__ __forceinline__ void tri_pair(int64_t b, int& tr, int& tc) {
-    int64_t c = (int64_t)((sqrt(8.0 * (double)b + 1.0) - 1.0) * 0.5);
-    while ((c + 1) * (c + 2) / 2 <= b) ++c;
-    while (c * (c + 1) / 2 > b) --c;
-    tc = (int)c;
-    tr = (int)(b - c * (c + 1) / 2);
-}
-
 // One block per upper-triangle tile pair (tr <= tc).  A symmetric pair is
 // computed once and written to both blocks of Z; otherwise the block also
 // computes (tc, tr) itself.  The EK image fill labels direct and mirrored

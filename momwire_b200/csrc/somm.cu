@@ -15,12 +15,19 @@
 // same bisection stack), nodes handed out through an atomic counter because
 // their cost varies by orders of magnitude (grazing Hankel-form rows).
 //
-// Q: one CTA per (row tile, column tile) of the fill's basis tiling.  Phase A
-// forms the per-segment-pair moments Jc[p][P] = sum_qr W_p(q) F(q, r) W_P(r)
-// over n_qp x n_qp Gauss nodes in shared memory (one thread per pair);
-// phase B contracts them with the basis polynomials and subtracts Q from the
-// Z tile (and refreshes its complex64 copy).  The grid tables are read
-// through the read-only cache: a node's four surfaces are one 64-byte line.
+// Q: one CTA per upper-triangle pair of the fill's basis tiles -- the reaction
+// is symmetric (observer and source see the same R1, theta and surfaces, and
+// the projection is symmetric in the two tangents), so a block is also written
+// transposed.  Phase A evaluates the projected field, one thread per (segment
+// pair, observer node), contracting the source nodes as it goes; the moments
+// Jc[p][P] = sum_qr W_p(q) F(q, r) W_P(r) are then contracted with the basis
+// polynomials in two stages (source side, observer side) and Q subtracted
+// from Z (and its complex64 copy).  The grid tables are read through the
+// read-only cache: a node's four surfaces are one 64-byte line.  What bounds
+// it is the field evaluation (square roots, an arc tangent, sine and cosine,
+// 64 grid loads).  One thread per segment pair and every ordered tile pair
+// left three quarters of the threads idle on short wires: the remainder of a
+// 20-cell plate (1,690 segments) took 6.55 ms on B200, 1.1 ms now.
 #include <vector>
 
 #include "common.cuh"
@@ -129,12 +136,26 @@ struct QArgs {
 // source tangent split (4)
 __host__ __device__ constexpr int q_seg_stride(int NM, int nq) { return nq * 3 + NM * nq + 7; }
 
+constexpr int kQThreads = 192;
+constexpr int kQChunk = 4;  // observer nodes evaluated at a time
+
 template <int D>
-static size_t q_smem_bytes(int nq, int smax, int tb) {
-    constexpr int NM = D + 1, NMM = NM * NM;
-    return sizeof(double) * ((size_t)2 * smax * q_seg_stride(NM, nq) + (size_t)smax * smax * NMM * 2 + 2 * tb * NMM) +
-           sizeof(int) * (2 * tb * NM);
-}
+struct QSmem {
+    static constexpr int NM = D + 1, NMM = NM * NM;
+    int chunk;
+    size_t nR, nJ, nT, bytes;  // complex elements; bytes in all
+    __host__ __device__ QSmem(int nq, int smax, int tb) {
+        nJ = (size_t)smax * smax * NMM;
+        nT = (size_t)NM * smax * (tb + 1);
+        for (chunk = nq < kQChunk ? nq : kQChunk;; --chunk) {  // (as many nodes as fit)
+            nR = (size_t)smax * smax * chunk * NM;
+            bytes = sizeof(cd) * (nR + nJ + nT) +
+                    sizeof(double) * ((size_t)2 * smax * q_seg_stride(NM, nq) + 2 * tb * NMM) +
+                    sizeof(int) * (2 * tb * NM);
+            if (chunk == 1 || bytes <= 227 * 1024) break;
+        }
+    }
+};
 
 template <int D>
 __device__ __forceinline__ void q_stage(double* dst, const QArgs& A, int s) {
@@ -169,46 +190,52 @@ __device__ __forceinline__ void q_stage(double* dst, const QArgs& A, int s) {
 }
 
 template <int D>
-__global__ void __launch_bounds__(256) somm_q_kernel(QArgs A) {
+__global__ void __launch_bounds__(kQThreads, 2) somm_q_kernel(QArgs A) {
     constexpr int NM = D + 1, NMM = NM * NM;
-    extern __shared__ double qsm[];
+    extern __shared__ __align__(16) unsigned char q_smem[];
     const int nq = A.nq;
     const int SD = q_seg_stride(NM, nq);
     const int SMAX = A.basis.max_tile_seg, TB = A.basis.max_tile_basis;
-    const int tr = blockIdx.y, tc = blockIdx.x;
+    int tr, tc;
+    tri_pair((int64_t)blockIdx.x, tr, tc);
     const int ns_r = A.basis.tile_ns[tr], ns_c = A.basis.tile_ns[tc];
     const int nb_r = A.basis.tile_nb[tr], nb_c = A.basis.tile_nb[tc];
     const int fb_r = A.basis.tile_first[tr], fb_c = A.basis.tile_first[tc];
-    double* s_row = qsm;
+    const QSmem<D> lay(nq, SMAX, TB);
+    cd* s_R = reinterpret_cast<cd*>(q_smem);  // [pair][observer node of the chunk][P]
+    cd* s_J = s_R + lay.nR;                   // [pair][p][P]
+    cd* s_T = s_J + lay.nJ;                   // [p][SMAX][TB + 1]
+    double* s_row = reinterpret_cast<double*>(s_T + lay.nT);
     double* s_col = s_row + SMAX * SD;
-    double* s_J = s_col + SMAX * SD;                   // SMAX*SMAX*NMM complex
-    double* s_pr = s_J + (size_t)SMAX * SMAX * NMM * 2;
+    double* s_pr = s_col + SMAX * SD;
     double* s_pc = s_pr + TB * NMM;
     int* s_loc_r = reinterpret_cast<int*>(s_pc + TB * NMM);
     int* s_loc_c = s_loc_r + TB * NM;
     const int tid = threadIdx.x;
-    for (int i = tid; i < ns_r; i += blockDim.x) q_stage<D>(s_row + i * SD, A, A.basis.tile_seg[(size_t)tr * SMAX + i]);
-    for (int i = tid; i < ns_c; i += blockDim.x) q_stage<D>(s_col + i * SD, A, A.basis.tile_seg[(size_t)tc * SMAX + i]);
-    for (int i = tid; i < nb_r * NMM; i += blockDim.x) s_pr[i] = A.basis.polys[(size_t)fb_r * NMM + i];
-    for (int i = tid; i < nb_c * NMM; i += blockDim.x) s_pc[i] = A.basis.polys[(size_t)fb_c * NMM + i];
-    for (int i = tid; i < nb_r * NM; i += blockDim.x) s_loc_r[i] = A.basis.loc[(size_t)fb_r * NM + i];
-    for (int i = tid; i < nb_c * NM; i += blockDim.x) s_loc_c[i] = A.basis.loc[(size_t)fb_c * NM + i];
+    for (int i = tid; i < ns_r + ns_c; i += kQThreads) {
+        const bool c = i >= ns_r;
+        const int l = c ? i - ns_r : i;
+        q_stage<D>((c ? s_col : s_row) + l * SD, A, A.basis.tile_seg[(size_t)(c ? tc : tr) * SMAX + l]);
+    }
+    for (int i = tid; i < nb_r * NMM; i += kQThreads) s_pr[i] = A.basis.polys[(size_t)fb_r * NMM + i];
+    for (int i = tid; i < nb_c * NMM; i += kQThreads) s_pc[i] = A.basis.polys[(size_t)fb_c * NMM + i];
+    for (int i = tid; i < nb_r * NM; i += kQThreads) s_loc_r[i] = A.basis.loc[(size_t)fb_r * NM + i];
+    for (int i = tid; i < nb_c * NM; i += kQThreads) s_loc_c[i] = A.basis.loc[(size_t)fb_c * NM + i];
     __syncthreads();
 
-    // phase A: Jc of every staged segment pair
-    for (int pidx = tid; pidx < ns_r * ns_c; pidx += blockDim.x) {
-        const int li = pidx / ns_c, lj = pidx - li * ns_c;
-        const double* so = s_row + li * SD;
-        const double* ss = s_col + lj * SD;
-        const double* to = so + nq * 3 + NM * nq;
-        const double* tsv = ss + nq * 3 + NM * nq;
-        const SrcTangent ts{tsv[3], tsv[4], tsv[5], tsv[6]};
-        cd J[NM][NM];
-#pragma unroll
-        for (int p = 0; p < NM; ++p)
-#pragma unroll
-            for (int P = 0; P < NM; ++P) J[p][P] = cd{0.0, 0.0};
-        for (int q = 0; q < nq; ++q) {
+    // phase A: the moments of every staged segment pair, kQChunk observer
+    // nodes at a time
+    const int npair = ns_r * ns_c;
+    for (int q0 = 0; q0 < nq; q0 += lay.chunk) {
+        const int nc = min(lay.chunk, nq - q0);
+        for (int e = tid; e < npair * nc; e += kQThreads) {
+            const int pidx = e / nc, q = q0 + e - pidx * nc;
+            const int li = pidx / ns_c, lj = pidx - li * ns_c;
+            const double* so = s_row + li * SD;
+            const double* ss = s_col + lj * SD;
+            const double* to = so + nq * 3 + NM * nq;
+            const double* tsv = ss + nq * 3 + NM * nq;
+            const SrcTangent ts{tsv[3], tsv[4], tsv[5], tsv[6]};
             cd row[NM];
 #pragma unroll
             for (int P = 0; P < NM; ++P) row[P] = cd{0.0, 0.0};
@@ -222,66 +249,80 @@ __global__ void __launch_bounds__(256) somm_q_kernel(QArgs A) {
                     row[P].im += F.im * w;
                 }
             }
+            cd* dst = s_R + (size_t)e * NM;
 #pragma unroll
-            for (int p = 0; p < NM; ++p) {
-                const double w = so[nq * 3 + p * nq + q];
+            for (int P = 0; P < NM; ++P) dst[P] = row[P];
+        }
+        __syncthreads();
+        for (int e = tid; e < npair * NM; e += kQThreads) {
+            const int pidx = e / NM, p = e - pidx * NM;
+            const double* W = s_row + (pidx / ns_c) * SD + nq * 3 + p * nq + q0;
+            cd* J = s_J + (size_t)e * NM;
+            cd v[NM];
+#pragma unroll
+            for (int P = 0; P < NM; ++P) v[P] = q0 == 0 ? cd{0.0, 0.0} : J[P];
+            for (int q = 0; q < nc; ++q) {
+                const cd* R = s_R + ((size_t)pidx * nc + q) * NM;
 #pragma unroll
                 for (int P = 0; P < NM; ++P) {
-                    J[p][P].re += w * row[P].re;
-                    J[p][P].im += w * row[P].im;
+                    v[P].re += W[q] * R[P].re;
+                    v[P].im += W[q] * R[P].im;
                 }
             }
+#pragma unroll
+            for (int P = 0; P < NM; ++P) J[P] = v[P];
         }
-        double* dst = s_J + (size_t)pidx * NMM * 2;
+        __syncthreads();
+    }
+
+    // phase B: Q = sum_ab C_m J C_n, source side then observer side
+    const int pitch = TB + 1, plane = SMAX * pitch;
+    for (int e = tid; e < ns_r * nb_c; e += kQThreads) {
+        const int la = e / nb_c, ni = e - la * nb_c;
+        cd a[NM];
 #pragma unroll
-        for (int p = 0; p < NM; ++p)
+        for (int p = 0; p < NM; ++p) a[p] = cd{0.0, 0.0};
+        for (int b = 0; b < NM; ++b) {
+            const int lb = s_loc_c[ni * NM + b];
+            if (lb < 0) continue;
+            const cd* J = s_J + ((size_t)la * ns_c + lb) * NMM;
+            const double* C = s_pc + ni * NMM + b * NM;
 #pragma unroll
-            for (int P = 0; P < NM; ++P) {
-                dst[(p * NM + P) * 2] = J[p][P].re;
-                dst[(p * NM + P) * 2 + 1] = J[p][P].im;
-            }
+            for (int p = 0; p < NM; ++p)
+#pragma unroll
+                for (int P = 0; P < NM; ++P) {
+                    a[p].re += C[P] * J[p * NM + P].re;
+                    a[p].im += C[P] * J[p * NM + P].im;
+                }
+        }
+#pragma unroll
+        for (int p = 0; p < NM; ++p) s_T[p * plane + la * pitch + ni] = a[p];
     }
     __syncthreads();
-
-    // phase B: Q = sum_ab C_m J C_n; Z -= Q
-    for (int pp = tid; pp < TB * TB; pp += blockDim.x) {
+    auto subtract = [&](int64_t m, int64_t n, cd Q) {
+        double2* zp = reinterpret_cast<double2*>(A.Z + 2 * (m + n * A.ldz));
+        const double2 z = *zp;
+        const double zr = z.x - Q.re, zi = z.y - Q.im;
+        *zp = make_double2(zr, zi);
+        if (A.Z32) *reinterpret_cast<float2*>(A.Z32 + 2 * (m + n * A.ldz32)) = make_float2((float)zr, (float)zi);
+    };
+    for (int pp = tid; pp < TB * TB; pp += kQThreads) {
         const int mi = pp % TB, ni = pp / TB;
         if (mi >= nb_r || ni >= nb_c) continue;
         cd Q{0.0, 0.0};
-        const double* Cm = s_pr + mi * NMM;
-        const double* Cn = s_pc + ni * NMM;
         for (int a = 0; a < NM; ++a) {
             const int la = s_loc_r[mi * NM + a];
             if (la < 0) continue;
-            for (int b = 0; b < NM; ++b) {
-                const int lb = s_loc_c[ni * NM + b];
-                if (lb < 0) continue;
-                const double* J = s_J + ((size_t)la * ns_c + lb) * NMM * 2;
+            const double* C = s_pr + mi * NMM + a * NM;
 #pragma unroll
-                for (int p = 0; p < NM; ++p) {
-                    cd rowv{0.0, 0.0};
-#pragma unroll
-                    for (int P = 0; P < NM; ++P) {
-                        const double c = Cn[b * NM + P];
-                        rowv.re += c * J[(p * NM + P) * 2];
-                        rowv.im += c * J[(p * NM + P) * 2 + 1];
-                    }
-                    const double cm = Cm[a * NM + p];
-                    Q.re += cm * rowv.re;
-                    Q.im += cm * rowv.im;
-                }
+            for (int p = 0; p < NM; ++p) {
+                const cd t = s_T[p * plane + la * pitch + ni];
+                Q.re += C[p] * t.re;
+                Q.im += C[p] * t.im;
             }
         }
-        const int64_t m = fb_r + mi, n = fb_c + ni;
-        double* zp = A.Z + 2 * (m + n * A.ldz);
-        const double zr = zp[0] - Q.re, zi = zp[1] - Q.im;
-        zp[0] = zr;
-        zp[1] = zi;
-        if (A.Z32) {
-            float* z32 = A.Z32 + 2 * (m + n * A.ldz32);
-            z32[0] = (float)zr;
-            z32[1] = (float)zi;
-        }
+        subtract(fb_r + mi, fb_c + ni, Q);
+        if (tr != tc) subtract(fb_c + ni, fb_r + mi, Q);
     }
 }
 
@@ -437,18 +478,15 @@ extern "C" mw_status mw_somm_remainder_q(const mw_segments* seg, const mw_basis*
     A.Z32 = Z32;
     A.ldz32 = ldz32;
     const int d = basis->degree;
-    const size_t smem = d == 1 ? q_smem_bytes<1>(n_qp, basis->max_tile_seg, basis->max_tile_basis)
-                               : q_smem_bytes<2>(n_qp, basis->max_tile_seg, basis->max_tile_basis);
-    dim3 grid2(basis->n_tile, basis->n_tile);
+    const int smax = basis->max_tile_seg, tb = basis->max_tile_basis;
+    const size_t smem = d == 1 ? QSmem<1>(n_qp, smax, tb).bytes : QSmem<2>(n_qp, smax, tb).bytes;
+    const int64_t nt = basis->n_tile;
+    const unsigned blocks = (unsigned)(nt * (nt + 1) / 2);
     const double nn = (double)seg->n_seg * n_qp;
     ProfileScope ps(PC_SOMM_Q, st, nn * nn * 420.0, 16.0 * 2.0 * basis->n_basis * basis->n_basis);
-    if (d == 1) {
-        MW_CHECK_CUDA(cudaFuncSetAttribute(somm_q_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        somm_q_kernel<1><<<grid2, 256, smem, st>>>(A);
-    } else {
-        MW_CHECK_CUDA(cudaFuncSetAttribute(somm_q_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        somm_q_kernel<2><<<grid2, 256, smem, st>>>(A);
-    }
+    auto kern = d == 1 ? somm_q_kernel<1> : somm_q_kernel<2>;
+    MW_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<blocks, kQThreads, smem, st>>>(A);
     MW_CHECK_CUDA(cudaGetLastError());
     count_launch();
     return MW_OK;
