@@ -43,6 +43,25 @@ __device__ __forceinline__ cf crcp_sp(cf z) {
     return cf{a * t, -b * t};
 }
 
+// a - b and the two products with their roundings spelled out: a complex
+// product has two contracted forms of its imaginary part, and which one the
+// compiler takes depends on the code around it.  FIRST rounds the product
+// a.im b.re before the fused a.re b.im; otherwise the other way round.  The
+// forms below are chosen per position so that the factors are, bit for bit,
+// those of 32-column panels and chunks, whatever the width used here.
+template <bool FIRST>
+__device__ __forceinline__ cf mul_rn(cf a, cf b) {
+    const float re = __fmaf_rn(a.re, b.re, -__fmul_rn(a.im, b.im));
+    const float im = FIRST ? __fmaf_rn(a.re, b.im, __fmul_rn(a.im, b.re))
+                           : __fmaf_rn(a.im, b.re, __fmul_rn(a.re, b.im));
+    return cf{re, im};
+}
+template <bool FIRST>
+__device__ __forceinline__ cf submul_rn(cf v, cf a, cf b) {
+    const cf p = mul_rn<FIRST>(a, b);
+    return cf{__fsub_rn(v.re, p.re), __fsub_rn(v.im, p.im)};
+}
+
 __device__ __forceinline__ float cabs1f(cf z) { return fabsf(z.re) + fabsf(z.im); }
 
 constexpr int kSpLD = kSpB + 2;  // column stride of the staged block (complex; 16-byte aligned columns)
@@ -115,23 +134,255 @@ __device__ __forceinline__ void sp_trailing(cf* S, int c0, int jb, int tid) {
 }
 
 // Factor A[j0 .. j0+jb) x [j0 .. j0+jb) in place, pivots among these rows
-// only: a blocked LU of the block staged in shared memory (column major),
-// 32 columns at a time.
-//   first   without interchanges: warps 0-3 hold the panel's rows in
-//           registers (thread r = row r); per column the pivot row, whose
-//           values are final, is published in shared memory, one 128-thread
-//           named barrier, then every row below takes its multiplier and
-//           updates its panel columns.  Kept when every pivot is nonzero and
-//           every |l| (|re| + |im|) stays within kSpNoPivotBound -- on the
-//           strongly diagonal Galerkin blocks partial pivoting would keep
-//           the diagonal anyway, and the factors are then the same.
+// only: a blocked LU of the block staged in shared memory (column major).
+//   first   without interchanges, 16 columns at a time (sp_nopivot): the
+//           first warp factors the 16 x 16 sub-block in registers (sp_sub16)
+//           while the others still apply the panel before to the rest of the
+//           block; then the rows below and the columns right of the sub-block
+//           are solved, a thread each.  Two block barriers per panel.  Kept
+//           when every pivot is nonzero and every |l| (|re| + |im|) stays
+//           within kSpNoPivotBound -- on the strongly diagonal Galerkin
+//           blocks partial pivoting would keep the diagonal anyway, and the
+//           factors are then the same.
 //   else    the block is staged again and factored with partial pivoting
-//           among its rows: thread (r, s) holds row r's panel columns
-//           8s .. 8s+7, every thread takes part in every column, rows are
-//           interchanged physically (registers for the panel, shared memory
-//           for the other columns); two block barriers per column.
-// Each panel is followed by its U12 and A22 updates (sp_trailing).
+//           among its rows, 32 columns at a time: thread (r, s) holds row r's
+//           panel columns 8s .. 8s+7, every thread takes part in every
+//           column, rows are interchanged physically (registers for the
+//           panel, shared memory for the other columns); two block barriers
+//           per column, then the panel's U12 and A22 updates (sp_trailing).
+// What bounds it is the chain of 128 columns: a reciprocal, a trip through
+// shared memory, a multiplier, an update.  32-column panels whose diagonal
+// sub-block one warp factored in shared memory while fifteen waited, then
+// rows, U12 and A22 in turn, took 162 us a block on B200; 67 us so, of
+// which 7 are the trips from and to global memory, 28 the sub-blocks, 13 the
+// rows and columns beside them and the rest the first panels' updates, for
+// which one SM's FP32 rate is the bound.
 constexpr float kSpNoPivotBound = 2.0f;
+
+constexpr int kSpNW = 16;  // columns of a panel without interchanges
+
+// A 4 x 4 tile, rows i0, i0 + 1, i1, i1 + 1 (even) of columns jc .. jc + 3,
+// of A -= L U over inner columns c0 .. c0 + 15, every entry's products in
+// column order.
+template <bool FIRST>
+__device__ __noinline__ void sp_rank16_tile(cf* S, int c0, int i0, int i1, int jc) {
+    cf acc[4][4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int a4 = 0; a4 < 4; a4 += 2) {
+            const float4 v = *reinterpret_cast<const float4*>(S + (jc + q) * kSpLD + (a4 ? i1 : i0));
+            acc[a4][q] = cf{v.x, v.y};
+            acc[a4 + 1][q] = cf{v.z, v.w};
+        }
+#pragma unroll 2
+    for (int jj = 0; jj < kSpNW; ++jj) {
+        const cf* lcol = S + (c0 + jj) * kSpLD;
+        const float4 l01 = *reinterpret_cast<const float4*>(lcol + i0);
+        const float4 l23 = *reinterpret_cast<const float4*>(lcol + i1);
+        const cf l[4] = {cf{l01.x, l01.y}, cf{l01.z, l01.w}, cf{l23.x, l23.y}, cf{l23.z, l23.w}};
+        cf u[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) u[q] = S[(jc + q) * kSpLD + c0 + jj];
+#pragma unroll
+        for (int a4 = 0; a4 < 4; ++a4)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[a4][q] = submul_rn<FIRST>(acc[a4][q], l[a4], u[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int a4 = 0; a4 < 4; a4 += 2)
+            *reinterpret_cast<float4*>(S + (jc + q) * kSpLD + (a4 ? i1 : i0)) =
+                make_float4(acc[a4][q].re, acc[a4][q].im, acc[a4 + 1][q].re, acc[a4 + 1][q].im);
+}
+
+// The tiles of rows [r0, r1) x columns [q0, q1) (row counts multiples of 8)
+// by `nt` threads (this one the t-th); a tile's row pairs lie half the rows
+// apart, so that a warp's loads are contiguous.
+template <bool FIRST>
+__device__ __forceinline__ void sp_rank16(cf* S, int c0, int r0, int r1, int q0, int q1, int t, int nt) {
+    const int ntr = (r1 - r0) / 4, ntc = (q1 - q0) / 4;
+    for (int tile = t; tile < ntr * ntc; tile += nt) {
+        const int i0 = r0 + 2 * (tile % ntr);
+        sp_rank16_tile<FIRST>(S, c0, i0, i0 + 2 * ntr, q0 + 4 * (tile / ntr));
+    }
+}
+
+// All of rows, columns >= t0 but the 16 x 16 sub-block at t0 itself, which
+// the first warp keeps up to date.
+__device__ __forceinline__ void sp_rank16_rest(cf* S, int c0, int jr, int t, int nt) {
+    const int t0 = c0 + kSpNW, t1 = t0 + kSpNW;
+    // positions within the 32-column group of c0 take the second form
+    if (t0 / kSpPW == c0 / kSpPW) {
+        sp_rank16<false>(S, c0, t1, jr, t0, t1, t, nt);
+        sp_rank16<false>(S, c0, t0, t1, t1, jr, nt - 1 - t, nt);
+    } else {
+        sp_rank16<true>(S, c0, t1, jr, t0, t1, t, nt);
+        sp_rank16<true>(S, c0, t0, t1, t1, jr, nt - 1 - t, nt);
+    }
+    sp_rank16<true>(S, c0, t1, jr, t1, jr, t, nt);
+}
+
+// The sub-block's registers brought up to date with the panel at cp.
+template <bool FIRST>
+__device__ __forceinline__ void sp_sub16_update(const cf* S, int c0, int cp, int r, int h, cf (&a)[kSpNW / 2]) {
+#pragma unroll 2
+    for (int jj = 0; jj < kSpNW; ++jj) {
+        const cf l = S[(cp + jj) * kSpLD + c0 + r];
+#pragma unroll
+        for (int x = 0; x < kSpNW / 2; ++x)
+            a[x] = submul_rn<FIRST>(a[x], l, S[(c0 + 2 * x + h) * kSpLD + cp + jj]);
+    }
+}
+
+// The 16 x 16 sub-block at c0 by one warp: lane (r, h) holds row r's columns
+// of parity h in registers, brought up to date with the panel before (cp =
+// its first column, < 0: none) on the way in.  Pivot, pivot row and the
+// row's own entry pass by shuffles; every lane computes the reciprocal.  The
+// loop over column pairs stays rolled, the slots turning by one each time
+// (eight turns put them back): unrolled it ran five times slower, waiting for
+// instructions that one warp executes once.  True when a pivot is zero or a
+// multiplier exceeds the bound.
+__device__ __forceinline__ bool sp_sub16(cf* S, int c0, int cp, cf* s_inv) {
+    const int lane = threadIdx.x & 31, r = lane & 15, h = lane >> 4;
+    constexpr int kX = kSpNW / 2;
+    cf a[kX];
+#pragma unroll
+    for (int x = 0; x < kX; ++x) a[x] = S[(c0 + 2 * x + h) * kSpLD + c0 + r];
+    if (cp >= 0) {
+        if (cp / kSpPW == c0 / kSpPW)
+            sp_sub16_update<false>(S, c0, cp, r, h, a);
+        else
+            sp_sub16_update<true>(S, c0, cp, r, h, a);
+    }
+    bool bad = false;
+    float lmax = 0.0f;
+#pragma unroll 1
+    for (int t = 0; t < kX; ++t) {
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+            const int j = 2 * t + o;  // held by lanes 16 o + r in slot 0
+            const cf piv{__shfl_sync(0xffffffffu, a[0].re, 16 * o + j), __shfl_sync(0xffffffffu, a[0].im, 16 * o + j)};
+            const cf v{__shfl_sync(0xffffffffu, a[0].re, 16 * o + r), __shfl_sync(0xffffffffu, a[0].im, 16 * o + r)};
+            const float pa = cabs1f(piv);
+            bad = bad || !(pa > 0.0f);
+            const cf inv = pa > 0.0f ? crcp_sp(piv) : cone<cf>();
+            if (lane == j) s_inv[c0 + j] = inv;
+            const cf l = mul_rn<true>(v, inv);
+            const bool below = r > j;
+#pragma unroll
+            for (int x = 0; x < kX; ++x) {
+                // slot x holds column 2 (t + x) + h, or a finished one
+                const cf u{__shfl_sync(0xffffffffu, a[x].re, 16 * h + j),
+                           __shfl_sync(0xffffffffu, a[x].im, 16 * h + j)};
+                const cf w = submul_rn<false>(a[x], l, u);
+                const bool later = x == 0 ? h > o : t + x < kX;
+                if (below && later) a[x] = w;
+            }
+            if (below && h == o) a[0] = l;
+            if (below) lmax = fmaxf(lmax, cabs1f(l));
+        }
+        const cf turn = a[0];
+#pragma unroll
+        for (int x = 0; x + 1 < kX; ++x) a[x] = a[x + 1];
+        a[kX - 1] = turn;
+    }
+#pragma unroll
+    for (int x = 0; x < kX; ++x) S[(c0 + 2 * x + h) * kSpLD + c0 + r] = a[x];
+    // NaN-safe: a NaN multiplier fails the comparison
+    return bad || !(lmax <= kSpNoPivotBound);
+}
+
+// A row below the sub-block at c0 (ROW: a U11 = x, reciprocal pivots in inv)
+// or a column right of it (L11 t = x), in place; entry x at p + x * step, and
+// the sub-block's entry (i, j) at S[(c0 + j) * kSpLD + c0 + i].  Four entries
+// are finished at a time, then leave the others up to date, in registers that
+// turn by four.  Returns the largest |re| + |im| of a row's result.
+template <bool ROW>
+__device__ __forceinline__ float sp_solve16(const cf* S, int c0, cf* p, int step, const cf* inv, bool near) {
+    cf a[kSpNW];
+    float lmax = 0.0f;
+    const cf* D = S + c0 * kSpLD + c0;
+#pragma unroll
+    for (int x = 0; x < kSpNW; ++x) a[x] = p[x * step];
+#pragma unroll 1
+    for (int b = 0; b < kSpNW; b += 4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (ROW) {
+                const cf d = inv[b + j];
+                a[j] = near ? mul_rn<true>(a[j], d) : mul_rn<false>(a[j], d);
+                lmax = fmaxf(lmax, cabs1f(a[j]));
+            }
+#pragma unroll
+            for (int x = j + 1; x < 4; ++x)
+                a[x] = ROW ? submul_rn<false>(a[x], a[j], D[(b + x) * kSpLD + b + j])
+                           : submul_rn<false>(a[x], D[(b + j) * kSpLD + b + x], a[j]);
+        }
+#pragma unroll
+        for (int g = 4; g < kSpNW; g += 4) {
+            if (b + g >= kSpNW) break;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int x = g; x < g + 4; ++x)
+                    a[x] = ROW ? submul_rn<false>(a[x], a[j], D[(b + x) * kSpLD + b + j])
+                               : submul_rn<false>(a[x], D[(b + j) * kSpLD + b + x], a[j]);
+        }
+        cf turn[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) turn[x] = a[x];
+#pragma unroll
+        for (int x = 0; x + 4 < kSpNW; ++x) a[x] = a[x + 4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) a[kSpNW - 4 + x] = turn[x];
+    }
+#pragma unroll
+    for (int x = 0; x < kSpNW; ++x) p[x * step] = a[x];
+    return lmax;
+}
+
+// The block in S without interchanges (all threads); false when a pivot is
+// zero or a multiplier exceeds the bound (S is then half factored).  Rows and
+// columns from jb on must hold the identity.  s_bad: two flags, cleared.
+__device__ __forceinline__ bool sp_nopivot(cf* S, int jb, cf* s_inv, int* s_bad) {
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform, and known to be)
+    const int jr = (jb + kSpNW - 1) / kSpNW * kSpNW;
+    for (int c0 = 0; c0 < jr; c0 += kSpNW) {
+        const int left = jr - c0;
+        if (warp == 0) {
+            if (sp_sub16(S, c0, c0 - kSpNW, s_inv)) s_bad[0] = 1;
+        } else if (c0 > 0) {
+            // once the rest is quicker than the sub-block, the warps that
+            // share the first one's scheduler (every fourth) leave it alone
+            if (left > 80)
+                sp_rank16_rest(S, c0 - kSpNW, jr, tid - 32, kSpDiagThreads - 32);
+            else if (warp & 3)
+                sp_rank16_rest(S, c0 - kSpNW, jr, (warp - 1 - warp / 4) * 32 + (tid & 31), kSpDiagThreads / 4 * 3);
+        }
+        __syncthreads();
+        if (s_bad[0]) return false;
+        const int t0 = c0 + kSpNW;
+        if (t0 >= jr) break;
+        // L below the sub-block (a row to a thread), U right of it (a column
+        // to a thread)
+        if (tid < kSpB) {
+            const int R = t0 + tid;
+            if (R < jr) {
+                const float lmax =
+                    sp_solve16<true>(S, c0, S + c0 * kSpLD + R, kSpLD, s_inv + c0, R / kSpPW == c0 / kSpPW);
+                if (!(lmax <= kSpNoPivotBound)) s_bad[1] = 1;
+            }
+        } else if (tid < 2 * kSpB) {
+            const int q = t0 + tid - kSpB;
+            if (q < jr) sp_solve16<false>(S, c0, S + q * kSpLD + c0, 1, nullptr, false);
+        }
+        __syncthreads();
+        if (s_bad[1]) return false;
+    }
+    return true;
+}
 
 __global__ void __launch_bounds__(kSpDiagThreads, 1)
     sp_diag_kernel(cf* __restrict__ A, int64_t lda, int64_t j0, int jb, int32_t* __restrict__ ipiv,
@@ -144,84 +395,27 @@ __global__ void __launch_bounds__(kSpDiagThreads, 1)
     __shared__ cf s_rc[2][kSpPW];                 // row c's panel values before the interchange
     __shared__ int s_row_at[kSpB];                // original row at each position
     __shared__ cf s_inv[kSpB];
-    __shared__ int s_bad;
+    __shared__ int s_bad[2];
     const int tid = threadIdx.x;
     const int lane = tid & 31;
-    for (int base = 0; base < kSpB * kSpB; base += 8 * kSpDiagThreads) {
-        cf t[8];
+    for (int base = 0; base < kSpB * kSpB; base += 16 * kSpDiagThreads) {
+        cf t[16];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < 16; ++u) {
             const int idx = base + u * kSpDiagThreads + tid;
             const int rr = idx % kSpB, col = idx / kSpB;
-            t[u] = (rr < jb && col < jb) ? A[(j0 + rr) + (j0 + col) * lda] : cf{0.0f, 0.0f};
+            // (a partial block's padding: the identity)
+            t[u] = (rr < jb && col < jb) ? A[(j0 + rr) + (j0 + col) * lda] : cf{rr == col ? 1.0f : 0.0f, 0.0f};
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < 16; ++u) {
             const int idx = base + u * kSpDiagThreads + tid;
             S[(idx / kSpB) * kSpLD + idx % kSpB] = t[u];
         }
     }
-    if (tid == 0) s_bad = 0;
+    if (tid < 2) s_bad[tid] = 0;
     __syncthreads();
-    // ---- without interchanges
-    for (int c0 = 0; c0 < jb; c0 += kSpPW) {
-        const int nck = (jb - c0) < kSpPW ? (jb - c0) : kSpPW;
-        const int warp = tid >> 5;
-        float lmax = 0.0f;
-        bool bad = false;
-        // (1) the panel's 32 x 32 diagonal sub-block by warp 0, lane = row
-        // c0 + lane: the pivot row is read in place (broadcast), one warp
-        // synchronisation per column
-        if (warp == 0) {
-            cf* row = S + c0 + lane;
-            for (int cc = 0; cc < nck; ++cc) {
-                __syncwarp();
-                const int c = c0 + cc;
-                const cf piv = S[c * kSpLD + c];
-                const float pa = cabs1f(piv);
-                bad = bad || !(pa > 0.0f);
-                const cf inv = pa > 0.0f ? crcp_sp(piv) : cone<cf>();
-                if (lane == cc) s_inv[c] = inv;
-                if (lane > cc && lane < nck) {
-                    const cf l = row[c * kSpLD] * inv;
-                    row[c * kSpLD] = l;
-                    lmax = fmaxf(lmax, cabs1f(l));
-#pragma unroll 4
-                    for (int q = cc + 1; q < nck; ++q)
-                        row[(c0 + q) * kSpLD] = row[(c0 + q) * kSpLD] - l * S[(c0 + q) * kSpLD + c];
-                }
-            }
-        }
-        __syncthreads();
-        // (2) in parallel: the rows below the sub-block, L = A U11^-1 (warps
-        // 0-3, a row each, right-looking along the row), and the columns
-        // right of it, U12 = L11^-1 A12 (warps 4-7, a column each)
-        const int t0 = c0 + kSpPW;
-        if (tid < kSpB) {
-            const int R = t0 + tid;
-            if (R < jb) {
-                cf* row = S + R;
-                for (int jj = 0; jj < nck; ++jj) {
-                    const cf l = row[(c0 + jj) * kSpLD] * s_inv[c0 + jj];
-                    row[(c0 + jj) * kSpLD] = l;
-                    lmax = fmaxf(lmax, cabs1f(l));
-#pragma unroll 4
-                    for (int q = jj + 1; q < nck; ++q)
-                        row[(c0 + q) * kSpLD] = row[(c0 + q) * kSpLD] - l * S[(c0 + q) * kSpLD + c0 + jj];
-                }
-            }
-        } else if (tid < 2 * kSpB) {
-            sp_u12(S, c0, jb, tid - kSpB);
-        }
-        // NaN-safe: a NaN multiplier fails the comparison
-        if (bad || !(lmax <= kSpNoPivotBound)) atomicOr(&s_bad, 1);
-        __syncthreads();
-        if (s_bad) break;
-        // (3) the trailing block
-        sp_a22(S, c0, jb, tid);
-        __syncthreads();
-    }
-    if (!s_bad) {
+    if (sp_nopivot(S, jb, s_inv, s_bad)) {
         for (int c = tid; c < jb; c += kSpDiagThreads) {
             ipiv[j0 + c] = (int32_t)(j0 + c + 1);
             inv_diag[c] = s_inv[c];
@@ -341,6 +535,7 @@ __global__ void __launch_bounds__(kSpDiagThreads, 1)
         if (tid < jb) perm[tid] = s_row_at[tid];
     }
     __syncthreads();
+#pragma unroll 8
     for (int base = 0; base < kSpB * kSpB; base += kSpDiagThreads) {
         const int idx = base + tid;
         const int rr = idx % kSpB, col = idx / kSpB;
@@ -374,35 +569,81 @@ __global__ void __launch_bounds__(256) sp_permute_kernel(cf* __restrict__ A, int
     }
 }
 
-// L21 = A21 U11^-1 for the rows below the diagonal block.  Four warps share
-// 32 rows: lane i holds row i, warp w its columns 32w .. 32w+31 in
-// registers.  The solve proceeds by column chunks: in phase k warp k
-// finishes chunk k lane-locally (x_j = a_j / U_jj, then a_l -= x_j U_jl for
-// the later columns of the chunk) and publishes it in shared memory; after
-// one barrier the warps of later chunks remove it from theirs (a 32 x 32
-// block product per lane).  No shuffles, no divergence; U11 (upper
-// triangle of the factored block) is staged row-major in shared memory and
-// read as broadcasts.  The largest |L21| goes to ws->lmax_bits.
-constexpr int kSpGroups = 2;                     // 32-row groups per CTA
-constexpr int kSpL21Threads = 32 * 4 * kSpGroups;
-constexpr int kSpXStride = 33;                   // complex elements per row of the exchange buffer
+// L21 = A21 U11^-1 for the rows below the diagonal block.  A warp solves
+// eight rows by itself, no barrier after U11 is staged: 16 columns at a time,
+// eight lanes to a row pair, lane (p, f) holding columns 2f, 2f + 1 of rows
+// 2p, 2p + 1.  The columns solved before are removed first (x from the
+// warp's strip of shared memory, U11 row-major there), then the chunk is
+// solved with x_j passed on by shuffles.  The CTA takes as many rows as
+// spread the panel evenly over the chip, up to kSpL21Warps warps' worth; its
+// other warps only help to stage U11 (64 KB from L2).  Bound by the FP32
+// pipe: 6 operations per update, 128 x 128 / 2 updates a row.  The largest
+// |L21| goes to ws->lmax_bits.
+// Four warps to 32 rows, handing solved chunks of 32 columns over through
+// block barriers, took 61 us a launch on B200 (mean over a 2835-unknown
+// matrix); 25 us so.
+constexpr int kSpChunk = 16;      // columns at a time
+constexpr int kSpWarpRows = 8;    // rows of a warp
+constexpr int kSpL21Warps = 11;   // warps of a CTA: the strips of x fill the shared memory beside U11
+constexpr int kSpSMs = 148;
+constexpr int kSpL21Threads = 32 * kSpL21Warps;
+constexpr size_t kSpL21Smem =
+    sizeof(cf) * ((size_t)kSpB * kSpUStride + kSpB + (size_t)kSpL21Warps * kSpWarpRows * kSpUStride);
 
-__device__ __forceinline__ void load_u2(const cf* __restrict__ src, cf& u0, cf& u1) {
-    const float4 v = *reinterpret_cast<const float4*>(src);
-    u0 = cf{v.x, v.y};
-    u1 = cf{v.z, v.w};
+__device__ __forceinline__ void load2(const cf* __restrict__ src, cf (&v)[2]) {
+    const float4 w = *reinterpret_cast<const float4*>(src);
+    v[0] = cf{w.x, w.y};
+    v[1] = cf{w.z, w.w};
+}
+
+// Columns [j0, j1) (even) of x removed from the lane's entries; x0 and x1 are
+// its two rows in the strip, u its columns of U11.  NEAR: the columns lie in
+// the chunk's own group of 32.
+template <bool NEAR>
+__device__ __forceinline__ void sp_l21_remove(cf (&a)[2][2], const cf* x0, const cf* x1, const cf* u, int j0, int j1) {
+#pragma unroll 2
+    for (int j = j0; j < j1; j += 2) {
+        cf x[2][2], ua[2], ub[2];
+        load2(x0 + j, x[0]);
+        load2(x1 + j, x[1]);
+        load2(u + (size_t)j * kSpUStride, ua);
+        load2(u + (size_t)(j + 1) * kSpUStride, ub);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            a[r][0] = submul_rn<NEAR>(a[r][0], x[r][0], ua[0]);
+            a[r][1] = submul_rn<false>(a[r][1], x[r][0], ua[1]);
+            a[r][0] = submul_rn<NEAR>(a[r][0], x[r][1], ub[0]);
+            a[r][1] = submul_rn<false>(a[r][1], x[r][1], ub[1]);
+        }
+    }
 }
 
 __global__ void __launch_bounds__(kSpL21Threads, 1)
-    sp_l21_kernel(cf* __restrict__ A, int64_t lda, int64_t j0, int jb, int64_t row_end,
+    sp_l21_kernel(cf* __restrict__ A, int64_t lda, int64_t j0, int jb, int64_t row_end, int64_t row_pad, int rows_cta,
                   const cf* __restrict__ inv_diag, PanelWs* ws, float* __restrict__ a_hi, float* __restrict__ a_lo) {
     extern __shared__ __align__(16) unsigned char sp_smem[];
-    cf* sU = reinterpret_cast<cf*>(sp_smem);                 // [kSpB][kSpUStride]
-    cf* sInv = sU + (size_t)kSpB * kSpUStride;               // [kSpB]
-    cf* sX = sInv + kSpB;                                    // [2][kSpGroups][32][kSpXStride]
-    const int tid = threadIdx.x;
-    // staged with sixteen loads in flight per thread before the stores
-    constexpr int kU = 16;
+    cf* sU = reinterpret_cast<cf*>(sp_smem);       // [kSpB][kSpUStride]
+    cf* sX = sU + (size_t)kSpB * kSpUStride;       // [rows of the CTA][kSpUStride]
+    cf* sInv = sX + (size_t)kSpL21Warps * kSpWarpRows * kSpUStride;  // [kSpB]
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int p = lane >> 3, f = lane & 7;
+    const int64_t base_row = j0 + jb + (int64_t)blockIdx.x * rows_cta;
+    const int64_t row = base_row + warp * kSpWarpRows + 2 * p;
+    const bool work = warp * kSpWarpRows < rows_cta && base_row + warp * kSpWarpRows < row_pad;
+    const int nchunks = (jb + kSpChunk - 1) / kSpChunk;
+    cf nxt[2][2];
+    auto fetch = [&](int k) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int col = kSpChunk * k + 2 * f + c;
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+                nxt[r][c] = (work && row + r < row_end && col < jb) ? A[row + r + (j0 + col) * lda] : cf{0.0f, 0.0f};
+        }
+    };
+    fetch(0);
+    // staged with eight loads in flight per thread before the stores
+    constexpr int kU = 8;
     for (int base = 0; base < kSpB * kSpB; base += kU * kSpL21Threads) {
         cf t[kU];
 #pragma unroll
@@ -418,74 +659,53 @@ __global__ void __launch_bounds__(kSpL21Threads, 1)
         }
     }
     for (int j = tid; j < kSpB; j += blockDim.x) sInv[j] = j < jb ? inv_diag[j] : cf{0.0f, 0.0f};
-    const int lane = tid & 31, warp = tid >> 5;
-    const int w = warp & 3;          // column chunk of this warp
-    const int grp = warp >> 2;       // 32-row group
-    const int64_t row = j0 + jb + ((int64_t)blockIdx.x * kSpGroups + grp) * 32 + lane;
-    const bool row_ok = row < row_end;
-    cf a[32];
-#pragma unroll
-    for (int l = 0; l < 32; ++l) {
-        const int col = 32 * w + l;
-        a[l] = (row_ok && col < jb) ? A[row + (j0 + col) * lda] : cf{0.0f, 0.0f};
-    }
     __syncthreads();
+    if (!work) return;
+    cf* x0 = sX + (size_t)(warp * kSpWarpRows + 2 * p) * kSpUStride;
+    cf* x1 = x0 + kSpUStride;
+    const int n_ks = tc_n_ks(jb);
     float lmax = 0.0f;
-    const int nchunks = (jb + 31) / 32;
     for (int k = 0; k < nchunks; ++k) {
-        cf* xb = sX + ((size_t)((k & 1) * kSpGroups + grp) * 32 + lane) * kSpXStride;
-        if (w == k) {
+        const int c0 = kSpChunk * k, g0 = c0 / kSpPW * kSpPW;
+        cf a[2][2] = {{nxt[0][0], nxt[0][1]}, {nxt[1][0], nxt[1][1]}};
+        if (k + 1 < nchunks) fetch(k + 1);
+        const cf* u = sU + c0 + 2 * f;
+        sp_l21_remove<false>(a, x0, x1, u, 0, g0);
+        sp_l21_remove<true>(a, x0, x1, u, g0, c0);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const cf* urow = sU + (size_t)(32 * k + j) * kSpUStride + 32 * k;
-                const cf x = a[j] * sInv[32 * k + j];
-                a[j] = x;
-                lmax = fmaxf(lmax, cabs1f(x));
+        for (int j = 0; j < kSpChunk; ++j) {
+            cf uj[2], x[2];
+            load2(u + (size_t)(c0 + j) * kSpUStride, uj);
+            const cf inv = sInv[c0 + j];
+            const int src = (lane & ~7) | (j / 2);
 #pragma unroll
-                for (int l0 = (j + 1) & ~1; l0 < 32; l0 += 2) {
-                    cf u0, u1;
-                    load_u2(urow + l0, u0, u1);
-                    if (l0 > j) a[l0] = a[l0] - x * u0;
-                    a[l0 + 1] = a[l0 + 1] - x * u1;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) xb[j] = a[j];
-        }
-        __syncthreads();
-        if (w > k) {
-            for (int j = 0; j < 32; ++j) {
-                const cf* urow = sU + (size_t)(32 * k + j) * kSpUStride + 32 * w;
-                const cf x = xb[j];
-#pragma unroll
-                for (int l0 = 0; l0 < 32; l0 += 2) {
-                    cf u0, u1;
-                    load_u2(urow + l0, u0, u1);
-                    a[l0] = a[l0] - x * u0;
-                    a[l0 + 1] = a[l0 + 1] - x * u1;
-                }
+            for (int r = 0; r < 2; ++r) {
+                const cf t = mul_rn<false>(a[r][j & 1], inv);
+                if (f == j / 2) a[r][j & 1] = t;
+                x[r] = cf{__shfl_sync(0xffffffffu, t.re, src), __shfl_sync(0xffffffffu, t.im, src)};
+                if (2 * f > j) a[r][0] = submul_rn<true>(a[r][0], x[r], uj[0]);
+                if (2 * f + 1 > j) a[r][1] = submul_rn<false>(a[r][1], x[r], uj[1]);
             }
         }
-    }
-    if (row_ok) {
+        *reinterpret_cast<float4*>(x0 + c0 + 2 * f) = make_float4(a[0][0].re, a[0][0].im, a[0][1].re, a[0][1].im);
+        *reinterpret_cast<float4*>(x1 + c0 + 2 * f) = make_float4(a[1][0].re, a[1][0].im, a[1][1].re, a[1][1].im);
+        __syncwarp();
+        // a packed row: each complex l is the 2 x 2 block [[re, -im], [im, re]]
+        // of the trailing updates' operand (rows from j0 + jb, inner dimension
+        // jb); rows past the matrix and columns past jb hold zeros, so that
+        // the tiles they pad contribute nothing
+        const int64_t kap4 = 2 * (c0 + 2 * f);
 #pragma unroll
-        for (int l = 0; l < 32; ++l) {
-            const int col = 32 * w + l;
-            if (col < jb) A[row + (j0 + col) * lda] = a[l];
-        }
-    }
-    if (a_hi != nullptr) {
-        // L21 also as the packed operand of the trailing updates (rows from
-        // j0 + jb, inner dimension jb): each complex l is the 2 x 2 block
-        // [[re, -im], [im, re]]; rows past the matrix and columns past jb
-        // hold zeros, so that the tiles they pad contribute nothing
-        const int n_ks = tc_n_ks(jb);
-        const int64_t rho = 2 * (row - (j0 + jb));
+        for (int r = 0; r < 2; ++r) {
+            const cf v0 = a[r][0], v1 = a[r][1];
+            lmax = fmaxf(lmax, fmaxf(cabs1f(v0), cabs1f(v1)));
+            if (row + r < row_end) {
 #pragma unroll
-        for (int l = 0; l < 32; l += 2) {
-            const int64_t kap4 = 2 * (32 * w + l);
-            if (kap4 < (int64_t)n_ks * TC_KS) {
-                const cf v0 = a[l], v1 = a[l + 1];
+                for (int c = 0; c < 2; ++c)
+                    if (c0 + 2 * f + c < jb) A[row + r + (j0 + c0 + 2 * f + c) * lda] = a[r][c];
+            }
+            if (a_hi != nullptr && kap4 < (int64_t)n_ks * TC_KS) {
+                const int64_t rho = 2 * (row + r - (j0 + jb));
                 tc_store_a4(a_hi, a_lo, n_ks, rho, kap4, make_float4(v0.re, -v0.im, v1.re, -v1.im));
                 tc_store_a4(a_hi, a_lo, n_ks, rho + 1, kap4, make_float4(v0.im, v0.re, v1.im, v1.re));
             }
@@ -509,9 +729,9 @@ mw_status static_panel_c64(cf* A, int64_t lda, int64_t n, int64_t j0, int jb, in
                            PanelWs* ws, cf* inv_diag, int32_t* perm, const TcPlanes* pack_a, cudaStream_t st) {
     MW_REQUIRE(jb >= 1 && jb <= kSpB, "static panel width %d outside 1..%d", jb, kSpB);
     static bool configured = false;
-    const size_t smem = sizeof(cf) * ((size_t)kSpB * kSpUStride + kSpB + (size_t)2 * kSpGroups * 32 * kSpXStride);
     if (!configured) {
-        MW_CHECK_CUDA(cudaFuncSetAttribute(sp_l21_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        MW_CHECK_CUDA(cudaFuncSetAttribute(sp_l21_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)kSpL21Smem));
         MW_CHECK_CUDA(cudaFuncSetAttribute(sp_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)kSpDiagSmem));
         configured = true;
@@ -525,11 +745,15 @@ mw_status static_panel_c64(cf* A, int64_t lda, int64_t n, int64_t j0, int jb, in
         const int64_t rows = n - j0 - jb;
         ProfileScope ps(PC_L21, st, 4.0 * (double)rows * jb * jb, 16.0 * (double)rows * jb);
         if (rows > 0) {
-            const int64_t per_cta = (int64_t)kSpGroups * 32;
-            const unsigned grid = (unsigned)((rows + per_cta - 1) / per_cta);
-            sp_l21_kernel<<<grid, kSpL21Threads, smem, st>>>(A, lda, j0, jb, n, inv_diag, ws,
-                                                             pack_a ? pack_a->a_hi : nullptr,
-                                                             pack_a ? pack_a->a_lo : nullptr);
+            // the packed operand's last tile is written whole (64 rows), and
+            // the rows are spread evenly over whole waves of CTAs, one to an SM
+            const int64_t pad = (rows + 63) / 64 * 64, full = (int64_t)kSpL21Warps * kSpWarpRows * kSpSMs;
+            const int64_t ctas = (pad + full - 1) / full * kSpSMs;
+            const int64_t per_cta = (pad + ctas * kSpWarpRows - 1) / (ctas * kSpWarpRows) * kSpWarpRows;
+            const unsigned grid = (unsigned)((pad + per_cta - 1) / per_cta);
+            sp_l21_kernel<<<grid, kSpL21Threads, kSpL21Smem, st>>>(
+                A, lda, j0, jb, n, j0 + jb + pad, (int)per_cta, inv_diag, ws, pack_a ? pack_a->a_hi : nullptr,
+                pack_a ? pack_a->a_lo : nullptr);
             count_launch();
         }
     }
