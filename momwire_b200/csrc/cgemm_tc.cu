@@ -202,9 +202,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) cgemm_tc_kernel(TcArgs P) {
     } else {
         // ------------------------------------------------ epilogue (warps 2..)
         const int quad = warp & 3;  // TMEM lane quadrant this warp may access
-        // with eight epilogue warps, two share a quadrant and split its columns
-        constexpr int kCols = TC_N * 4 / TC_EPI_WARPS;
-        const int cbeg = ((warp - 2) / 4) * kCols;
+        // with eight epilogue warps, two share a quadrant and split the
+        // columns that the tile has evenly, 32 to a round
+        constexpr int kGroups = TC_EPI_WARPS / 4;
+        const int group = (warp - 2) / 4;
+        const int64_t cstep = 2 * P.ldc;
         uint32_t ph_accf[2] = {0, 0};
         bool dead = false;
         int lt = 0;
@@ -220,22 +222,38 @@ __global__ void __launch_bounds__(TC_THREADS, 1) cgemm_tc_kernel(TcArgs P) {
             tc_fence_after();
             const int64_t r = (int64_t)mb * TC_M + quad * 32 + lane;  // real row
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * TC_N;
-            // 32 columns per round: all loads of C issue before any store so
-            // that they overlap (a store may alias the next load otherwise)
-            for (int c0 = cbeg; c0 < cbeg + kCols; c0 += 32) {
+            const int64_t left = P.n - (int64_t)nb * TC_N;
+            const int used = left < TC_N ? (int)left : TC_N;
+            const int share = (used + 32 * kGroups - 1) / (32 * kGroups) * 32;
+            const int cbeg = group * share, cend = min(cbeg + share, used);
+            const int64_t row0 = (int64_t)mb * TC_M + quad * 32;
+            float* ctile = P.C + (int64_t)bt * P.c_stride + r + (int64_t)nb * TC_N * cstep;
+            // all loads of C of a round issue before any store so that they
+            // overlap (a store may alias the next load otherwise); rounds
+            // with every row and column present, nearly all of them, carry no
+            // predicates, and rounds past the last column are not run.  With 64-bit
+            // tests and products per element in all 256 columns, instructions
+            // bounded it: 66 us on B200 for 1344 tiles of 48 columns at k = 16
+            // (29 so), 101 for 256 columns (92), 513 for 10240^2 at k = 128 (490)
+            for (int c0 = cbeg; c0 < cend; c0 += 32) {
                 float v[32], old[32];
                 tmem_ld16(taddr + c0, v);
                 tmem_ld16(taddr + c0 + 16, v + 16);
-                const int64_t col0 = (int64_t)nb * TC_N + c0;
-                const bool row_ok = r < P.m_real;
-                float* cbase = P.C + (int64_t)bt * P.c_stride + r + col0 * 2 * P.ldc;
-                const int64_t cstep = 2 * P.ldc;
+                float* cbase = ctile + c0 * cstep;
+                if (c0 + 32 <= cend && row0 + 32 <= P.m_real) {
+                    const float* src = cbase;
 #pragma unroll
-                for (int e = 0; e < 32; ++e)
-                    old[e] = (row_ok && col0 + e < P.n) ? __ldcs(cbase + e * cstep) : 0.f;
+                    for (int e = 0; e < 32; ++e, src += cstep) old[e] = __ldcs(src);
 #pragma unroll
-                for (int e = 0; e < 32; ++e)
-                    if (row_ok && col0 + e < P.n) __stcs(cbase + e * cstep, old[e] - v[e]);
+                    for (int e = 0; e < 32; ++e, cbase += cstep) __stcs(cbase, old[e] - v[e]);
+                } else if (r < P.m_real) {
+                    const float* src = cbase;
+#pragma unroll
+                    for (int e = 0; e < 32; ++e, src += cstep) old[e] = c0 + e < cend ? __ldcs(src) : 0.f;
+#pragma unroll
+                    for (int e = 0; e < 32; ++e, cbase += cstep)
+                        if (c0 + e < cend) __stcs(cbase, old[e] - v[e]);
+                }
             }
             tc_fence_before();
             __syncwarp();
@@ -291,40 +309,44 @@ __global__ void pack_a_kernel(const cf* __restrict__ A, int64_t lda, int64_t m, 
 }
 
 // Breal^T (n x 2k, from complex B at B + (l + j*ldb)) packed as
-// [nb][ks][chunk TC_CHUNKS][row 256][4]; zero beyond (n, 2k).
-__global__ void pack_b_kernel(const cf* __restrict__ B, int64_t ldb, int64_t k, int64_t n, int n_nb, int n_ks,
-                              float* __restrict__ hi, float* __restrict__ lo, int64_t b_stride, int64_t p_stride) {
-    const int64_t total = (int64_t)n_nb * n_ks * TC_CHUNKS * TC_N;
+// [nb][ks][chunk TC_CHUNKS][row 256][4]; zero beyond (n, 2k).  A block takes
+// 32 columns x 64 rows of B through shared memory, so that reads run down the
+// columns and writes along the plane.  A thread per float4 of the plane, its
+// reads a column apart, took 13.1 us at k = 128, n = 10240 on B200 and 11 us
+// for 192 matrices with k = 64, n <= 430; 7.0 and 7 us so.
+constexpr int kPackCols = 32, kPackRows = 64;
+__global__ void __launch_bounds__(256)
+    pack_b_kernel(const cf* __restrict__ B, int64_t ldb, int k, int64_t n, int n_nb, int n_ks, float* __restrict__ hi,
+                  float* __restrict__ lo, int64_t b_stride, int64_t p_stride) {
+    __shared__ cf tile[kPackRows][kPackCols + 1];
     B += blockIdx.y * b_stride;  // batch entry
     hi += blockIdx.y * p_stride;
     lo += blockIdx.y * p_stride;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-        const int row = (int)(q % TC_N);
-        int64_t rest = q / TC_N;
-        const int ch = (int)(rest % TC_CHUNKS);
-        rest /= TC_CHUNKS;
-        const int ks = (int)(rest % n_ks);
-        const int nb = (int)(rest / n_ks);
-        const int64_t j = (int64_t)nb * TC_N + row;
-        const int64_t kap0 = (int64_t)ks * TC_KS + ch * 4;
-        float4 vh, vl;
-        float* ph = &vh.x;
-        float* pl = &vl.x;
+    const int ncg = n_nb * (TC_N / kPackCols);
+    const int64_t jbase = (int64_t)(blockIdx.x % ncg) * kPackCols;
+    const int l0 = (blockIdx.x / ncg) * kPackRows;
+    const int tl = threadIdx.x & 63, tj = threadIdx.x >> 6;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int64_t kap = kap0 + e;
-            float x = 0.f;
-            if (j < n && kap < 2 * k) {
-                const cf b = B[(kap >> 1) + j * ldb];
-                x = (kap & 1) ? b.im : b.re;
-            }
-            const float h = tf32_hi(x);
-            ph[e] = h;
-            pl[e] = x - h;
-        }
-        reinterpret_cast<float4*>(hi)[q] = vh;
-        reinterpret_cast<float4*>(lo)[q] = vl;
+    for (int u = 0; u < kPackCols / 4; ++u) {
+        const int64_t j = jbase + tj + 4 * u;
+        tile[tl][tj + 4 * u] = (j < n && l0 + tl < k) ? B[(l0 + tl) + j * ldb] : cf{0.f, 0.f};
     }
+    __syncthreads();
+    const int pairs = n_ks * TC_CHUNKS;
+    const int col = threadIdx.x & 31;
+    const int64_t nb = jbase / TC_N;
+    const int row = (int)(jbase % TC_N) + col;
+#pragma unroll
+    for (int u = 0; u < kPackRows / 2 / 8; ++u) {
+        const int c = (threadIdx.x >> 5) + 8 * u, cp = l0 / 2 + c;
+        if (cp >= pairs) break;
+        const cf a = tile[2 * c][col], b = tile[2 * c + 1][col];
+        tc_split_store(hi, lo, (nb * pairs + cp) * TC_N + row, make_float4(a.re, a.im, b.re, b.im));
+    }
+}
+
+static unsigned pack_b_blocks(int n_nb, int n_ks) {
+    return (unsigned)n_nb * (TC_N / kPackCols) * (unsigned)((n_ks * TC_CHUNKS + kPackRows / 2 - 1) / (kPackRows / 2));
 }
 
 size_t tc_pack_a_bytes(int64_t m, int64_t k) {
@@ -357,10 +379,11 @@ mw_status cgemm_tc_update_batched(int64_t m, int64_t n, int64_t k, int batch, co
     float* b_lo = reinterpret_cast<float*>(w + 2 * al(ab * batch) + al(bb * batch));
     {
         ProfileScope ps(PC_MISC, st);
-        int64_t qa = (int64_t)n_mb * n_ks * TC_CHUNKS * TC_M, qb = (int64_t)n_nb * n_ks * TC_CHUNKS * TC_N;
-        dim3 ga((unsigned)((qa + 255) / 256), (unsigned)batch), gb((unsigned)((qb + 255) / 256), (unsigned)batch);
+        MW_REQUIRE(k < (1 << 30), "inner dimension too large");
+        const int64_t qa = (int64_t)n_mb * n_ks * TC_CHUNKS * TC_M;
+        const dim3 ga((unsigned)((qa + 255) / 256), (unsigned)batch), gb(pack_b_blocks(n_nb, n_ks), (unsigned)batch);
         pack_a_kernel<<<ga, 256, 0, st>>>(A, lda, m, k, n_mb, n_ks, a_hi, a_lo, sa, (int64_t)(ab / 4));
-        pack_b_kernel<<<gb, 256, 0, st>>>(B, ldb, k, n, n_nb, n_ks, b_hi, b_lo, sb, (int64_t)(bb / 4));
+        pack_b_kernel<<<gb, 256, 0, st>>>(B, ldb, (int)k, n, n_nb, n_ks, b_hi, b_lo, sb, (int64_t)(bb / 4));
         count_launch(2);
     }
     static int sms = 0;

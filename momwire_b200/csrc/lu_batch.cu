@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kBThreads) panel1_kernel(cf* A, int64_t lda, i
     __shared__ int s_i[kBThreads / 32];
     __shared__ int s_p;
     __shared__ double s_pv;
-    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     A += (int64_t)b * stride;
     ipiv += (int64_t)b * n;
     const int m = n - j0;

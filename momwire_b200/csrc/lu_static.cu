@@ -7,11 +7,11 @@
 // Demmel 1998: factor with pivots chosen locally, recover accuracy by
 // iterative refinement): the panel no longer needs a pivot search over all
 // the rows below it, so it has no grid-wide exchange per column.  A panel is
-//   sp_diag_kernel  one CTA factors the diagonal block in registers with
-//                   partial pivoting among its own rows (row interchanges
-//                   kept as a row arrangement, written back once), and
+//   sp_diag_kernel  one CTA factors the diagonal block in shared memory,
+//                   without interchanges where it can and with partial
+//                   pivoting among its own rows where it must, and
 //   sp_l21_kernel   every row below is solved against the block's upper
-//                   factor, L21 = A21 U11^-1, four warps per 32 rows.
+//                   factor, L21 = A21 U11^-1, eight rows to a warp.
 // The growth the restriction allows is measured: sp_l21_kernel raises the
 // largest |L21| (|re| + |im|) into PanelWs::lmax_bits, and an exact zero
 // pivot sets it to +inf.  The caller refactors with full partial pivoting
