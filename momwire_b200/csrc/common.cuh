@@ -49,6 +49,25 @@ __host__ __device__ __forceinline__ cf cdiv(cf a, cf b) {
 }
 __host__ __device__ __forceinline__ double cabs1(cd z) { return fabs(z.re) + fabs(z.im); }
 __host__ __device__ __forceinline__ double cabs1(cf z) { return (double)fabsf(z.re) + (double)fabsf(z.im); }
+#ifdef __CUDACC__
+// a b and v - a b with their roundings spelled out: a complex product has two
+// contracted forms of its imaginary part, and which one the compiler takes
+// depends on the code around it.  FIRST rounds the product a.im b.re before
+// the fused a.re b.im; otherwise the other way round.  Kernels that must give
+// the same bits whatever their tiling use these.
+template <bool FIRST>
+__device__ __forceinline__ cf mul_rn(cf a, cf b) {
+    const float re = __fmaf_rn(a.re, b.re, -__fmul_rn(a.im, b.im));
+    const float im = FIRST ? __fmaf_rn(a.re, b.im, __fmul_rn(a.im, b.re))
+                           : __fmaf_rn(a.im, b.re, __fmul_rn(a.re, b.im));
+    return cf{re, im};
+}
+template <bool FIRST>
+__device__ __forceinline__ cf submul_rn(cf v, cf a, cf b) {
+    const cf p = mul_rn<FIRST>(a, b);
+    return cf{__fsub_rn(v.re, p.re), __fsub_rn(v.im, p.im)};
+}
+#endif
 template <class T> __host__ __device__ __forceinline__ T cone();
 template <> __host__ __device__ __forceinline__ cd cone<cd>() { return cd{1.0, 0.0}; }
 template <> __host__ __device__ __forceinline__ cf cone<cf>() { return cf{1.0f, 0.0f}; }

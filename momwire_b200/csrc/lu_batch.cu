@@ -75,9 +75,9 @@ __global__ void __launch_bounds__(kBThreads) panel1_kernel(cf* A, int64_t lda, i
             for (int off = 16; off > 0; off >>= 1)
                 amax_merge(best, bi, __shfl_xor_sync(0xffffffffu, best, off), __shfl_xor_sync(0xffffffffu, bi, off));
             if (lane == 0) {
-                s_p = bi;
+                s_p = bi < m ? bi : jj;  // nothing but NaN: no interchange
                 s_pv = best;
-                ipiv[j0 + jj] = j0 + bi + 1;
+                ipiv[j0 + jj] = j0 + s_p + 1;
             }
         }
         __syncthreads();
@@ -108,6 +108,124 @@ __global__ void __launch_bounds__(kBThreads) panel1_kernel(cf* A, int64_t lda, i
     }
 }
 
+// The panel with a row to a thread, its W columns (>= jb) in registers: slot 0
+// is the current column, the slots turn by one per column (W turns put them
+// back).  Each warp offers its largest entry with that row; after one barrier
+// every thread knows the pivot.  Bound by the chain of jb columns (the pivot
+// search over m <= NT rows, a complex reciprocal) and, with one or two CTAs an
+// SM, by the slots' updates.  From the slab in shared memory with four
+// barriers a column this took 75 us at m = 437, jb = 16, 192 matrices, on
+// B200; 30 us so
+// (@PANELX@)  Entry for entry the slab's operations (mul_rn and
+// submul_rn spell its roundings out).
+template <int W, int NT>
+__global__ void __launch_bounds__(NT) panel_rows_kernel(cf* A, int64_t lda, int64_t stride, int n, int j0, int jb,
+                                                        int32_t* ipiv, int32_t* info) {
+    __shared__ __align__(16) cf s_cand[2][NT / 32][W];  // a warp's candidate row
+    __shared__ __align__(16) cf s_cur[2][W];            // row jj itself
+    __shared__ unsigned s_hi[2][32], s_lo[2][32];
+    __shared__ int s_row[2][32];
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0), warps = blockDim.x / 32;
+    A += (int64_t)b * stride + j0 + tid + (int64_t)j0 * lda;
+    ipiv += (int64_t)b * n;
+    const int m = n - j0;
+    const bool live = tid < m;
+    cf a[W];
+#pragma unroll
+    for (int x = 0; x < W; ++x) a[x] = (live && x < jb) ? A[x * lda] : cf{0.f, 0.f};
+#pragma unroll 1
+    for (int jj = 0; jj < W; ++jj) {
+        cf last = a[0];
+        bool upd = false;
+        cf l{0.f, 0.f};
+        const cf* u = s_cand[0][0];
+        if (jj < jb) {
+            const int par = jj & 1;
+            // (a NaN is never the pivot; 0 marks rows that are no candidates)
+            const double v = cabs1(a[0]);
+            const unsigned long long key =
+                (live && tid >= jj && v >= 0.0) ? (unsigned long long)__double_as_longlong(v) + 1ull : 0ull;
+            const unsigned kh = (unsigned)(key >> 32), kl = (unsigned)key;
+            const unsigned mh = __reduce_max_sync(0xffffffffu, kh);
+            const unsigned ml = __reduce_max_sync(0xffffffffu, kh == mh ? kl : 0u);
+            const int src = __ffs(__ballot_sync(0xffffffffu, kh == mh && kl == ml)) - 1;
+            if (lane == src) {
+                s_hi[par][warp] = kh;
+                s_lo[par][warp] = kl;
+                s_row[par][warp] = tid;
+#pragma unroll
+                for (int x = 0; x < W; ++x) s_cand[par][warp][x] = a[x];
+            }
+            if (tid == jj) {
+#pragma unroll
+                for (int x = 0; x < W; ++x) s_cur[par][x] = a[x];
+            }
+            __syncthreads();
+            const unsigned wh = lane < warps ? s_hi[par][lane] : 0u, wl = lane < warps ? s_lo[par][lane] : 0u;
+            const unsigned bh = __reduce_max_sync(0xffffffffu, wh);
+            const unsigned bl = __reduce_max_sync(0xffffffffu, wh == bh ? wl : 0u);
+            const int bw = __ffs(__ballot_sync(0xffffffffu, wh == bh && wl == bl)) - 1;
+            const bool none = (bh | bl) == 0u;  // nothing but NaN: no interchange
+            const bool zero = bh == 0u && bl == 1u;
+            const int p = none ? jj : s_row[par][bw];
+            u = none ? s_cur[par] : s_cand[par][bw];
+            if (tid == 0) {
+                ipiv[j0 + jj] = j0 + p + 1;
+                if (zero && info[b] == 0) info[b] = j0 + jj + 1;
+            }
+            if (p != jj) {
+                if (tid == jj) {
+#pragma unroll
+                    for (int x = 0; x < W; ++x) a[x] = u[x];
+                } else if (tid == p) {
+#pragma unroll
+                    for (int x = 0; x < W; ++x) a[x] = s_cur[par][x];
+                }
+            }
+            last = a[0];
+            upd = tid > jj && !zero;
+            if (!zero) {
+                l = mul_rn<true>(a[0], cdiv(cf{1.f, 0.f}, u[0]));
+                if (upd) last = l;
+            }
+        }
+#pragma unroll
+        for (int x = 1; x < W; ++x) {
+            cf t = a[x];
+            if (x + jj < jb) {  // a column of the panel still ahead
+                const cf w = submul_rn<false>(t, l, u[x]);
+                if (upd) t = w;
+            }
+            a[x - 1] = t;
+        }
+        a[W - 1] = last;
+    }
+    if (live) {
+#pragma unroll
+        for (int x = 0; x < W; ++x)
+            if (x < jb) A[x * lda] = a[x];
+    }
+}
+
+// The launch of a panel: rows in registers where a thread each is enough, the
+// slab in shared memory otherwise.
+static void panel_batched(cf* A, int64_t lda, int64_t stride, int n, int j0, int jb, int32_t* ipiv, int32_t* info,
+                          int batch, cudaStream_t st) {
+    const int m = n - j0, nt = (m + 31) / 32 * 32;
+    if (jb <= 8 && m <= 1024)
+        panel_rows_kernel<8, 1024><<<batch, nt, 0, st>>>(A, lda, stride, n, j0, jb, ipiv, info);
+    else if (jb <= 16 && m <= 512)
+        panel_rows_kernel<16, 512><<<batch, nt, 0, st>>>(A, lda, stride, n, j0, jb, ipiv, info);
+    else if (jb <= 16 && m <= 1024)
+        panel_rows_kernel<16, 1024><<<batch, nt, 0, st>>>(A, lda, stride, n, j0, jb, ipiv, info);
+    else if (jb <= 32 && m <= 512)
+        panel_rows_kernel<32, 512><<<batch, nt, 0, st>>>(A, lda, stride, n, j0, jb, ipiv, info);
+    else
+        panel1_kernel<<<batch, kBThreads, (size_t)m * jb * sizeof(cf), st>>>(A, lda, stride, n, j0, jb, ipiv, info);
+    count_launch();
+}
+
 template <class T>
 __global__ void laswp_batched_kernel(T* A, int64_t lda, int64_t stride, int col0, int ncols, const int32_t* ipiv,
                                      int n, int k1, int k2) {
@@ -125,76 +243,262 @@ __global__ void laswp_batched_kernel(T* A, int64_t lda, int64_t stride, int col0
     }
 }
 
-__device__ __forceinline__ cf shfl_cf(cf v, int src) {
-    return cf{__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
-}
-
-// X <- L^-1 X (unit lower) or U^-1 X (upper) for the jb x jb diagonal block
-// at T (jb <= 64); a warp per column at a time, batch on blockIdx.y.
-constexpr int kTrsmColsPerWarp = 8;
-template <bool UPPER>
-__global__ void __launch_bounds__(256) trsm_batched_kernel(const cf* Tm, int64_t ldt, int64_t ts, cf* X, int64_t ldx,
-                                                           int64_t xs, int jb, int ncols) {
-    __shared__ cf sT[64][65];
-    __shared__ cf sD[64];  // U: reciprocals of the diagonal
+// X <- L^-1 X for the unit lower jb x jb (jb <= NB) diagonal block at T, a
+// column of X to a thread, in registers; batch on blockIdx.y.  Four rows are
+// finished at a time, then leave the rows below up to date, the registers
+// turning by four; L is read as broadcasts from shared memory.  Bound by the
+// FP32 pipe (6 operations per entry of L and column).  A warp per column with
+// a shuffle per row took 330 us for 64 x 373, 192 matrices, on B200; 74 us so.
+// submul_rn's form is that kernel's.
+constexpr int kTrsmThreads = 64;
+template <int NB>
+__global__ void __launch_bounds__(kTrsmThreads) trsm_lower_batched_kernel(const cf* Tm, int64_t ldt, int64_t ts, cf* X,
+                                                                          int64_t ldx, int64_t xs, int jb, int ncols) {
+    constexpr int kRows = 16;
+    __shared__ __align__(16) cf sL[NB][NB];                       // sL[k][i] = L(i, k)
+    __shared__ cf sX[kTrsmThreads / 32][32][kRows + 1];           // a warp's columns, kRows rows of them
     Tm += (int64_t)blockIdx.y * ts;
     X += (int64_t)blockIdx.y * xs;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (UPPER && tid < jb) sD[tid] = cdiv(cf{1.f, 0.f}, Tm[tid + (int64_t)tid * ldt]);
-    for (int i = tid; i < jb * jb; i += blockDim.x) {
-        const int r = i % jb, c = i / jb;
-        sT[r][c] = Tm[r + (int64_t)c * ldt];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+#pragma unroll 8
+    for (int q = tid; q < NB * NB; q += kTrsmThreads) {
+        const int i = q % NB, k = q / NB;
+        sL[k][i] = (i < jb && k < i) ? Tm[i + (int64_t)k * ldt] : cf{0.f, 0.f};
+    }
+    const int col0 = blockIdx.x * kTrsmThreads + 32 * warp;
+    cf a[NB];
+    // coalesced: lanes along the rows, 32 / kRows columns at a time
+    constexpr int kPer = 32 / kRows;
+    const int lr = lane % kRows, lc = lane / kRows;
+#pragma unroll
+    for (int h = 0; h < NB; h += kRows) {
+#pragma unroll 8
+        for (int c = 0; c < 32; c += kPer) {
+            const int col = col0 + c + lc;
+            sX[warp][c + lc][lr] =
+                (h + lr < jb && col < ncols) ? X[h + lr + (int64_t)col * ldx] : cf{0.f, 0.f};
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) a[h + r] = sX[warp][lane][r];
+        __syncwarp();
     }
     __syncthreads();
-    // each warp solves kTrsmColsPerWarp columns in turn (the staged triangle
-    // serves 8 x kTrsmColsPerWarp consecutive columns)
-    for (int cc = 0; cc < kTrsmColsPerWarp; ++cc) {
-        const int col = (blockIdx.x * kTrsmColsPerWarp + cc) * 8 + warp;
-        if (col >= ncols) return;  // whole warp leaves together
-        cf* x = X + (int64_t)col * ldx;
-        cf x0 = lane < jb ? x[lane] : cf{0.f, 0.f};
-        cf x1 = lane + 32 < jb ? x[lane + 32] : cf{0.f, 0.f};
-        if (!UPPER) {
-            for (int k = 0; k < jb; ++k) {
-                const cf xk = shfl_cf(k < 32 ? x0 : x1, k & 31);
-                if (lane > k && lane < jb) x0 = x0 - sT[lane][k] * xk;
-                if (lane + 32 > k && lane + 32 < jb) x1 = x1 - sT[lane + 32][k] * xk;
-            }
-        } else {
-            for (int k = jb - 1; k >= 0; --k) {
-                if (k < 32) {
-                    if (lane == k) x0 = x0 * sD[k];
-                } else if (lane == k - 32) {
-                    x1 = x1 * sD[k];
-                }
-                const cf xk = shfl_cf(k < 32 ? x0 : x1, k & 31);
-                if (lane < k) x0 = x0 - sT[lane][k] * xk;
-                if (lane + 32 < k) x1 = x1 - sT[lane + 32][k] * xk;
+#pragma unroll 1
+    for (int b = 0; b < NB; b += 4) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int x = j + 1; x < 4; ++x) a[x] = submul_rn<true>(a[x], sL[b + j][b + x], a[j]);
+#pragma unroll
+        for (int g = 4; g < NB; g += 4) {
+            if (b + g >= NB) break;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 l01 = *reinterpret_cast<const float4*>(&sL[b + j][b + g]);
+                const float4 l23 = *reinterpret_cast<const float4*>(&sL[b + j][b + g + 2]);
+                a[g] = submul_rn<true>(a[g], cf{l01.x, l01.y}, a[j]);
+                a[g + 1] = submul_rn<true>(a[g + 1], cf{l01.z, l01.w}, a[j]);
+                a[g + 2] = submul_rn<true>(a[g + 2], cf{l23.x, l23.y}, a[j]);
+                a[g + 3] = submul_rn<true>(a[g + 3], cf{l23.z, l23.w}, a[j]);
             }
         }
-        if (lane < jb) x[lane] = x0;
-        if (lane + 32 < jb) x[lane + 32] = x1;
+        cf turn[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) turn[x] = a[x];
+#pragma unroll
+        for (int x = 0; x + 4 < NB; ++x) a[x] = a[x + 4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) a[NB - 4 + x] = turn[x];
+    }
+#pragma unroll
+    for (int h = 0; h < NB; h += kRows) {
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) sX[warp][lane][r] = a[h + r];
+        __syncwarp();
+#pragma unroll 8
+        for (int c = 0; c < 32; c += kPer) {
+            const int col = col0 + c + lc;
+            if (h + lr < jb && col < ncols) X[h + lr + (int64_t)col * ldx] = sX[warp][c + lc][lr];
+        }
     }
 }
 
-static dim3 trsm_batched_grid(int ncols, int batch) {
-    return dim3((unsigned)((ncols + 8 * kTrsmColsPerWarp - 1) / (8 * kTrsmColsPerWarp)), (unsigned)batch);
+static void trsm_lower_batched(const cf* Tm, int64_t ldt, int64_t ts, cf* X, int64_t ldx, int64_t xs, int jb, int ncols,
+                               int batch, cudaStream_t st) {
+    const dim3 grid((unsigned)((ncols + kTrsmThreads - 1) / kTrsmThreads), (unsigned)batch);
+    if (jb <= 16)
+        trsm_lower_batched_kernel<16><<<grid, kTrsmThreads, 0, st>>>(Tm, ldt, ts, X, ldx, xs, jb, ncols);
+    else if (jb <= 32)
+        trsm_lower_batched_kernel<32><<<grid, kTrsmThreads, 0, st>>>(Tm, ldt, ts, X, ldx, xs, jb, ncols);
+    else
+        trsm_lower_batched_kernel<64><<<grid, kTrsmThreads, 0, st>>>(Tm, ldt, ts, X, ldx, xs, jb, ncols);
+    count_launch();
 }
 
-// Y (m x nr) -= A (m x k) X (k x nr), complex64, batch on blockIdx.y;
-// one thread per row (k <= 64, nr small).
-__global__ void gemm_small_batched_kernel(const cf* A, int64_t lda, int64_t as, const cf* X, int64_t ldx, int64_t xs,
-                                          cf* Y, int64_t ldy, int64_t ys, int m, int k, int nr) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    A += (int64_t)blockIdx.y * as;
-    X += (int64_t)blockIdx.y * xs;
-    Y += (int64_t)blockIdx.y * ys;
-    for (int c = 0; c < nr; ++c) {
-        cf acc{0.f, 0.f};
-        for (int l = 0; l < k; ++l) acc = acc + A[i + (int64_t)l * lda] * X[l + (int64_t)c * ldx];
-        Y[i + (int64_t)c * ldy] = Y[i + (int64_t)c * ldy] - acc;
+// B <- U^-1 L^-1 P B for one matrix and up to C of its right-hand sides per
+// CTA (right-hand sides on blockIdx.x, batch on blockIdx.y), the right-hand
+// sides in shared memory.  Per 64-row block: a warp per column solves the
+// diagonal block (lane = rows r and r + 32), then every row outside it takes
+// the 64 products, summed from zero in column order, off at once.  The next
+// diagonal block is on its way (cp.async) meanwhile, and each thread's first
+// row has half its entries in registers before the block is solved: what
+// bounds it is latency, 2 n / 64 times a block's chain of 64 rows and a row's
+// loads, then the factors' one pass through HBM (8 n^2 bytes a matrix).  As a
+// block solve and a row update per launch it took 460 us for 192 matrices of
+// order 437 on B200; 100 us so.
+constexpr int kGsThreads = 256;
+constexpr int kGsAhead = 32;  // entries of a row in registers ahead of time
+constexpr size_t kGsSmemMax = 200 * 1024;
+template <int C>
+__global__ void __launch_bounds__(kGsThreads, 2) getrs_batched_kernel(const cf* LU, int64_t lda, int64_t stride, int n,
+                                                                      const int32_t* ipiv, cf* B, int nr) {
+    extern __shared__ __align__(16) unsigned char gs_smem[];
+    cf* sT = reinterpret_cast<cf*>(gs_smem);  // [2][64][64], sT[k * 64 + i] = T(i, k)
+    cf* sX = sT + 2 * kBSB * kBSB;            // [C][n]
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int c0 = blockIdx.x * C, nc = min(C, nr - c0);
+    LU += (int64_t)blockIdx.y * stride;
+    ipiv += (int64_t)blockIdx.y * n;
+    B += (int64_t)blockIdx.y * n * nr + (int64_t)c0 * n;
+    const int nblk = (n + kBSB - 1) / kBSB;
+    auto block_of = [&](int step) { return (step >= nblk ? 2 * nblk - 1 - step : step) * kBSB; };
+    auto issue = [&](int step) {
+        const int j0 = block_of(step), jb = min(kBSB, n - j0);
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(sT + (step & 1) * kBSB * kBSB);
+        const cf* src = LU + j0 + (int64_t)j0 * lda;
+        for (int q = tid; q < kBSB * kBSB; q += kGsThreads) {
+            const int i = q % kBSB, k = q / kBSB;
+            if (i < jb && k < jb)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * q),
+                             "l"(src + i + (int64_t)k * lda)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    issue(0);
+    for (int q = tid; q < C * n; q += kGsThreads) sX[q] = q < nc * n ? B[q] : cf{0.f, 0.f};
+    __syncthreads();
+    if (warp < nc) {
+        cf* x = sX + warp * n;
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            const int i = i0 + lane, p = i < n ? ipiv[i] - 1 : i;
+            unsigned todo = __ballot_sync(0xffffffffu, p != i);
+            while (todo) {
+                const int r = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const int q = __shfl_sync(0xffffffffu, p, r);
+                if (lane == 0) {
+                    const cf t = x[i0 + r];
+                    x[i0 + r] = x[q];
+                    x[q] = t;
+                }
+                __syncwarp();
+            }
+        }
     }
+#pragma unroll 1
+    for (int step = 0; step < 2 * nblk; ++step) {
+        const bool upper = step >= nblk;
+        const int j0 = block_of(step), jb = min(kBSB, n - j0);
+        // the rows still to be solved
+        const int lo = upper ? 0 : j0 + jb, hi = upper ? j0 : n;
+        const cf* panel = LU + (int64_t)j0 * lda;
+        int i = lo + tid;
+        cf t[kGsAhead];
+        auto ahead = [&]() {
+#pragma unroll
+            for (int l = 0; l < kGsAhead; ++l)
+                t[l] = (i < hi && l < jb) ? panel[i + (int64_t)l * lda] : cf{0.f, 0.f};
+        };
+        ahead();
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (step + 1 < 2 * nblk) issue(step + 1);
+        if (warp < nc) {
+            const cf* T = sT + (step & 1) * kBSB * kBSB;
+            cf* x = sX + warp * n + j0;
+            cf x0 = lane < jb ? x[lane] : cf{0.f, 0.f};
+            cf x1 = lane + 32 < jb ? x[lane + 32] : cf{0.f, 0.f};
+            auto pass = [&](cf v, int src) {
+                return cf{__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
+            };
+            if (!upper) {
+                const int ka = min(jb, 32);
+#pragma unroll 4
+                for (int k = 0; k < ka; ++k) {
+                    const cf xk = pass(x0, k);
+                    const cf w0 = submul_rn<true>(x0, T[k * kBSB + lane], xk);
+                    const cf w1 = submul_rn<true>(x1, T[k * kBSB + lane + 32], xk);
+                    if (lane > k && lane < jb) x0 = w0;
+                    if (lane + 32 < jb) x1 = w1;
+                }
+#pragma unroll 4
+                for (int k = 32; k < jb; ++k) {
+                    const cf xk = pass(x1, k - 32);
+                    const cf w1 = submul_rn<true>(x1, T[k * kBSB + lane + 32], xk);
+                    if (lane + 32 > k && lane + 32 < jb) x1 = w1;
+                }
+            } else {
+                // reciprocals of the diagonal
+                const cf one = cone<cf>();
+                const cf d0 = lane < jb ? cdiv(one, T[lane * (kBSB + 1)]) : one;
+                const cf d1 = lane + 32 < jb ? cdiv(one, T[(lane + 32) * (kBSB + 1)]) : one;
+#pragma unroll 4
+                for (int k = jb - 1; k >= 32; --k) {
+                    if (lane == k - 32) x1 = mul_rn<false>(x1, d1);
+                    const cf xk = pass(x1, k - 32);
+                    const cf w1 = submul_rn<true>(x1, T[k * kBSB + lane + 32], xk);
+                    x0 = submul_rn<true>(x0, T[k * kBSB + lane], xk);
+                    if (lane + 32 < k) x1 = w1;
+                }
+#pragma unroll 4
+                for (int k = min(jb, 32) - 1; k >= 0; --k) {
+                    if (lane == k) x0 = mul_rn<false>(x0, d0);
+                    const cf xk = pass(x0, k);
+                    const cf w0 = submul_rn<true>(x0, T[k * kBSB + lane], xk);
+                    if (lane < k) x0 = w0;
+                }
+            }
+            if (lane < jb) x[lane] = x0;
+            if (lane + 32 < jb) x[lane + 32] = x1;
+        }
+        __syncthreads();
+        while (i < hi) {
+            cf acc[C];
+#pragma unroll
+            for (int c = 0; c < C; ++c) acc[c] = cf{0.f, 0.f};
+            auto take = [&](cf v, int l) {
+#pragma unroll
+                for (int c = 0; c < C; ++c) {
+                    const cf p = mul_rn<false>(v, sX[c * n + j0 + l]);
+                    acc[c] = cf{__fadd_rn(acc[c].re, p.re), __fadd_rn(acc[c].im, p.im)};
+                }
+            };
+#pragma unroll 1
+            for (int h = 0; h < kBSB; h += kGsAhead / 2) {
+                // t: entries h .. h + 31; the first half is used up and refilled
+#pragma unroll
+                for (int l = 0; l < kGsAhead / 2; ++l)
+                    if (h + l < jb) take(t[l], h + l);
+#pragma unroll
+                for (int l = 0; l < kGsAhead / 2; ++l) {
+                    t[l] = t[l + kGsAhead / 2];
+                    const int q = h + kGsAhead + l;
+                    t[l + kGsAhead / 2] = q < jb ? panel[i + (int64_t)q * lda] : cf{0.f, 0.f};
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < C; ++c) sX[c * n + i] = sX[c * n + i] - acc[c];
+            i += kGsThreads;
+            if (i < hi) ahead();
+        }
+    }
+    __syncthreads();
+    for (int q = tid; q < nc * n; q += kGsThreads) B[q] = sX[q];
 }
 
 // R = B - Z X  (complex128; B shared across the batch when bs == 0)
@@ -220,6 +524,17 @@ __global__ void resid_batched_kernel(const cd* Z, int64_t ldz, int64_t zs, const
         }
         const cd bb = B[i + (int64_t)c * ldb];
         R[i + (int64_t)c * ldr] = cd{bb.re - ar, bb.im - ai};
+    }
+}
+
+// The first residual, R32 = B rounded (X = 0; B with its own leading dimension
+// and stride), one launch for the batch.
+__global__ void narrow_rhs_batched_kernel(const cd* B, int64_t ldb, int64_t bs, cf* R32, int n, int nr,
+                                          int64_t total) {
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t col = q / n;
+        const cd v = B[(col / nr) * bs + (col % nr) * ldb + (q - col * n)];
+        R32[q] = cf{(float)v.re, (float)v.im};
     }
 }
 
@@ -303,9 +618,7 @@ static mw_status cgetrf_batched(int n, int batch, cf* A, int64_t lda, int64_t st
             const int jb = (J0 + bw - j0) < pw ? (J0 + bw - j0) : pw;
             {
                 ProfileScope ps(PC_PANEL, st, 4.0 * (double)(n - j0) * jb * jb * batch);
-                panel1_kernel<<<batch, kBThreads, (size_t)(n - j0) * jb * sizeof(cf), st>>>(A, lda, stride, n, j0, jb,
-                                                                                            ipiv, info);
-                count_launch();
+                panel_batched(A, lda, stride, n, j0, jb, ipiv, info, batch, st);
             }
             if (j0 > 0) {
                 ProfileScope ps(PC_LASWP, st);
@@ -324,10 +637,9 @@ static mw_status cgetrf_batched(int n, int batch, cf* A, int64_t lda, int64_t st
                 cf* A12 = A + j0 + (int64_t)(j0 + jb) * lda;
                 {
                     ProfileScope ps(PC_TRSM, st, 4.0 * (double)jb * jb * inner * batch);
-                    trsm_batched_kernel<false><<<trsm_batched_grid(inner, batch), 256, 0, st>>>(A11, lda, stride, A12,
-                                                                                             lda, stride, jb, inner);
+                    trsm_lower_batched(A11, lda, stride, A12, lda, stride, jb, inner, batch, st);
                 }
-                count_launch(2);
+                count_launch();
                 mw_status s = cgemm_tc_update_batched(n - j0 - jb, inner, jb, batch, A + (j0 + jb) + (int64_t)j0 * lda,
                                                       lda, stride, A12, lda, stride,
                                                       A + (j0 + jb) + (int64_t)(j0 + jb) * lda, lda, stride, w.tc,
@@ -346,10 +658,9 @@ static mw_status cgetrf_batched(int n, int batch, cf* A, int64_t lda, int64_t st
             cf* A12 = A + J0 + (int64_t)(J0 + bw) * lda;
             {
                 ProfileScope ps(PC_TRSM, st, 4.0 * (double)bw * bw * right * batch);
-                trsm_batched_kernel<false><<<trsm_batched_grid(right, batch), 256, 0, st>>>(A11, lda, stride, A12, lda,
-                                                                                         stride, bw, right);
+                trsm_lower_batched(A11, lda, stride, A12, lda, stride, bw, right, batch, st);
             }
-            count_launch(2);
+            count_launch();
             mw_status s = cgemm_tc_update_batched(right, right, bw, batch, A + (J0 + bw) + (int64_t)J0 * lda, lda,
                                                   stride, A12, lda, stride, A + (J0 + bw) + (int64_t)(J0 + bw) * lda,
                                                   lda, stride, w.tc, w.tc_bytes, w.tc_err, st, 0);
@@ -361,37 +672,33 @@ static mw_status cgetrf_batched(int n, int batch, cf* A, int64_t lda, int64_t st
 }
 
 // In-place solve of the batch's B (n x nr each, column-major, ld n).
-static mw_status cgetrs_batched(int n, int nr, int batch, const cf* LU, int64_t lda, int64_t stride,
-                                const int32_t* ipiv, cf* B, cudaStream_t st) {
-    const int64_t bs = (int64_t)n * nr;
-    ProfileScope ps(PC_ZGEMM, st, 8.0 * (double)n * n * nr * batch);  // the whole batched getrs
-    laswp_batched_kernel<cf><<<dim3((nr + 127) / 128, batch), 128, 0, st>>>(B, n, bs, 0, nr, ipiv, n, 0, n);
+template <int C>
+static mw_status getrs_launch(int n, int nr, int batch, const cf* LU, int64_t lda, int64_t stride, const int32_t* ipiv,
+                              cf* B, cudaStream_t st) {
+    static bool attr = false;
+    if (!attr) {
+        MW_CHECK_CUDA(cudaFuncSetAttribute(getrs_batched_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)kGsSmemMax));
+        attr = true;
+    }
+    const size_t smem = sizeof(cf) * ((size_t)2 * kBSB * kBSB + (size_t)C * n);
+    getrs_batched_kernel<C><<<dim3((unsigned)((nr + C - 1) / C), (unsigned)batch), kGsThreads, smem, st>>>(
+        LU, lda, stride, n, ipiv, B, nr);
     count_launch();
-    for (int j0 = 0; j0 < n; j0 += kBSB) {
-        const int jb = (n - j0) < kBSB ? (n - j0) : kBSB;
-        trsm_batched_kernel<false><<<trsm_batched_grid(nr, batch), 256, 0, st>>>(LU + j0 + (int64_t)j0 * lda, lda, stride,
-                                                                             B + j0, n, bs, jb, nr);
-        count_launch();
-        const int rest = n - j0 - jb;
-        if (rest > 0) {
-            gemm_small_batched_kernel<<<dim3((rest + 127) / 128, batch), 128, 0, st>>>(
-                LU + (j0 + jb) + (int64_t)j0 * lda, lda, stride, B + j0, n, bs, B + j0 + jb, n, bs, rest, jb, nr);
-            count_launch();
-        }
-    }
-    for (int j0 = ((n - 1) / kBSB) * kBSB; j0 >= 0; j0 -= kBSB) {
-        const int jb = (n - j0) < kBSB ? (n - j0) : kBSB;
-        trsm_batched_kernel<true><<<trsm_batched_grid(nr, batch), 256, 0, st>>>(LU + j0 + (int64_t)j0 * lda, lda, stride,
-                                                                            B + j0, n, bs, jb, nr);
-        count_launch();
-        if (j0 > 0) {
-            gemm_small_batched_kernel<<<dim3((j0 + 127) / 128, batch), 128, 0, st>>>(
-                LU + (int64_t)j0 * lda, lda, stride, B + j0, n, bs, B, n, bs, j0, jb, nr);
-            count_launch();
-        }
-    }
     MW_CHECK_CUDA(cudaGetLastError());
     return MW_OK;
+}
+
+static mw_status cgetrs_batched(int n, int nr, int batch, const cf* LU, int64_t lda, int64_t stride,
+                                const int32_t* ipiv, cf* B, cudaStream_t st) {
+    ProfileScope ps(PC_ZGEMM, st, 8.0 * (double)n * n * nr * batch);  // the whole batched getrs
+    // as many right-hand sides a CTA as there are (to 8), where they fit
+    // beside the block; n <= 3200 (panels of 8 columns) leaves room for four
+    auto fits = [&](int c) { return sizeof(cf) * ((size_t)2 * kBSB * kBSB + (size_t)c * n) <= kGsSmemMax; };
+    if (nr > 4 && fits(8)) return getrs_launch<8>(n, nr, batch, LU, lda, stride, ipiv, B, st);
+    if (nr > 2 && fits(4)) return getrs_launch<4>(n, nr, batch, LU, lda, stride, ipiv, B, st);
+    if (nr > 1 && fits(2)) return getrs_launch<2>(n, nr, batch, LU, lda, stride, ipiv, B, st);
+    return getrs_launch<1>(n, nr, batch, LU, lda, stride, ipiv, B, st);
 }
 
 }  // namespace mw
@@ -427,18 +734,18 @@ extern "C" mw_status mw_zgesv_mixed_batched(int32_t n, int32_t nrhs, int32_t bat
     cd* Xc = reinterpret_cast<cd*>(X);
     const cd* Zc = reinterpret_cast<const cd*>(Z);
     const cd* Bc = reinterpret_cast<const cd*>(B);
-    // R = B (X = 0): the residual kernel with X = 0 would read Z; copy B instead
+    // X = 0: the first residual is B itself
     MW_CHECK_CUDA(cudaMemsetAsync(Xc, 0, sizeof(cd) * tot, st));
-    for (int b = 0; b < batch; ++b)
-        MW_CHECK_CUDA(cudaMemcpy2DAsync(w.R + (int64_t)b * per, sizeof(cd) * n, Bc + (int64_t)b * b_stride,
-                                        sizeof(cd) * ldb, sizeof(cd) * n, nrhs, cudaMemcpyDeviceToDevice, st));
     std::vector<double> hn(2 * (size_t)batch), prev((size_t)batch, 0.0);
     std::vector<int32_t> hinfo(batch);
     double corr = INFINITY;
     int it = 0;
     const unsigned g1 = (unsigned)((tot + 255) / 256 < 8192 ? (tot + 255) / 256 : 8192);
     for (;; ++it) {
-        narrow_batched_kernel<<<g1, 256, 0, st>>>(w.R, w.R32, tot);
+        if (it == 0)
+            narrow_rhs_batched_kernel<<<g1, 256, 0, st>>>(Bc, ldb, b_stride, w.R32, n, nrhs, tot);
+        else
+            narrow_batched_kernel<<<g1, 256, 0, st>>>(w.R, w.R32, tot);
         count_launch();
         s = cgetrs_batched(n, nrhs, batch, Z32c, ldz32, z32_stride, ipiv, w.R32, st);
         if (s != MW_OK) return s;

@@ -32,6 +32,10 @@ constexpr int kSpUStride = kSpB + 2;  // complex elements per shared-memory row 
 
 namespace {
 
+// (mul_rn, submul_rn: the forms are chosen per position so that the factors
+// are, bit for bit, those of 32-column panels and chunks, whatever the width
+// used here)
+
 __device__ __forceinline__ cf crcp_sp(cf z) {
     // 1 / z with z scaled by its larger component (|z|^2 neither overflows
     // nor underflows); two reciprocals instead of Smith's three divisions
@@ -41,25 +45,6 @@ __device__ __forceinline__ cf crcp_sp(cf z) {
     const float a = z.re * rs, b = z.im * rs;
     const float t = rs * __frcp_rn(a * a + b * b);
     return cf{a * t, -b * t};
-}
-
-// a - b and the two products with their roundings spelled out: a complex
-// product has two contracted forms of its imaginary part, and which one the
-// compiler takes depends on the code around it.  FIRST rounds the product
-// a.im b.re before the fused a.re b.im; otherwise the other way round.  The
-// forms below are chosen per position so that the factors are, bit for bit,
-// those of 32-column panels and chunks, whatever the width used here.
-template <bool FIRST>
-__device__ __forceinline__ cf mul_rn(cf a, cf b) {
-    const float re = __fmaf_rn(a.re, b.re, -__fmul_rn(a.im, b.im));
-    const float im = FIRST ? __fmaf_rn(a.re, b.im, __fmul_rn(a.im, b.re))
-                           : __fmaf_rn(a.im, b.re, __fmul_rn(a.re, b.im));
-    return cf{re, im};
-}
-template <bool FIRST>
-__device__ __forceinline__ cf submul_rn(cf v, cf a, cf b) {
-    const cf p = mul_rn<FIRST>(a, b);
-    return cf{__fsub_rn(v.re, p.re), __fsub_rn(v.im, p.im)};
 }
 
 __device__ __forceinline__ float cabs1f(cf z) { return fabsf(z.re) + fabsf(z.im); }
