@@ -5,9 +5,9 @@
 // numpy.linalg.solve over the k axis) factorises one small complex matrix per
 // frequency.  Here a whole batch of same-order matrices (one structure at
 // many frequencies) is factorised together in complex64:
-//   panel   one CTA per matrix, the panel (rows j0..n, 8-32 columns) resident
-//           in shared memory; pivot search, swap, scale and rank-1 update
-//           synchronise with __syncthreads only;
+//   panel   one CTA per matrix, the panel (rows j0..n, 8-32 columns) in
+//           registers, a row to a thread, or in shared memory where the
+//           threads run out;
 //   update  the batched tcgen05 3xTF32 update of cgemm_tc.cu over all
 //           matrices' tiles in one persistent launch;
 // then every matrix is solved and refined in FP64 against its own Z
@@ -115,8 +115,7 @@ __global__ void __launch_bounds__(kBThreads) panel1_kernel(cf* A, int64_t lda, i
 // search over m <= NT rows, a complex reciprocal) and, with one or two CTAs an
 // SM, by the slots' updates.  From the slab in shared memory with four
 // barriers a column this took 75 us at m = 437, jb = 16, 192 matrices, on
-// B200; 30 us so
-// (@PANELX@)  Entry for entry the slab's operations (mul_rn and
+// B200; 30 us so.  Entry for entry the slab's operations (mul_rn and
 // submul_rn spell its roundings out).
 template <int W, int NT>
 __global__ void __launch_bounds__(NT) panel_rows_kernel(cf* A, int64_t lda, int64_t stride, int n, int j0, int jb,
@@ -248,7 +247,8 @@ __global__ void laswp_batched_kernel(T* A, int64_t lda, int64_t stride, int col0
 // finished at a time, then leave the rows below up to date, the registers
 // turning by four; L is read as broadcasts from shared memory.  Bound by the
 // FP32 pipe (6 operations per entry of L and column).  A warp per column with
-// a shuffle per row took 330 us for 64 x 373, 192 matrices, on B200; 74 us so.
+// a shuffle per row took 330 us for 64 x 373, 192 matrices, on B200; 74 us so (mean of the
+// Yagi sweep's launches).
 // submul_rn's form is that kernel's.
 constexpr int kTrsmThreads = 64;
 template <int NB>
@@ -347,8 +347,8 @@ static void trsm_lower_batched(const cf* Tm, int64_t ldt, int64_t ts, cf* X, int
 // row has half its entries in registers before the block is solved: what
 // bounds it is latency, 2 n / 64 times a block's chain of 64 rows and a row's
 // loads, then the factors' one pass through HBM (8 n^2 bytes a matrix).  As a
-// block solve and a row update per launch it took 460 us for 192 matrices of
-// order 437 on B200; 100 us so.
+// block solve and a row update per launch it took 460 us (mean of the solves of
+// a sweep over 24 Yagis x 64 frequencies) on B200; 225 us so.
 constexpr int kGsThreads = 256;
 constexpr int kGsAhead = 32;  // entries of a row in registers ahead of time
 constexpr size_t kGsSmemMax = 200 * 1024;
