@@ -165,6 +165,10 @@ __device__ __forceinline__ cd crecip(cd z) { return recip_special(z) ? cdiv(cd{1
 // lane without a candidate if all do).  Values are non-negative doubles,
 // whose bits order like the values.  One reduction settles it unless two
 // lanes share the high word.
+// (The warp index of the kernels comes from a shuffle: that makes it the same
+// in every lane as far as the compiler can see, and the votes and shuffles
+// behind branches on it need no code that gathers the warp first.  47.7 -> 42.2
+// us at order 21 on B200, 326 -> 306 at 200, 521 -> 495 at 300.)
 __device__ __forceinline__ int warp_pick(unsigned mh, unsigned hi, unsigned lo, unsigned pos) {
     const bool h = pos != kNone && hi == mh;
     unsigned eq = __ballot_sync(0xffffffffu, h);
@@ -204,7 +208,7 @@ struct Shared {
 // register slots rotate.
 __device__ __forceinline__ void panel_solo(Shared& S, cd* A, int64_t lda, int32_t* ipiv, int32_t* info, int n, int c0,
                                            int w) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int cnt = n - c0, nw = min(kCWarps, (cnt + 31) / 32);  // warps that hold rows
     if (warp >= nw) return;
     cd a[kW];
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
     Shared& S = *reinterpret_cast<Shared*>(zlu_smem);
     cg::cluster_group cl = cg::this_cluster();
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int64_t mat = blockIdx.x / C;
     cd* const A = P.A + mat * P.a_stride;
     cd* const B = P.B + mat * P.b_stride;
@@ -760,7 +764,7 @@ __global__ void __launch_bounds__(kCT) zblock_solve_kernel(SolveArgs P) {
     cd* dinv = Ls + kW * kSMax;
     int* src = reinterpret_cast<int*>(dinv + kW);
     int* disp = src + kSMax;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nleft = (P.left + kSN - 1) / kSN;
     const bool isleft = (int)blockIdx.x < nleft;
     const int q0 = ((int)blockIdx.x - (isleft ? 0 : nleft)) * kSN;
