@@ -48,6 +48,8 @@ mw_status cgemm_tc_prepacked2(int64_t m, int64_t n, int64_t k1, const TcPlanes& 
                               cf* C, int64_t ldc, int* err, cudaStream_t st, int max_ctas);
 
 // static-pivot panel of the complex64 path (lu_static.cu)
+mw_status static_u12_c64(const cf* L, int64_t ldl, int jb, cf* X, int64_t ldx, int64_t ncols, const int32_t* perm,
+                         const TcPlanes* pack_b, cudaStream_t st);
 mw_status static_panel_c64(cf* A, int64_t lda, int64_t n, int64_t j0, int jb, int32_t* ipiv, int32_t* info,
                            PanelWs* ws, cf* inv_diag, int32_t* perm, const TcPlanes* pack_a, cudaStream_t st);
 void static_permute_c64(cf* A, int64_t lda, int64_t row0, int jb, int64_t col0, int64_t ncols, const int32_t* perm,
@@ -1680,6 +1682,13 @@ static mw_status critical_end(AuxStreams* ax, cudaStream_t caller) {
     return MW_OK;
 }
 
+// Columns from which the static path's block rows are permuted, solved and
+// packed by one kernel (static_u12_c64) instead of a permutation and two
+// leaves: the leaves' chain is shorter while their CTAs find SMs (20 us against
+// 22 at 1,000 columns on B200), the one pass wins from about 2,000 (24 against
+// 27) and by far at 10,240 (33 against 100).
+constexpr int64_t kU12Wide = 1536;
+
 template <class T>
 static mw_status getrf_lookahead(int64_t n, T* A, int64_t lda, int32_t* ipiv, int32_t* info, char* ws,
                                  const volatile int32_t* cancel, const Updater& up_main, const Updater& up_trail,
@@ -1793,10 +1802,21 @@ static mw_status getrf_lookahead(int64_t n, T* A, int64_t lda, int32_t* ipiv, in
         // trail: everything right of the next block, after panel j
         MW_CHECK_CUDA(cudaStreamWaitEvent(tr, ax->ev_main, 0));
         if (n - c2 > 0) {
-            swap_rows(A, lda, c2, n - c2, tr);
-            s = trsm_lower_blocked<T>(A + j0 + j0 * lda, lda, A + j0 + c2 * lda, lda, jb, n - c2, up_trail, tr,
-                                      prepacked ? &pl_trail : nullptr);
-            if (s != MW_OK) return s;
+            bool solved = false;
+            if constexpr (std::is_same<T, cf>::value) {
+                if (perm != nullptr && n - c2 >= kU12Wide) {
+                    s = static_u12_c64(A + j0 + j0 * lda, lda, jb, A + j0 + c2 * lda, lda, n - c2, perm,
+                                       prepacked ? &pl_trail : nullptr, tr);
+                    if (s != MW_OK) return s;
+                    solved = true;
+                }
+            }
+            if (!solved) {
+                swap_rows(A, lda, c2, n - c2, tr);
+                s = trsm_lower_blocked<T>(A + j0 + j0 * lda, lda, A + j0 + c2 * lda, lda, jb, n - c2, up_trail, tr,
+                                          prepacked ? &pl_trail : nullptr);
+                if (s != MW_OK) return s;
+            }
             s = prepacked ? update_prepacked(n - c1, n - c2, jb, pl_trail, A + c1 + c2 * lda, lda, up_trail, tr)
                           : block_update(A + c1 + j0 * lda, lda, A + j0 + c2 * lda, lda, A + c1 + c2 * lda, lda,
                                          n - c1, n - c2, jb, up_trail, tr);

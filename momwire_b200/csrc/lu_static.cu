@@ -702,7 +702,140 @@ __global__ void __launch_bounds__(kSpL21Threads, 1)
     if (lane == 0) atomicMax(&ws->lmax_bits, (lmax == lmax) ? __float_as_uint(lmax) : 0x7f800000u);
 }
 
+// U12 = L11^-1 P A12 for many columns right of the diagonal block: the rows in
+// the block's order (perm), the unit lower solve and the packed B operand of
+// the update that follows, in one pass.  The mirror image of sp_l21_kernel: a
+// warp solves eight columns by itself, 16 rows at a time, eight lanes to a
+// column pair; the columns stay in the warp's strip of shared memory from the
+// gather to the end.  Every entry takes its products in row order, in the
+// form of the leaves it replaces.  Bound by the FP32 pipe, as L21.  Beside the
+// row permutation, two leaves of 64 rows with a warp to four columns took
+// 100 us for 10,240 columns on B200 (5 + 36 + 59, one after the other before
+// each trailing update); 33 us so, 24 for 2,500 columns.
+__global__ void __launch_bounds__(kSpL21Threads, 1)
+    sp_u12_kernel(const cf* __restrict__ L, int64_t ldl, int jb, cf* __restrict__ X, int64_t ldx, int64_t ncols,
+                  int cols_cta, const int32_t* __restrict__ perm, float* __restrict__ b_hi,
+                  float* __restrict__ b_lo) {
+    extern __shared__ __align__(16) unsigned char sp_smem[];
+    cf* sL = reinterpret_cast<cf*>(sp_smem);  // sL[j * kSpUStride + i] = L(i, j)
+    cf* sX = sL + (size_t)kSpB * kSpUStride;  // [columns of the CTA][kSpUStride]
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int p = lane >> 3, f = lane & 7;
+    const int64_t base_col = (int64_t)blockIdx.x * cols_cta + warp * kSpWarpRows;
+    const bool work = warp * kSpWarpRows < cols_cta && base_col < ncols;
+    cf* strip = sX + (size_t)warp * kSpWarpRows * kSpUStride;
+    if (work) {
+#pragma unroll
+        for (int h = 0; h < kSpB; h += 32) {
+            const int i = h + lane;
+            const int src = i < jb ? perm[i] : 0;
+            cf t[kSpWarpRows];
+#pragma unroll
+            for (int c = 0; c < kSpWarpRows; ++c)
+                t[c] = (i < jb && base_col + c < ncols) ? X[src + (base_col + c) * ldx] : cf{0.0f, 0.0f};
+#pragma unroll
+            for (int c = 0; c < kSpWarpRows; ++c) strip[c * kSpUStride + i] = t[c];
+        }
+    }
+    constexpr int kU = 8;
+    for (int base = 0; base < kSpB * kSpB; base += kU * kSpL21Threads) {
+        cf t[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int idx = base + u * kSpL21Threads + tid;
+            const int i = idx % kSpB, j = idx / kSpB;
+            t[u] = (idx < kSpB * kSpB && i > j && i < jb) ? L[i + (int64_t)j * ldl] : cf{0.0f, 0.0f};
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int idx = base + u * kSpL21Threads + tid;
+            if (idx < kSpB * kSpB) sL[(idx / kSpB) * kSpUStride + idx % kSpB] = t[u];
+        }
+    }
+    __syncthreads();
+    if (!work) return;
+    cf* x0 = strip + (size_t)(2 * p) * kSpUStride;
+    cf* x1 = x0 + kSpUStride;
+    const int64_t col = base_col + 2 * p;
+    const int n_ks = tc_n_ks(jb);
+    const int nchunks = (jb + kSpChunk - 1) / kSpChunk;
+    for (int k = 0; k < nchunks; ++k) {
+        const int r0 = kSpChunk * k + 2 * f;  // this lane's rows r0, r0 + 1 of columns col, col + 1
+        cf a[2][2];
+        load2(x0 + r0, a[0]);
+        load2(x1 + r0, a[1]);
+#pragma unroll 2
+        for (int j = 0; j < kSpChunk * k; j += 2) {
+            cf x[2][2], la[2], lb[2];
+            load2(x0 + j, x[0]);
+            load2(x1 + j, x[1]);
+            load2(sL + (size_t)j * kSpUStride + r0, la);
+            load2(sL + (size_t)(j + 1) * kSpUStride + r0, lb);
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    a[c][r] = submul_rn<false>(a[c][r], la[r], x[c][0]);
+                    a[c][r] = submul_rn<false>(a[c][r], lb[r], x[c][1]);
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < kSpChunk; ++j) {
+            cf lj[2];
+            load2(sL + (size_t)(kSpChunk * k + j) * kSpUStride + r0, lj);
+            const int src = (lane & ~7) | (j / 2);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const cf v = a[c][j & 1];
+                const cf x{__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+                    if (2 * f + r > j) a[c][r] = submul_rn<false>(a[c][r], lj[r], x);
+            }
+        }
+        *reinterpret_cast<float4*>(x0 + r0) = make_float4(a[0][0].re, a[0][0].im, a[0][1].re, a[0][1].im);
+        *reinterpret_cast<float4*>(x1 + r0) = make_float4(a[1][0].re, a[1][0].im, a[1][1].re, a[1][1].im);
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            if (col + c >= ncols) continue;
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+                if (r0 + r < jb) X[r0 + r + (col + c) * ldx] = a[c][r];
+            if (b_hi != nullptr && 2 * r0 < n_ks * TC_KS)
+                tc_store_b4(b_hi, b_lo, n_ks, col + c, 2 * r0,
+                            make_float4(a[c][0].re, a[c][0].im, a[c][1].re, a[c][1].im));
+        }
+    }
+}
+
 }  // namespace
+
+// U12 of a static-pivot panel: L11^-1 P X for the jb <= 128 rows at X, ncols
+// columns, L11 at L (unit lower), the block's row order in `perm`; with
+// `pack_b` set also as the packed B operand of the update with inner dimension
+// jb.
+mw_status static_u12_c64(const cf* L, int64_t ldl, int jb, cf* X, int64_t ldx, int64_t ncols, const int32_t* perm,
+                         const TcPlanes* pack_b, cudaStream_t st) {
+    MW_REQUIRE(jb >= 1 && jb <= kSpB, "static panel width %d outside 1..%d", jb, kSpB);
+    if (ncols <= 0) return MW_OK;
+    static bool configured = false;
+    if (!configured) {
+        MW_CHECK_CUDA(cudaFuncSetAttribute(sp_u12_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)kSpL21Smem));
+        configured = true;
+    }
+    const int64_t full = (int64_t)kSpL21Warps * kSpWarpRows * kSpSMs;
+    const int64_t ctas = (ncols + full - 1) / full * kSpSMs;
+    const int64_t per_cta = (ncols + ctas * kSpWarpRows - 1) / (ctas * kSpWarpRows) * kSpWarpRows;
+    ProfileScope ps(PC_TRSM, st, 4.0 * (double)jb * jb * ncols, 16.0 * (double)jb * ncols);
+    sp_u12_kernel<<<(unsigned)((ncols + per_cta - 1) / per_cta), kSpL21Threads, kSpL21Smem, st>>>(
+        L, ldl, jb, X, ldx, ncols, (int)per_cta, perm, pack_b ? pack_b->b_hi : nullptr,
+        pack_b ? pack_b->b_lo : nullptr);
+    MW_CHECK_CUDA(cudaGetLastError());
+    count_launch();
+    return MW_OK;
+}
 
 // The panel of columns [j0, j0+jb) (jb <= 128) over rows [j0, n): the
 // diagonal block factored with pivots among its own rows, then L21.

@@ -112,3 +112,21 @@ def test_rows_beyond_one_wave(cuda_device):
     assert np.array_equal(piv, np.arange(n))
     res = torch.linalg.norm(A @ X - B) / torch.linalg.norm(B)
     assert float(res) <= 1e-9
+
+
+@pytest.mark.parametrize("n", [1795, 1800])
+def test_wide_block_rows(n, cuda_device):
+    """Block rows of 1,536 columns and more, with interchanges inside the
+    blocks (each block's rows reversed): permuted, solved and packed in one
+    pass."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    order = np.concatenate([np.arange(min(b + 128, n) - 1, b - 1, -1) for b in range(0, n, 128)])
+    A = _matrix(n, rng)[order]
+    B = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
+    F, piv, X, used = _solve(torch.from_numpy(A).to(cuda_device), torch.from_numpy(B).to(cuda_device))
+    assert used == 0
+    _check_factors(A, F.cpu().numpy().T.astype(np.complex128), piv)
+    want = np.linalg.solve(A, B)
+    assert np.linalg.norm(X.cpu().numpy() - want) <= 1e-9 * np.linalg.norm(want)
