@@ -17,17 +17,10 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "fill_args.cuh"
 #include "pair_moments.cuh"
 
 namespace mw {
-
-struct GLParams {
-    int nq;
-    double t[8];    // nodes on [0,1]
-    double w[8];    // weights on [0,1]
-    double x20[20]; // 20-point nodes on [-1,1] (static panels)
-    double w20[20];
-};
 
 static GLParams make_gl(int nq) {
     GLParams g{};
@@ -269,26 +262,6 @@ __global__ void __launch_bounds__(kTableThreads) same_edge_table_kernel(
 // --------------------------------------------------------------------------
 // Fused fill kernel
 // --------------------------------------------------------------------------
-
-struct FillArgs {
-    mw_segments seg;
-    mw_basis basis;
-    const double* table;
-    const int32_t* e_n;        // edges: segments per edge
-    const int64_t* e_off;      // edges: table offsets
-    mw_ground ground;
-    double k, omega, eps0, mu0;
-    double* Z;
-    int64_t ldz;
-    float* Z32;
-    int64_t ldz32;
-    // frequency batch (blockIdx.z): per-entry k / omega (NULL = the scalars
-    // above) and the strides between consecutive tables and matrices
-    const double* kb;
-    const double* omegab;
-    int64_t table_stride, z_stride, z32_stride;
-    int nbatch;
-};
 
 // Column bases per contraction round: half a tile, so that three blocks'
 // shared memory fits an SM.
@@ -582,6 +555,13 @@ constexpr size_t kFillSmemSM = 227 * 1024;
 
 template <int D, bool IMAGE, bool EK>
 static mw_status launch_fill(const FillArgs& A, const GLParams& gl, cudaStream_t st) {
+    // A single system with a complex64 copy is about to be solved through
+    // complex64 factors.  Single coefficients of a large one follow the
+    // copy's roundings to 6e-8 (16 x 16 array, 10,496 unknowns), and this
+    // kernel's sums differ from fill_rows.cu's by 1e-13 of an entry, enough to
+    // turn a thousand of them: there Z keeps fill_rows.cu's order of sums,
+    // 11.9 ms against 6.7 here.  Sweeps' small systems move by 1e-11.
+    if (A.Z32 && A.nbatch == 0) return fill_rows(A, gl, IMAGE, EK, fill_flops(D, gl.nq, A.seg.n_seg, A.basis.n_basis), st);
     const size_t smem = FillSmem<D, IMAGE>(gl.nq, A.basis.max_tile_seg, A.basis.max_tile_basis).bytes;
     const size_t fit = kFillSmemSM / (smem + 1024);
     auto kern = fit >= 3 ? fill_kernel<D, IMAGE, EK, 128>
