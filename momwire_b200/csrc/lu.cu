@@ -1552,51 +1552,6 @@ static mw_status panel_factor(T* A, int64_t lda, int64_t n, int64_t j0, int jb, 
     return MW_OK;
 }
 
-// Right-looking blocked LU of an n x n column-major matrix.
-template <class T>
-static mw_status getrf(int64_t n, T* A, int64_t lda, int32_t* ipiv, int32_t* info, char* ws,
-                       const volatile int32_t* cancel, const Updater& up, cudaStream_t st) {
-    MW_CHECK_CUDA(cudaMemsetAsync(info, 0, 2 * sizeof(int32_t), st));
-    MW_CHECK_CUDA(cudaMemsetAsync(ws, 0, sizeof(PanelWs), st));
-    {
-        size_t ov, oi, orow, ocur;
-        ws_layout(kMaxPanelGrid, &ov, &oi, &orow, &ocur);
-        MW_CHECK_CUDA(cudaMemsetAsync(ws + oi, 0, sizeof(int64_t) * 2 * kMaxPanelGrid, st));
-        // and the complex64 panel's tagged records (no tag from an earlier
-        // factorisation may match)
-        MW_CHECK_CUDA(cudaMemsetAsync(ws + orow, 0, sizeof(unsigned long long) * 2 * 2 * kC64RecStride, st));
-    }
-    {
-        mw_status s0 = trsm_setup<T>();
-        if (s0 != MW_OK) return s0;
-    }
-    PanelWs* pws = reinterpret_cast<PanelWs*>(ws);
-    for (int64_t j0 = 0; j0 < n; j0 += kOuterNB) {
-        if (cancel && *cancel) {
-            set_error("factorisation cancelled");
-            return MW_ERR_CANCELLED;
-        }
-        const int jb = (int)((n - j0) < kOuterNB ? (n - j0) : kOuterNB);
-        mw_status s = panel_factor<T>(A, lda, n, j0, jb, ipiv, info, ws, up, st);
-        if (s != MW_OK) return s;
-        const int64_t left = j0, right = n - j0 - jb;
-        laswp_launch<T>(A, lda, 0, left, ipiv, j0, j0 + jb, st);
-        if (right > 0) {
-            laswp_launch<T>(A, lda, j0 + jb, right, ipiv, j0, j0 + jb, st);
-            T* A11 = A + j0 + j0 * lda;
-            T* A12 = A + j0 + (j0 + jb) * lda;
-            trsm_lower_blocked<T>(A11, lda, A12, lda, jb, right, up, st);
-            s = block_update(A + (j0 + jb) + j0 * lda, lda, A12, lda, A + (j0 + jb) + (j0 + jb) * lda, lda, right, right,
-                             jb, up, st);
-            if (s != MW_OK) return s;
-        }
-        MW_CHECK_CUDA(cudaGetLastError());
-    }
-    // a barrier timeout anywhere is reported in info[1]
-    MW_CHECK_CUDA(cudaMemcpyAsync(info + 1, &pws->err, sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    return MW_OK;
-}
-
 // ------------------------------------------------------------ look-ahead
 // Right-looking LU with a look-ahead of one block (both precisions).
 // The factorisation splits into two streams:
@@ -2269,8 +2224,8 @@ static mw_status getrs(int64_t n, int64_t nrhs, const T* LU, int64_t lda, const 
 
 // Orders one cluster factors and solves by itself (lu_cluster.cu); beyond,
 // the blocked factorisation's update on every SM wins.  Measured on B200
-// with 17 right-hand sides: 0.52 ms at 300, 1.48 ms at 640 in one launch,
-// 2.12 ms at 656 by blocks.
+// with 17 right-hand sides: 0.50 ms at 300, 1.43 ms at 640 in one launch,
+// 1.60 ms at 641 by blocks.
 static int64_t zlu_full_max() { return 640; }
 // A batch fills the device with clusters up to the order its back
 // substitution holds; a few matrices alone follow the rule of one.

@@ -30,7 +30,7 @@
 //
 // Measured on B200 (order 306, one right-hand side): 2.0 ms as a sequence of
 // cooperative panels, swaps, leaves and products, 0.52 ms as one launch; 64
-// such systems 125 ms one after the other, 0.88 ms as one batch.  A column
+// such systems 125 ms one after the other, 0.80 ms as one batch.  A column
 // of the exchange costs about 2,000 cycles, latencies all: the pivot's pick
 // and reciprocal 600, the next search 200, sending the row 400, the flight
 // (the other columns' update runs under it) 650.  512 threads a CTA with one
@@ -952,7 +952,8 @@ mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas
     // CTAs per cluster: one up to a single panel, eight up to 256 rows (the
     // panel is one CTA's, the rest of the work still spreads: 49 us at order
     // 21 against 66 with one CTA, 355 at 200 against 408 with four and 362
-    // with sixteen), sixteen beyond (549 against 601 us at 300)
+    // with sixteen), sixteen beyond (549 against 601 us at 300); the panels have
+    // become quicker for all of them since: 43, 306 and 495 us
     const int want = m <= kW ? 1 : (m <= kCT ? 8 : kMaxC);
     int C = 1;
     while (2 * C <= cap && C < want && C < max_cluster<1>()) C *= 2;
@@ -1005,7 +1006,8 @@ class Pace {
 // rest's product is one block per tile, so that SMs free up in between and
 // the next panel's cluster finds its sixteen together.  Measured on B200,
 // factorisation and solve with 64 right-hand sides, one stream against two:
-// 11.2 -> 9.5 ms at order 2,624, 32.9 -> 25.2 at 5,000, 162 -> 133 at 10,496.
+// 11.2 -> 9.5 ms at order 2,624, 32.9 -> 25.2 at 5,000, 162 -> 133 at 10,496 (8.2, 20.8 and 121 since, with
+// quicker updates and block solves).
 mw_status zlu_blocked(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* info, cd* B, int64_t ldb, int64_t nrhs,
                       int32_t* rid, const volatile int32_t* cancel, cudaStream_t caller) {
     const int nb = kZluBlock;
