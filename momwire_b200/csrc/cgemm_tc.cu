@@ -312,8 +312,9 @@ __global__ void pack_a_kernel(const cf* __restrict__ A, int64_t lda, int64_t m, 
 // [nb][ks][chunk TC_CHUNKS][row 256][4]; zero beyond (n, 2k).  A block takes
 // 32 columns x 64 rows of B through shared memory, so that reads run down the
 // columns and writes along the plane.  A thread per float4 of the plane, its
-// reads a column apart, took 13.1 us at k = 128, n = 10240 on B200 and 11 us
-// for 192 matrices with k = 64, n <= 430; 7.0 and 7 us so.
+// reads a column apart, took 13.1 us at k = 128, n = 10240 on B200; 7.0 us so.
+// (The batched factorisation's and the static panels' solves write B's planes
+// themselves.)
 constexpr int kPackCols = 32, kPackRows = 64;
 __global__ void __launch_bounds__(256)
     pack_b_kernel(const cf* __restrict__ B, int64_t ldb, int k, int64_t n, int n_nb, int n_ks, float* __restrict__ hi,
@@ -361,6 +362,7 @@ size_t tc_pack_b_bytes(int64_t k, int64_t n) {
 // Batched: C_b (m x n, complex64 col-major) -= A_b (m x k) B_b (k x n) for
 // b < batch, matrices `sa`, `sb`, `sc` complex elements apart; packed
 // planes in `ws` (a_hi | a_lo | b_hi | b_lo, each 1 KB aligned, batch-major).
+// With B == nullptr its planes are there already (tc_batched_b_planes).
 mw_status cgemm_tc_update_batched(int64_t m, int64_t n, int64_t k, int batch, const cf* A, int64_t lda, int64_t sa,
                                   const cf* B, int64_t ldb, int64_t sb, cf* C, int64_t ldc, int64_t sc, void* ws,
                                   size_t ws_bytes, int* err, cudaStream_t st, int max_ctas) {
@@ -383,8 +385,8 @@ mw_status cgemm_tc_update_batched(int64_t m, int64_t n, int64_t k, int batch, co
         const int64_t qa = (int64_t)n_mb * n_ks * TC_CHUNKS * TC_M;
         const dim3 ga((unsigned)((qa + 255) / 256), (unsigned)batch), gb(pack_b_blocks(n_nb, n_ks), (unsigned)batch);
         pack_a_kernel<<<ga, 256, 0, st>>>(A, lda, m, k, n_mb, n_ks, a_hi, a_lo, sa, (int64_t)(ab / 4));
-        pack_b_kernel<<<gb, 256, 0, st>>>(B, ldb, (int)k, n, n_nb, n_ks, b_hi, b_lo, sb, (int64_t)(bb / 4));
-        count_launch(2);
+        if (B) pack_b_kernel<<<gb, 256, 0, st>>>(B, ldb, (int)k, n, n_nb, n_ks, b_hi, b_lo, sb, (int64_t)(bb / 4));
+        count_launch(B ? 2 : 1);
     }
     static int sms = 0;
     if (sms == 0) {
@@ -410,6 +412,18 @@ mw_status cgemm_tc_update_batched(int64_t m, int64_t n, int64_t k, int batch, co
     MW_CHECK_CUDA(cudaGetLastError());
     count_launch();
     return MW_OK;
+}
+
+// Where cgemm_tc_update_batched(m, n, k, batch) keeps the B planes in its
+// workspace, and the floats between those of consecutive matrices.
+void tc_batched_b_planes(void* ws, int64_t m, int64_t n, int64_t k, int batch, float** b_hi, float** b_lo,
+                         int64_t* p_stride) {
+    auto al = [](size_t x) { return (x + 1023) & ~size_t(1023); };
+    const size_t ab = al(tc_pack_a_bytes(m, k) * batch), bb = tc_pack_b_bytes(k, n);
+    char* w = static_cast<char*>(ws);
+    *b_hi = reinterpret_cast<float*>(w + 2 * ab);
+    *b_lo = reinterpret_cast<float*>(w + 2 * ab + al(bb * batch));
+    *p_stride = (int64_t)(bb / 4);
 }
 
 // The four planes inside a workspace laid out as cgemm_tc_workspace(m_max,

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "tc_layout.cuh"
 
 namespace mw {
 
@@ -24,6 +25,8 @@ mw_status cgemm_tc_update_batched(int64_t m, int64_t n, int64_t k, int batch, co
                                   const cf* B, int64_t ldb, int64_t sb, cf* C, int64_t ldc, int64_t sc, void* ws,
                                   size_t ws_bytes, int* err, cudaStream_t st, int max_ctas);
 size_t cgemm_tc_workspace_batched(int64_t m, int64_t n, int64_t k, int batch);
+void tc_batched_b_planes(void* ws, int64_t m, int64_t n, int64_t k, int batch, float** b_hi, float** b_lo,
+                         int64_t* p_stride);
 
 constexpr int kBNB = 16;       // default panel width of the batched factorisation
 constexpr int kBNBMax = 32;    // widest panel of the batched factorisation (<= kBOuter)
@@ -212,10 +215,14 @@ __global__ void __launch_bounds__(NT) panel_rows_kernel(cf* A, int64_t lda, int6
 static void panel_batched(cf* A, int64_t lda, int64_t stride, int n, int j0, int jb, int32_t* ipiv, int32_t* info,
                           int batch, cudaStream_t st) {
     const int m = n - j0, nt = (m + 31) / 32 * 32;
+    // (768 threads leave 85 registers a thread and no spill; 1,024 leave 64: 59
+    // against 65 us a panel of 16 columns and 513 to 768 rows)
     if (jb <= 8 && m <= 1024)
         panel_rows_kernel<8, 1024><<<batch, nt, 0, st>>>(A, lda, stride, n, j0, jb, ipiv, info);
     else if (jb <= 16 && m <= 512)
         panel_rows_kernel<16, 512><<<batch, nt, 0, st>>>(A, lda, stride, n, j0, jb, ipiv, info);
+    else if (jb <= 16 && m <= 768)
+        panel_rows_kernel<16, 768><<<batch, nt, 0, st>>>(A, lda, stride, n, j0, jb, ipiv, info);
     else if (jb <= 16 && m <= 1024)
         panel_rows_kernel<16, 1024><<<batch, nt, 0, st>>>(A, lda, stride, n, j0, jb, ipiv, info);
     else if (jb <= 32 && m <= 512)
@@ -245,15 +252,20 @@ __global__ void laswp_batched_kernel(T* A, int64_t lda, int64_t stride, int col0
 // X <- L^-1 X for the unit lower jb x jb (jb <= NB) diagonal block at T, a
 // column of X to a thread, in registers; batch on blockIdx.y.  Four rows are
 // finished at a time, then leave the rows below up to date, the registers
-// turning by four; L is read as broadcasts from shared memory.  Bound by the
+// turning by four; L is read as broadcasts from shared memory.  The solved rows
+// also go out as the packed B operand of the update that follows (inner
+// dimension jb; rows past it hold zeros), which saves that its packing pass:
+// 1.7 ms of packing against 0.35 here in a sweep of 24 Yagis.  Bound by the
 // FP32 pipe (6 operations per entry of L and column).  A warp per column with
 // a shuffle per row took 330 us for 64 x 373, 192 matrices, on B200; 74 us so (mean of the
-// Yagi sweep's launches).
+// Yagi sweep's launches), 81 with the packed operand.
 // submul_rn's form is that kernel's.
 constexpr int kTrsmThreads = 64;
 template <int NB>
 __global__ void __launch_bounds__(kTrsmThreads) trsm_lower_batched_kernel(const cf* Tm, int64_t ldt, int64_t ts, cf* X,
-                                                                          int64_t ldx, int64_t xs, int jb, int ncols) {
+                                                                          int64_t ldx, int64_t xs, int jb, int ncols,
+                                                                          float* b_hi, float* b_lo,
+                                                                          int64_t b_pstride) {
     constexpr int kRows = 16;
     __shared__ __align__(16) cf sL[NB][NB];                       // sL[k][i] = L(i, k)
     __shared__ cf sX[kTrsmThreads / 32][32][kRows + 1];           // a warp's columns, kRows rows of them
@@ -312,6 +324,16 @@ __global__ void __launch_bounds__(kTrsmThreads) trsm_lower_batched_kernel(const 
 #pragma unroll
         for (int x = 0; x < 4; ++x) a[NB - 4 + x] = turn[x];
     }
+    if (col0 + lane < ncols) {
+        const int n_ks = tc_n_ks(jb);
+        b_hi += blockIdx.y * b_pstride;
+        b_lo += blockIdx.y * b_pstride;
+#pragma unroll
+        for (int i = 0; i < NB; i += 2)
+            if (2 * i < n_ks * TC_KS)
+                tc_store_b4(b_hi, b_lo, n_ks, col0 + lane, 2 * i,
+                            make_float4(a[i].re, a[i].im, a[i + 1].re, a[i + 1].im));
+    }
 #pragma unroll
     for (int h = 0; h < NB; h += kRows) {
         __syncwarp();
@@ -326,15 +348,20 @@ __global__ void __launch_bounds__(kTrsmThreads) trsm_lower_batched_kernel(const 
     }
 }
 
+// m: rows of the update that follows, whose workspace tc_ws takes the packed
+// operand.
 static void trsm_lower_batched(const cf* Tm, int64_t ldt, int64_t ts, cf* X, int64_t ldx, int64_t xs, int jb, int ncols,
-                               int batch, cudaStream_t st) {
+                               int batch, int m, void* tc_ws, cudaStream_t st) {
+    float *b_hi, *b_lo;
+    int64_t bp;
+    tc_batched_b_planes(tc_ws, m, ncols, jb, batch, &b_hi, &b_lo, &bp);
     const dim3 grid((unsigned)((ncols + kTrsmThreads - 1) / kTrsmThreads), (unsigned)batch);
     if (jb <= 16)
-        trsm_lower_batched_kernel<16><<<grid, kTrsmThreads, 0, st>>>(Tm, ldt, ts, X, ldx, xs, jb, ncols);
+        trsm_lower_batched_kernel<16><<<grid, kTrsmThreads, 0, st>>>(Tm, ldt, ts, X, ldx, xs, jb, ncols, b_hi, b_lo, bp);
     else if (jb <= 32)
-        trsm_lower_batched_kernel<32><<<grid, kTrsmThreads, 0, st>>>(Tm, ldt, ts, X, ldx, xs, jb, ncols);
+        trsm_lower_batched_kernel<32><<<grid, kTrsmThreads, 0, st>>>(Tm, ldt, ts, X, ldx, xs, jb, ncols, b_hi, b_lo, bp);
     else
-        trsm_lower_batched_kernel<64><<<grid, kTrsmThreads, 0, st>>>(Tm, ldt, ts, X, ldx, xs, jb, ncols);
+        trsm_lower_batched_kernel<64><<<grid, kTrsmThreads, 0, st>>>(Tm, ldt, ts, X, ldx, xs, jb, ncols, b_hi, b_lo, bp);
     count_launch();
 }
 
@@ -637,11 +664,11 @@ static mw_status cgetrf_batched(int n, int batch, cf* A, int64_t lda, int64_t st
                 cf* A12 = A + j0 + (int64_t)(j0 + jb) * lda;
                 {
                     ProfileScope ps(PC_TRSM, st, 4.0 * (double)jb * jb * inner * batch);
-                    trsm_lower_batched(A11, lda, stride, A12, lda, stride, jb, inner, batch, st);
+                    trsm_lower_batched(A11, lda, stride, A12, lda, stride, jb, inner, batch, n - j0 - jb, w.tc, st);
                 }
                 count_launch();
                 mw_status s = cgemm_tc_update_batched(n - j0 - jb, inner, jb, batch, A + (j0 + jb) + (int64_t)j0 * lda,
-                                                      lda, stride, A12, lda, stride,
+                                                      lda, stride, nullptr, 0, 0,
                                                       A + (j0 + jb) + (int64_t)(j0 + jb) * lda, lda, stride, w.tc,
                                                       w.tc_bytes, w.tc_err, st, 0);
                 if (s != MW_OK) return s;
@@ -658,11 +685,11 @@ static mw_status cgetrf_batched(int n, int batch, cf* A, int64_t lda, int64_t st
             cf* A12 = A + J0 + (int64_t)(J0 + bw) * lda;
             {
                 ProfileScope ps(PC_TRSM, st, 4.0 * (double)bw * bw * right * batch);
-                trsm_lower_batched(A11, lda, stride, A12, lda, stride, bw, right, batch, st);
+                trsm_lower_batched(A11, lda, stride, A12, lda, stride, bw, right, batch, right, w.tc, st);
             }
             count_launch();
             mw_status s = cgemm_tc_update_batched(right, right, bw, batch, A + (J0 + bw) + (int64_t)J0 * lda, lda,
-                                                  stride, A12, lda, stride, A + (J0 + bw) + (int64_t)(J0 + bw) * lda,
+                                                  stride, nullptr, 0, 0, A + (J0 + bw) + (int64_t)(J0 + bw) * lda,
                                                   lda, stride, w.tc, w.tc_bytes, w.tc_err, st, 0);
             if (s != MW_OK) return s;
         }
