@@ -560,7 +560,7 @@ static mw_status launch_fill(const FillArgs& A, const GLParams& gl, cudaStream_t
     // copy's roundings to 6e-8 (16 x 16 array, 10,496 unknowns), and this
     // kernel's sums differ from fill_rows.cu's by 1e-13 of an entry, enough to
     // turn a thousand of them: there Z keeps fill_rows.cu's order of sums,
-    // 11.9 ms against 6.7 here.  Sweeps' small systems move by 1e-11.
+    // 11.0 ms against 6.7 here.  Sweeps' small systems move by 1e-11.
     if (A.Z32 && A.nbatch == 0) return fill_rows(A, gl, IMAGE, EK, fill_flops(D, gl.nq, A.seg.n_seg, A.basis.n_basis), st);
     const size_t smem = FillSmem<D, IMAGE>(gl.nq, A.basis.max_tile_seg, A.basis.max_tile_basis).bytes;
     const size_t fit = kFillSmemSM / (smem + 1024);

@@ -14,7 +14,8 @@
 // thread computes a segment pair.  Bound by the FP64 pipe: 62 operations a
 // sample against 36 in fill.cu, whose order is free.  Four lanes to a pair,
 // each an observer point, and a shuffle reduction of the 18 sums took 13.3 ms
-// on the 16 x 16 array (10,496 unknowns) on B200; 11.9 ms so.
+// on the 16 x 16 array (10,496 unknowns) on B200; 11.0 ms so, 11.9 with the full
+// sine and cosine in line and every step tested for the series' range.
 #include "common.cuh"
 #include "fill_args.cuh"
 #include "ground_weights.cuh"
@@ -92,10 +93,14 @@ __device__ __forceinline__ void phase_step_long(double x, double* sx, double* cx
     *sx = fma(s * t, x, x);
 }
 
+// (out of line: in line it is most of a pair's code)
+__device__ __noinline__ void full_phase(double x, double* s, double* c) { sincos(x, s, c); }
+
 // The sums over the source points of observer point qi, one per source power.
 // NQ > 0: the quadrature order is known at compile time (nq == NQ), so the
 // source-point loop unrolls and its independent samples interleave.
-template <int D, bool EK, int NQ = 0>
+// NARROW: no phase step of the tile pair exceeds kRowPhaseMax.
+template <int D, bool EK, int NQ, bool NARROW>
 __device__ __forceinline__ void pair_row(const double* si, const double* sj, int nq_rt, int qi,
                                          double k, bool ek_on, cd accP[D + 1]) {
     constexpr int NM = D + 1;
@@ -114,17 +119,19 @@ __device__ __forceinline__ void pair_row(const double* si, const double* sj, int
         double dx = xi - sj[r * 3 + 0];
         double dy = yi - sj[r * 3 + 1];
         double dz = zi - sj[r * 3 + 2];
-        double R2 = dx * dx + dy * dy + dz * dz + a2;
+        // (roundings spelled out: which products are fused must not depend on
+        // the code around them)
+        const double R2 = __dadd_rn(__fma_rn(dz, dz, __fma_rn(dx, dx, __dmul_rn(dy, dy))), a2);
         // one reciprocal square root serves both R and 1/R
         double iR = rsqrt(R2);
-        double R = R2 * iR;
+        const double R = __dmul_rn(R2, iR);
         double s, c;
         // the first source point's phase in full; the others rotate it by
         // k (R - R0), at most k times a segment length, through that angle's
         // Taylor series (phase_step) -- a full sincos where it is wider
-        const double x = k * (R - R0);
-        if (r == 0 || fabs(x) > kRowPhaseMax) {
-            sincos(k * R, &s, &c);
+        const double x = __dmul_rn(k, __dsub_rn(R, R0));
+        if (r == 0 || (!NARROW && fabs(x) > kRowPhaseMax)) {
+            full_phase(k * R, &s, &c);
             if (r == 0) {
                 R0 = R;
                 s0 = s;
@@ -133,8 +140,8 @@ __device__ __forceinline__ void pair_row(const double* si, const double* sj, int
         } else {
             double sx, cx;
             phase_step_long(x, &sx, &cx);
-            s = s0 * cx + c0 * sx;
-            c = c0 * cx - s0 * sx;
+            s = __fma_rn(s0, cx, __dmul_rn(c0, sx));
+            c = __fma_rn(c0, cx, -__dmul_rn(s0, sx));
         }
         double g = kInv4Pi * iR;
         cd G = cd{c * g, -s * g};
@@ -159,7 +166,7 @@ __device__ __forceinline__ cd add_rn(cd a, cd b) { return cd{__dadd_rn(a.re, b.r
 
 // All (D+1)^2 moments of a pair by one thread, to dst: observer points q and
 // q + 4 first, then (0, 1), (2, 3), then these two sums.
-template <int D, bool EK, int NQ>
+template <int D, bool EK, int NQ, bool NARROW>
 __device__ __forceinline__ void pair_moments_rows(const double* si, const double* sj, int nq, double k, bool ek_on,
                                                   double* dst) {
     constexpr int NM = D + 1, kHalf = NQ == 4 ? 1 : 2;
@@ -167,7 +174,7 @@ __device__ __forceinline__ void pair_moments_rows(const double* si, const double
 #pragma unroll
     for (int h = 0; h < kHalf; ++h)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pair_row<D, EK, NQ>(si, sj, nq, q + 4 * h, k, ek_on, acc[h][q]);
+        for (int q = 0; q < 4; ++q) pair_row<D, EK, NQ, NARROW>(si, sj, nq, q + 4 * h, k, ek_on, acc[h][q]);
 #pragma unroll
     for (int p = 0; p < NM; ++p)
 #pragma unroll
@@ -229,7 +236,7 @@ __device__ __forceinline__ bool fill_rows_tile(const FillArgs& A, const GLParams
 
     // ---- staging: segment lists, Gauss points, basis polynomials
     const double r_ref = A.seg.radius[A.basis.tile_seg[(size_t)tr * SMAX]];
-    int odd_radius = 0;
+    int odd_radius = 0, wide = nq != 4;
     for (int i = tid; i < ns_r; i += blockDim.x) {
         int s = A.basis.tile_seg[(size_t)tr * SMAX + i];
         odd_radius |= A.seg.radius[s] != r_ref;
@@ -243,6 +250,12 @@ __device__ __forceinline__ bool fill_rows_tile(const FillArgs& A, const GLParams
     for (int i = tid; i < ns_c; i += blockDim.x) {
         int s = A.basis.tile_seg[(size_t)tc * SMAX + i];
         odd_radius |= A.seg.radius[s] != r_ref;
+        {
+            // a phase step is at most k times the source segment's length
+            const double *l = A.seg.seg_l + 3 * s, *r = A.seg.seg_r + 3 * s;
+            const double dx = r[0] - l[0], dy = r[1] - l[1], dz = r[2] - l[2];
+            wide |= !(kz * sqrt(dx * dx + dy * dy + dz * dz) < 0.98 * kRowPhaseMax);
+        }
         s_seg_c[i] = s;
         s_edge_c[i] = A.seg.edge[s];
         s_pos_c[i] = A.seg.pos_in_edge[s];
@@ -257,6 +270,8 @@ __device__ __forceinline__ bool fill_rows_tile(const FillArgs& A, const GLParams
     for (int i = tid; i < nb_r * NM; i += blockDim.x) s_loc_r[i] = A.basis.loc[(size_t)fb_r * NM + i];
     for (int i = tid; i < nb_c * NM; i += blockDim.x) s_loc_c[i] = A.basis.loc[(size_t)fb_c * NM + i];
     const bool mirror = __syncthreads_or(odd_radius) == 0 && allow_mirror;
+    // the default rule, short segments: unrolled, with no step's own test
+    const bool narrow = __syncthreads_or(wide) == 0;
 
     // ---- phase A: moments of every staged segment pair, a thread each
     const int npair = ns_r * ns_c;
@@ -271,10 +286,10 @@ __device__ __forceinline__ bool fill_rows_tile(const FillArgs& A, const GLParams
             for (int x = 0; x < NMM * 2; ++x) dst[x] = src[x];
         } else {
             const bool ek_on = EK && (s_grp_r[li] == s_grp_c[lj]);
-            if (nq == 4)
-                pair_moments_rows<D, EK, 4>(s_row + li * SD, s_col + lj * SD, 4, kz, ek_on, dst);
+            if (narrow)
+                pair_moments_rows<D, EK, 4, true>(s_row + li * SD, s_col + lj * SD, 4, kz, ek_on, dst);
             else
-                pair_moments_rows<D, EK, 0>(s_row + li * SD, s_col + lj * SD, nq, kz, ek_on, dst);
+                pair_moments_rows<D, EK, 0, false>(s_row + li * SD, s_col + lj * SD, nq, kz, ek_on, dst);
         }
         if (IMAGE) {
                 // per-pair image weights
