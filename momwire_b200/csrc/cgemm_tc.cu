@@ -15,8 +15,8 @@
 //               (M=128, N=256, K=8, kind::tf32) into one of two TMEM
 //               accumulators and commits to mbarriers;
 //   warps 2..   epilogue: tcgen05.ld the accumulator, C -= D with coalesced
-//               loads/stores (two warps per TMEM lane quadrant, each half
-//               of the columns, so twice the loads are in flight), then
+//               loads/stores (two warps per TMEM lane quadrant, sharing the
+//               tile's columns, so twice the loads are in flight), then
 //               hand the accumulator back.
 // Operands are packed by the two pack kernels below into the shared-memory
 // image of a K-major, no-swizzle UMMA tile: [block][stage][chunk][row][4],
