@@ -251,10 +251,10 @@ __device__ __forceinline__ bool fill_rows_tile(const FillArgs& A, const GLParams
         int s = A.basis.tile_seg[(size_t)tc * SMAX + i];
         odd_radius |= A.seg.radius[s] != r_ref;
         {
-            // a phase step is at most k times the source segment's length
+            // a phase step is at most |k| times the source segment's length
             const double *l = A.seg.seg_l + 3 * s, *r = A.seg.seg_r + 3 * s;
             const double dx = r[0] - l[0], dy = r[1] - l[1], dz = r[2] - l[2];
-            wide |= !(kz * sqrt(dx * dx + dy * dy + dz * dz) < 0.98 * kRowPhaseMax);
+            wide |= !(fabs(kz) * sqrt(dx * dx + dy * dy + dz * dz) < 0.98 * kRowPhaseMax);
         }
         s_seg_c[i] = s;
         s_edge_c[i] = A.seg.edge[s];

@@ -7,7 +7,7 @@
 // per SM), so the samples are stripped to what differs between them:
 //   * the phase of the first node pair, exp(-j k R_00) / (4 pi), multiplies
 //     the finished moments; a sample only needs exp(-j k (R - R_00)), whose
-//     argument is at most k (h_i + h_j), from a Taylor series as long as that
+//     argument is at most |k| (h_i + h_j), from a Taylor series as long as that
 //     bound asks for (a warp-uniform choice);
 //   * one reciprocal square root, without special cases, serves R and 1 / R.
 // That is 36 FP64 operations a sample instead of about 62, and no shuffles
@@ -223,7 +223,8 @@ template <int D, bool EK>
 __device__ __forceinline__ void pair_moments_any(const double* si, const double* sj, int nq, double k, double a2,
                                                  double ek_a, bool active, cd* dst) {
     constexpr int NM = D + 1;
-    const double span = active ? k * (seg_tail<D>(si, nq)[7] + seg_tail<D>(sj, nq)[7]) : 0.0;
+    // (the sign of k, that of the time convention, is free)
+    const double span = active ? fabs(k) * (seg_tail<D>(si, nq)[7] + seg_tail<D>(sj, nq)[7]) : 0.0;
     const bool brief = __all_sync(0xffffffffu, span <= kPhaseShort);
     const bool series = __all_sync(0xffffffffu, span <= kPhaseLong);
     if (!active) return;
