@@ -1,6 +1,6 @@
 // Segment-pair moments and their Galerkin contraction (FP64, sm_100a): the
-// arithmetic shared by the impedance fill (fill.cu) and the off-edge block
-// sampler (offedge_block.cu).
+// arithmetic of the impedance fill (fill.cu), whose phase series and reciprocal
+// root the off-edge block sampler (offedge_block.cu) uses too.
 //
 // A pair's (d+1)^2 moments J[p][P] = sum_qr w_q u_q^p  G(R_qr)  w_r u_r^P are
 // computed by ONE thread.  What bounds it is the FP64 pipe (64 lanes a clock

@@ -1,0 +1,72 @@
+"""Precision of the block sampler on far blocks of smooth bases, where the
+charges of a basis's wings cancel: against the oracle (both take the phases
+at the rounded k R).
+
+Tolerance, in the block's norm: u times the norm of the sums of the terms'
+magnitudes.  A term carries about eight roundings of u / sqrt(3) each; the 64
+to 144 terms of an entry being independent leaves a third of the tolerance,
+moments contracted with cancelling coefficients go past it."""
+
+import numpy as np
+import pytest
+
+from oracle import block_oracle as BO
+
+from momwire_b200 import accel
+
+pytestmark = pytest.mark.gpu
+
+UNIT = {1: [[0, 1], [1, -1]], 2: [[0, 0, 0.5], [0.5, 1, -1], [0.5, -1, 0.5]]}
+
+
+def _wires(n_wires, n_seg, degree, x0):
+    """Parallel half-wave wires from x0 on, their inner B-splines."""
+    L = 0.48 * (1 + 0.003 * np.arange(n_wires))
+    supp, polys, l, r = [], [], [], []
+    for w in range(n_wires):
+        h = L[w] / n_seg
+        z = -L[w] / 2 + h * np.arange(n_seg + 1)
+        p = np.stack([np.full(n_seg + 1, x0 + 0.5 * (w % 2)), np.full(n_seg + 1, 0.5 * (w // 2)), z], 1)
+        for j in range(n_seg - degree):
+            supp.append(w * n_seg + j + np.arange(degree + 1))
+            polys.append(np.array(UNIT[degree]) / h ** np.arange(degree + 1))
+        l.append(p[:-1])
+        r.append(p[1:])
+    l, r = np.vstack(l), np.vstack(r)
+    return np.array(supp), np.array(polys), l, r, np.tile([0.0, 0.0, 1.0], (len(l), 1))
+
+
+def _magnitudes(I, J, a2, k, om, eps, mu, t, w):
+    """Per entry, the sum of its terms' magnitudes (parallel wires)."""
+    out = 0.0
+    nodes = []
+    for supp, polys, l, r, _t in (I, J):
+        h = np.linalg.norm(r - l, axis=1)[supp]
+        u = h[..., None] * t
+        e = np.arange(polys.shape[2])
+        wl = w * h[..., None]
+        f = np.abs((u[..., None] ** e * polys[:, :, None, :]).sum(-1)) * wl
+        df = np.abs((e * u[..., None] ** np.maximum(e - 1, 0) * polys[:, :, None, :]).sum(-1)) * wl
+        x = (1 - t)[:, None] * l[supp][:, :, None, :] + t[:, None] * r[supp][:, :, None, :]
+        n = len(supp)
+        nodes.append((f.reshape(n, -1), df.reshape(n, -1), x.reshape(n, -1, 3)))
+    (fi, gi, xi), (fj, gj, xj) = nodes
+    for q in range(fi.shape[1]):
+        for s in range(fj.shape[1]):
+            G = 1.0 / (4 * np.pi * np.sqrt(((xi[:, None, q] - xj[None, :, s]) ** 2).sum(-1) + a2))
+            out = out + G * (om * mu * fi[:, q, None] * fj[None, :, s] + gi[:, q, None] * gj[None, :, s] / (om * eps))
+    return out
+
+
+@pytest.mark.parametrize("degree", [1, 2])
+def test_far_block_keeps_the_terms_precision(degree, cuda_device):
+    I, J = _wires(3, 41, degree, 0.0), _wires(4, 41, degree, 3.0)
+    t, w = np.polynomial.legendre.leggauss(4)
+    t, w = 0.5 * (t + 1.0), 0.5 * w
+    a2, k, eps, mu = 2.5e-7, 6.2, 8.8541878188e-12, 1.25663706127e-6
+    om = k / np.sqrt(eps * mu)
+    got = accel.bspline_assemble_offedge_block(*I, *J, a2, k, om, eps, mu, degree, t, w)
+    want = BO.offedge_block(*I, *J, a2, k, om, eps, mu, t, w, group=None, a_ek=0.0, refl=None)
+    u = np.finfo(float).eps / 2
+    tol = u * np.linalg.norm(_magnitudes(I, J, a2, k, om, eps, mu, t, w))
+    assert np.linalg.norm(got - want) < tol
