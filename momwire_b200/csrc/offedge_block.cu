@@ -61,6 +61,7 @@ struct ObArgs {
     double a2, k, omega, eps0, mu0;
     int nq;
     double t[kObMaxQ], w[kObMaxQ];
+    double reach;  // times two segments' lengths: bound of a phase step between a pair's samples
     int refl;
     double er, ei, c0r, c0i, c1r, c1i;
     double a_ek;  // > 0: extended kernel on eligible pairs
@@ -145,7 +146,8 @@ __device__ __forceinline__ int ob_list(ObShared<D>& S, int side, const ObSide& X
 
 // The nq^2 samples 4 pi G(R) of one segment pair, observer node major.  The first
 // sample's phase is taken in full and multiplies the others, whose own steps
-// are at most |k| (h_i + h_j).
+// are at most |k| (h_i + h_j) (ObArgs::reach: more where the caller's nodes
+// leave the segments).
 template <bool EK, int NQ, int MODE>
 __device__ __forceinline__ void ob_samples(const double* xi, const double* xj, int nq_rt, double k, double a2,
                                            double a_ek, cd* G) {
@@ -276,7 +278,7 @@ __global__ void __launch_bounds__(kObThreads, 3) offedge_block_kernel(ObArgs A) 
                 const bool valid = tid < nr * ns_j;
                 const int li = valid ? g0 + tid / ns_j : 0, lj = valid ? tid % ns_j : 0;
                 const double *xi = seg(0, li), *xj = seg(1, lj), *ti = xi + 3 * nq, *tj = xj + 3 * nq;
-                const double span = valid ? fabs(A.k) * (ti[6] + tj[6]) : 0.0;
+                const double span = valid ? A.reach * (ti[6] + tj[6]) : 0.0;
                 const bool brief = __all_sync(0xffffffffu, span <= kPhaseShort);
                 const bool series = __all_sync(0xffffffffu, span <= kPhaseLong);
                 if (valid) {
@@ -422,10 +424,13 @@ extern "C" mw_status mw_offedge_block(int32_t degree, const mw_block_side* I, co
     A.eps0 = freq->eps0;
     A.mu0 = freq->mu0;
     A.nq = n_qp;
+    double spread = 1.0;  // of the nodes, in segment lengths (the caller's rule need not stay on [0, 1])
     for (int i = 0; i < n_qp; ++i) {
         A.t[i] = gl_t[i];
         A.w[i] = gl_w[i];
+        spread = fmax(spread, fabs(gl_t[i] - gl_t[0]));
     }
+    A.reach = fabs(A.k) * spread;
     A.refl = refl != nullptr;
     if (refl) {
         A.er = refl->eps_re;

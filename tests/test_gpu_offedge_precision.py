@@ -10,7 +10,9 @@ moments contracted with cancelling coefficients go past it."""
 import numpy as np
 import pytest
 
+from conftest import rel_err
 from oracle import block_oracle as BO
+from test_gpu_offedge_tiles import _side
 
 from momwire_b200 import accel
 
@@ -70,3 +72,19 @@ def test_far_block_keeps_the_terms_precision(degree, cuda_device):
     u = np.finfo(float).eps / 2
     tol = u * np.linalg.norm(_magnitudes(I, J, a2, k, om, eps, mu, t, w))
     assert np.linalg.norm(got - want) < tol
+
+
+@pytest.mark.parametrize("lo,hi", [(-3.0, 4.0), (2.0, -2.0)])
+def test_nodes_off_the_segments(lo, hi, cuda_device):
+    """The rule is the caller's: nodes past a segment's ends are integrated
+    where they lie, with phase steps up to seven times those of the segments.
+    Tolerance as for the tiles, 1e-12 of the largest entry."""
+    rng = np.random.default_rng(5)
+    I, J = _side(rng, 20, 2, 9.0, False), _side(rng, 18, 2, 0.0, False)
+    t, w = np.polynomial.legendre.leggauss(4)
+    t = lo + (hi - lo) * 0.5 * (t + 1.0)
+    k = 0.45  # |k| times two lengths below 0.3: the shortest series, were it for the lengths alone
+    args = (*I[:5], *J[:5], 1e-5, k, k * 3e8, 8.85e-12, 1.2566e-6)
+    got = accel.bspline_assemble_offedge_block(*args, 2, t, 0.5 * w)
+    want = BO.offedge_block(*args, t, 0.5 * w, group=None, a_ek=0.0, refl=None)
+    assert rel_err(got, want) < 1e-12
