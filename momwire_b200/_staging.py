@@ -2,11 +2,15 @@
 
 A set of host arrays becomes one page-locked buffer (256-byte aligned
 pieces) and one stream-ordered copy: a copy per array from pageable memory
-makes the host wait for the device each time.  Results come back the same
-way, as arrays on page-locked memory that live as long as they are used.
+makes the host wait for the device each time.  A solver's results come back
+the same way, as arrays on page-locked memory that live as long as they are
+used; results that a host keeps by the thousand (``to_host``) come back as
+ordinary arrays, through a page-locked buffer of fixed size.
 """
 
 from __future__ import annotations
+
+import threading
 
 import numpy as np
 
@@ -44,3 +48,55 @@ def read_back(torch, stream, tensors):
         out.append(h)
     stream.synchronize()
     return [h.numpy() for h in out]
+
+
+class _Bounce(threading.local):
+    """Two page-locked slots and their events, per host thread and given back
+    with it."""
+
+    SLOT = 4 << 20  # bytes
+    slots = events = None
+
+    def get(self, torch):
+        if self.slots is None:
+            with torch.inference_mode(False):  # (a caller's mode must not stick to them)
+                self.slots = [torch.empty(self.SLOT, dtype=torch.uint8, pin_memory=True) for _ in range(2)]
+            self.events = {}
+        return self.slots
+
+    def event(self, torch, device, i):
+        key = (device, i)
+        if key not in self.events:
+            self.events[key] = torch.cuda.Event()
+        return self.events[key]
+
+
+_bounce = _Bounce()
+
+
+def to_host(torch, stream, t):
+    """An ordinary array with a contiguous device tensor's values: slice by
+    slice through the thread's page-locked slots, one on its way from the
+    device while the other is copied out."""
+    out = np.empty(tuple(t.shape), dtype=torch.empty(0, dtype=t.dtype).numpy().dtype)
+    if out.size == 0:
+        return out
+    slots, S = _bounce.get(torch), _bounce.SLOT
+    with torch.inference_mode():  # (no version counters, no autograd)
+        src, dst = t.view(-1).view(torch.uint8), torch.from_numpy(out.reshape(-1).view(np.uint8))
+        n = dst.numel()
+        cuts = [(o, min(o + S, n)) for o in range(0, n, S)]
+
+        def fetch(i):
+            a, b = cuts[i]
+            slots[i % 2][: b - a].copy_(src[a:b], non_blocking=True)
+            _bounce.event(torch, t.device, i % 2).record(stream)
+
+        for i in range(min(2, len(cuts))):
+            fetch(i)
+        for i, (a, b) in enumerate(cuts):
+            _bounce.event(torch, t.device, i % 2).synchronize()
+            dst[a:b].copy_(slots[i % 2][: b - a])
+            if i + 2 < len(cuts):
+                fetch(i + 2)
+    return out

@@ -9,10 +9,12 @@ the same four functions with the same arguments and the same (nI, nJ)
 complex128 result, computed by ``mw_offedge_block`` on the current CUDA
 device, so a maintainer can route those calls here (INTEGRATION.md shows
 how).  Inputs are host arrays, as the reference takes them; they are
-uploaded in one copy, the block is filled on the device and comes back on
-page-locked memory (an ordinary array that is page-locked while it lives).
+uploaded in one copy, the block is filled on the device and comes back as an
+ordinary array, through a page-locked buffer of 8 MB per host thread: an
+H-matrix host keeps its blocks, and page-locked results would lock all of
+its compressed matrix (and a new page-locked 21 MB costs 15 ms).
 A 1025 x 1311 block measured 5.6 ms through pageable copies, most of it the
-21 MB on their way back, and 0.7 ms so.
+21 MB on their way back, and 1.1 ms so, 2.5 with every block kept.
 """
 
 from __future__ import annotations
@@ -81,7 +83,7 @@ def _block(supp_I, polys_I, segl_I, segr_I, tan_I, supp_J, polys_J, segl_J, segr
     _lib.call("mw_offedge_block", int(max_d), C.byref(sI), C.byref(sJ), float(a_squared), C.byref(fr), t.size,
               t.ctypes.data, w.ctypes.data, C.byref(rf) if rf is not None else None, float(a_ek), Z.data_ptr(),
               Z.shape[1], stream.cuda_stream)
-    return _staging.read_back(torch, stream, [Z])[0][:nI, :nJ]
+    return _staging.to_host(torch, stream, Z[:nI, :nJ])
 
 
 def bspline_assemble_offedge_block(supp_I, polys_I, segl_I, segr_I, tan_I, supp_J, polys_J, segl_J, segr_J, tan_J,
