@@ -355,8 +355,10 @@ size_t mw_getrf_workspace_size(int64_t n);
  * P A = L U, pivots 1-based as LAPACK zgetrf (ipiv device, length n).
  * Replaces LAPACK zgetrf inside scipy.linalg.solve (bspline.py:2979).
  * `info` (device, 2 int32): info[0] receives LAPACK's info (0, or j+1 for an
- * exact zero pivot U(j,j)), info[1] a device wait's timeout.  `cancel` (host-mapped or device int32, may be NULL)
- * is polled between panels; a raised flag returns MW_ERR_CANCELLED.
+ * exact zero pivot U(j,j)), info[1] a device wait's timeout.  `cancel` (host-mapped int32, may be NULL)
+ * is polled before the call's first launch and between the 128-column blocks
+ * of a larger system (up to order 640 it is one launch, 1.5 ms at most); a
+ * raised flag returns MW_ERR_CANCELLED.
  */
 mw_status mw_zgetrf(int64_t n, double* A, int64_t lda, int32_t* ipiv,
                     int32_t* info, void* workspace, size_t workspace_bytes,
@@ -386,7 +388,10 @@ mw_status mw_zgesv(int64_t n, int64_t nrhs, double* A, int64_t lda, int32_t* ipi
  * its right-hand sides at B + 2 b b_stride (strides in complex elements),
  * its pivots at ipiv + b n, its two status words at info + 2 b.  Replaces
  * the stacked numpy.linalg.solve of a swept solve (bspline.py:4181-4440).
- * Workspace: mw_getrf_workspace_size(n).
+ * Workspace: mw_getrf_workspace_size(n).  Given `cancel`, systems that share
+ * a launch (order 640; 1,696 from eight systems on) are launched as many at a
+ * time as the device holds at once, one enqueued while one runs and the flag
+ * polled in between; without it all of them in one.
  */
 mw_status mw_zgesv_batched(int64_t n, int64_t nrhs, int32_t batch, double* A, int64_t lda, int64_t a_stride,
                            int32_t* ipiv, int32_t* info, double* B, int64_t ldb, int64_t b_stride,

@@ -51,7 +51,9 @@ class SolveAborted(Exception):
 class CancelToken:
     """One-shot cancellation flag shared with a solve (same surface as the
     reference's ``_cancel.CancelToken``).  The factorisation polls it
-    between panels; the host polls it at phase seams."""
+    between its launches (a system of up to 640 unknowns is one, a batch of
+    them as many as the device holds at once); the host polls it at phase
+    seams."""
 
     def __init__(self):
         self._flag = np.zeros(1, dtype=np.int32)
@@ -1361,6 +1363,7 @@ class BSplineSolver:
                     raise SolveAborted() from e
                 raise
             hinfo = info.cpu().numpy()
+            self._checkpoint()  # a flag raised during the batch, the last one too
             if np.any(hinfo[:, 1] != 0):
                 raise RuntimeError("factorisation: a bounded device wait timed out")
             if np.any(hinfo[:, 0] > 0):

@@ -2382,27 +2382,44 @@ extern "C" mw_status mw_zgesv_batched(int64_t n, int64_t nrhs, int32_t batch, do
     cd* A = reinterpret_cast<cd*>(Ad);
     cd* B = reinterpret_cast<cd*>(Bd);
     if (n <= zlu_batch_max(batch) && nrhs <= 64) {
-        if (cancel && *cancel) {
-            set_error("factorisation cancelled");
-            return MW_ERR_CANCELLED;
-        }
         ProfileScope ps(PC_FACTOR, st, batch * (8.0 / 3.0 * (double)n * n * n + 8.0 * (double)n * n * nrhs), 0.0);
         MW_CHECK_CUDA(cudaMemsetAsync(info, 0, 2 * sizeof(int32_t) * batch, st));
-        ZluArgs P{};
-        P.A = A;
-        P.lda = lda;
-        P.a_stride = a_stride;
-        P.n = P.jb = (int)n;
-        P.ipiv = ipiv;
-        P.ipiv_stride = n;
-        P.info = info;
-        P.info_stride = 2;
-        P.B = B;
-        P.ldb = ldb;
-        P.b_stride = b_stride;
-        P.nrhs = (int)nrhs;
-        P.back = 1;
-        return zlu_cluster(P, batch, st, zlu_batch_ctas(batch));
+        const int ctas = zlu_batch_ctas(batch);
+        // with a flag to poll, as many systems a launch as the device holds at
+        // once, the next one enqueued while one runs
+        const int32_t wave = cancel ? panel_sms<cd>() / zlu_cluster_ctas((int)n, ctas) : batch;
+        Pace<1> pace;
+        if (cancel) {
+            mw_status s = pace.start(st);
+            if (s != MW_OK) return s;
+        }
+        for (int32_t b0 = 0, j = 0; b0 < batch; b0 += wave, ++j) {
+            if (cancel) {
+                mw_status s = pace.step(j, st);
+                if (s != MW_OK) return s;
+                if (*cancel) {
+                    set_error("factorisation cancelled");
+                    return MW_ERR_CANCELLED;
+                }
+            }
+            ZluArgs P{};
+            P.A = A + b0 * a_stride;
+            P.lda = lda;
+            P.a_stride = a_stride;
+            P.n = P.jb = (int)n;
+            P.ipiv = ipiv + b0 * n;
+            P.ipiv_stride = n;
+            P.info = info + 2 * (int64_t)b0;
+            P.info_stride = 2;
+            P.B = B + b0 * b_stride;
+            P.ldb = ldb;
+            P.b_stride = b_stride;
+            P.nrhs = (int)nrhs;
+            P.back = 1;
+            mw_status s = zlu_cluster(P, batch - b0 < wave ? batch - b0 : wave, st, ctas);
+            if (s != MW_OK) return s;
+        }
+        return MW_OK;
     }
     for (int32_t b = 0; b < batch; ++b) {
         mw_status s = mw_zgesv(n, nrhs, reinterpret_cast<double*>(A + b * a_stride), lda, ipiv + b * n, info + 2 * b,

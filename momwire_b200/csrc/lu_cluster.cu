@@ -944,10 +944,7 @@ mw_status launch(const ZluArgs& P, int C, int batch, cudaStream_t st) {
 
 int zlu_cluster_max_rows() { return max_cluster<3>() * kCT * 3; }
 
-mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas) {
-    MW_REQUIRE(batch >= 1 && P.jb >= 1 && P.j0 >= 0 && P.j0 + P.jb <= P.n, "bad block");
-    MW_REQUIRE(!P.back || (P.j0 == 0 && P.jb == P.n && P.n <= kBackRows), "back substitution needs the whole matrix");
-    const int m = P.n - P.j0;
+int zlu_cluster_ctas(int m, int max_ctas) {
     const int cap = max_ctas > 0 && max_ctas < kMaxC ? max_ctas : kMaxC;
     // CTAs per cluster: one up to a single panel, eight up to 256 rows (the
     // panel is one CTA's, the rest of the work still spreads: 49 us at order
@@ -959,6 +956,13 @@ mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas
     while (2 * C <= cap && C < want && C < max_cluster<1>()) C *= 2;
     // enough rows per thread for the panel
     while (C < kMaxC && (m + C - 1) / C > 3 * kCT) C *= 2;
+    return C;
+}
+
+mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas) {
+    MW_REQUIRE(batch >= 1 && P.jb >= 1 && P.j0 >= 0 && P.j0 + P.jb <= P.n, "bad block");
+    MW_REQUIRE(!P.back || (P.j0 == 0 && P.jb == P.n && P.n <= kBackRows), "back substitution needs the whole matrix");
+    const int m = P.n - P.j0, C = zlu_cluster_ctas(m, max_ctas);
     const int per = (m + C - 1) / C;
     if (per <= kCT) return launch<1>(P, C, batch, st);
     if (per <= 2 * kCT) return launch<2>(P, C, batch, st);
@@ -967,37 +971,6 @@ mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas
 }
 
 // ------------------------------------------------------------------ driver
-// Keeps the host at most kDepth blocks ahead of the device, so that a
-// cancellation flag polled before each block is seen while the device still
-// works (the whole factorisation is enqueued in about two milliseconds).
-class Pace {
-  public:
-    static constexpr int kDepth = 4;
-    mw_status start(cudaStream_t st) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        MW_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
-        if (cap != cudaStreamCaptureStatusNone) return MW_OK;  // nothing runs yet
-        for (auto& e : ev_) MW_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        on_ = true;
-        return MW_OK;
-    }
-    mw_status step(int64_t j, cudaStream_t st) {
-        if (!on_) return MW_OK;
-        cudaEvent_t e = ev_[j % kDepth];
-        if (j >= kDepth) MW_CHECK_CUDA(cudaEventSynchronize(e));
-        MW_CHECK_CUDA(cudaEventRecord(e, st));
-        return MW_OK;
-    }
-    ~Pace() {
-        for (auto e : ev_)
-            if (e) cudaEventDestroy(e);
-    }
-
-  private:
-    cudaEvent_t ev_[kDepth] = {};
-    bool on_ = false;
-};
-
 // Blocked factorisation of the whole matrix with nrhs carried columns (B <-
 // L^-1 P B).  `rid`: n + 4 kZluBlock ints of workspace.  A look-ahead of one
 // block on two streams: the critical one (highest priority) updates the next
@@ -1017,7 +990,7 @@ mw_status zlu_blocked(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_t* inf
     MW_CHECK_CUDA(cudaEventRecord(zs.ev_handover, caller));
     MW_CHECK_CUDA(cudaStreamWaitEvent(st, zs.ev_handover, 0));
     MW_CHECK_CUDA(cudaStreamWaitEvent(tr, zs.ev_handover, 0));
-    Pace pace;
+    Pace<4> pace;  // (the whole factorisation is enqueued in about two milliseconds)
     if (cancel) {
         mw_status s = pace.start(st);
         if (s != MW_OK) return s;

@@ -36,8 +36,42 @@ struct ZluStreams {
 };
 mw_status zlu_streams(ZluStreams* out);
 
+// Keeps the host at most DEPTH steps ahead of the one that the device works
+// on, so that a cancellation flag polled before each step is seen meanwhile.  Off while the stream is being captured (nothing runs yet).
+template <int DEPTH>
+class Pace {
+  public:
+    mw_status start(cudaStream_t st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        MW_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
+        if (cap != cudaStreamCaptureStatusNone) return MW_OK;
+        for (auto& e : ev_) MW_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        on_ = true;
+        return MW_OK;
+    }
+    // before step j is enqueued on st
+    mw_status step(int64_t j, cudaStream_t st) {
+        if (!on_) return MW_OK;
+        cudaEvent_t e = ev_[j % DEPTH];
+        if (j >= DEPTH) MW_CHECK_CUDA(cudaEventSynchronize(e));
+        MW_CHECK_CUDA(cudaEventRecord(e, st));
+        return MW_OK;
+    }
+    ~Pace() {
+        for (auto e : ev_)
+            if (e) cudaEventDestroy(e);
+    }
+
+  private:
+    cudaEvent_t ev_[DEPTH] = {};
+    bool on_ = false;
+};
+
 // Rows one cluster can hold.
 int zlu_cluster_max_rows();
+// CTAs of the cluster that takes m rows, at most max_ctas (> 0) if they hold
+// them.
+int zlu_cluster_ctas(int m, int max_ctas);
 mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas = 0);
 
 // Columns of a block of the blocked factorisation.
