@@ -66,7 +66,7 @@ int32_t mw_profile_read(int32_t cls, int64_t* launches, double* total_ms,
  * kernels have no device waits): runs one of this library's bounded device
  * waits with a short limit and an event that never comes -- which = 0 the
  * complex128 panel's grid barrier, 1 the tensor-core kernels' mbarrier
- * wait -- and returns the status the wait recorded: MW_ERR_TIMEOUT when it
+ * wait, 2 the cluster LU's pivot exchange -- and returns the status the wait recorded: MW_ERR_TIMEOUT when it
  * gave up as designed (the context stays usable).  spin_limit in
  * [256, 2^24]; workspace: 16 bytes of device memory; synchronises stream. */
 mw_status mw_selftest_wait_timeout(int32_t which, int64_t spin_limit, void* workspace, void* stream);

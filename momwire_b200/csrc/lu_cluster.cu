@@ -112,6 +112,21 @@ __device__ __forceinline__ bool mbar_try(unsigned mbar, unsigned parity) {
     return ok != 0;
 }
 
+// Waits for the phase of an mbarrier, all lanes of a warp together.  True when
+// it gave up, after `limit` polls of at most a microsecond, and recorded
+// MW_ERR_TIMEOUT.
+__device__ __forceinline__ bool exchange_wait(unsigned mbar, unsigned parity, int limit, int32_t* err) {
+    int spins = 0;
+    bool dead = false;
+    while (!mbar_try(mbar, parity))
+        if (++spins > limit) {
+            dead = true;
+            *err = MW_ERR_TIMEOUT;
+            break;
+        }
+    return __any_sync(0xffffffffu, dead);
+}
+
 // L2 loads: another CTA of the cluster may have written the line
 __device__ __forceinline__ cd ld2(const cd* p) {
     const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
@@ -428,16 +443,8 @@ __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
             for (int jj = 0; jj < w; ++jj, ++step) {
                 const int buf = step & 3;
                 const unsigned c = (unsigned)(c0 + jj);
-                if (!dead) {
-                    int spins = 0;
-                    while (!mbar_try(smem_u32(&S.mbar[buf]), (unsigned)((step >> 2) & 1)))
-                        if (++spins > kSpinLimit) {
-                            dead = true;
-                            info[1] = MW_ERR_TIMEOUT;
-                            break;
-                        }
-                    dead = __any_sync(0xffffffffu, dead);
-                }
+                if (!dead)
+                    dead = exchange_wait(smem_u32(&S.mbar[buf]), (unsigned)((step >> 2) & 1), kSpinLimit, info + 1);
                 // the winner, from this CTA's own copies; each lane takes the
                 // reciprocal of one candidate in the reduction's shadow
                 const uint4 k = S.key[buf][lane & (kMaxC - 1)];
@@ -727,6 +734,22 @@ __global__ void __launch_bounds__(kCT, 1) zlu_cluster_kernel(ZluArgs P) {
     }
 }
 
+// The exchange's wait on rows that are expected and never sent.
+__global__ void __launch_bounds__(32) exchange_wait_selftest_kernel(int32_t* err, int limit) {
+    __shared__ __align__(8) unsigned long long mbar;
+    const unsigned m = smem_u32(&mbar);
+    if (threadIdx.x == 0) {
+        mbar_init(m, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    cluster_barrier();
+    mbar_expect(threadIdx.x == 0, m, 2 * kXchBytes);
+    exchange_wait(m, 0, limit, err);
+    __syncwarp();
+    cluster_barrier();
+}
+
 // ------------------------------------------------------------ block solves
 // X <- T^-1 P X for the jb <= 128 rows [j0, j0 + jb) of many columns, T the
 // unit lower (or, UPPER, the upper) triangle of the diagonal block and P the
@@ -968,6 +991,21 @@ mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas
     if (per <= 2 * kCT) return launch<2>(P, C, batch, st);
     MW_REQUIRE(per <= 3 * kCT, "block of %d rows too large for one cluster", m);
     return launch<3>(P, C, batch, st);
+}
+
+mw_status zlu_exchange_wait_selftest(int32_t* err, int limit, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(32);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    MW_CHECK_CUDA(cudaLaunchKernelEx(&cfg, exchange_wait_selftest_kernel, err, limit));
+    return MW_OK;
 }
 
 // ------------------------------------------------------------------ driver

@@ -73,6 +73,8 @@ int zlu_cluster_max_rows();
 // them.
 int zlu_cluster_ctas(int m, int max_ctas);
 mw_status zlu_cluster(const ZluArgs& P, int batch, cudaStream_t st, int max_ctas = 0);
+// Makes the exchange's wait run out after `limit` polls (selftest.cu).
+mw_status zlu_exchange_wait_selftest(int32_t* err, int limit, cudaStream_t st);
 
 // Columns of a block of the blocked factorisation.
 constexpr int kZluBlock = 128;

@@ -1,13 +1,17 @@
 // mw_selftest_wait_timeout: makes one of the library's bounded device waits
 // run out on purpose, with a short spin limit, so that a test can check
 // that the wait ends, records MW_ERR_TIMEOUT and leaves the context usable.
-// The waits are the production helpers themselves (waits.cuh, tc_common.cuh);
+// The waits are the production helpers themselves (waits.cuh, tc_common.cuh,
+// lu_cluster.cu);
 // only the limit is shortened and the awaited event never comes:
 //   which = 0: the grid barrier of the complex128 LU panel, two CTAs waiting
 //              for three arrivals;
 //   which = 1: the mbarrier wait of the tensor-core kernels, one thread
-//              waiting on a barrier that nobody arrives at.
+//              waiting on a barrier that nobody arrives at;
+//   which = 2: the pivot exchange of the complex128 cluster LU, two CTAs of a
+//              cluster waiting for rows that neither sends.
 #include "common.cuh"
+#include "lu_cluster.cuh"
 #include "tc_common.cuh"
 #include "waits.cuh"
 
@@ -35,7 +39,7 @@ __global__ void mbar_wait_selftest_kernel(int* err, long long limit) {
 
 extern "C" mw_status mw_selftest_wait_timeout(int32_t which, int64_t spin_limit, void* workspace, void* stream) {
     using namespace mw;
-    MW_REQUIRE(which == 0 || which == 1, "which must be 0 (grid barrier) or 1 (mbarrier), got %d", which);
+    MW_REQUIRE(which >= 0 && which <= 2, "which must be 0 (grid barrier), 1 (mbarrier) or 2 (exchange), got %d", which);
     MW_REQUIRE(spin_limit >= 256 && spin_limit <= (int64_t(1) << 24),
                "spin_limit must lie in [256, 2^24] (got %lld)", (long long)spin_limit);
     MW_REQUIRE(workspace != nullptr, "NULL workspace");
@@ -44,16 +48,18 @@ extern "C" mw_status mw_selftest_wait_timeout(int32_t which, int64_t spin_limit,
     MW_CHECK_CUDA(cudaMemsetAsync(ws, 0, sizeof(PanelWs), st));
     if (which == 0)
         grid_wait_selftest_kernel<<<2, 32, 0, st>>>(ws, spin_limit);
-    else
+    else if (which == 1)
         mbar_wait_selftest_kernel<<<1, 32, 0, st>>>(&ws->err, spin_limit);
+    else if (mw_status s = zlu_exchange_wait_selftest(&ws->err, (int)spin_limit, st); s != MW_OK)
+        return s;
     count_launch();
     MW_CHECK_CUDA(cudaGetLastError());
     int err = 0;
     MW_CHECK_CUDA(cudaMemcpyAsync(&err, &ws->err, sizeof(int), cudaMemcpyDeviceToHost, st));
     MW_CHECK_CUDA(cudaStreamSynchronize(st));
     if (err != 0) {
-        set_error("bounded %s wait gave up after %lld polls (self-test)", which == 0 ? "grid barrier" : "mbarrier",
-                  (long long)spin_limit);
+        static const char* const name[] = {"grid barrier", "mbarrier", "exchange"};
+        set_error("bounded %s wait gave up after %lld polls (self-test)", name[which], (long long)spin_limit);
         return err;
     }
     return MW_OK;
