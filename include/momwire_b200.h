@@ -71,6 +71,12 @@ int32_t mw_profile_read(int32_t cls, int64_t* launches, double* total_ms,
  * [256, 2^24]; workspace: 16 bytes of device memory; synchronises stream. */
 mw_status mw_selftest_wait_timeout(int32_t which, int64_t spin_limit, void* workspace, void* stream);
 
+/* The kernels' own elementary functions on n pairs of doubles (device, 16-byte
+ * aligned), results in pairs: which = 0 1 / sqrt(x) and sqrt(x) of the first, 1
+ * the complex reciprocal, 2 / 3 / 4 sine and cosine of the first by the phase
+ * series to 0.3, to 0.75, and with the full functions beyond. */
+mw_status mw_selftest_math(int32_t which, int64_t n, const double* in, double* out, void* stream);
+
 /* Ground models served by the fill (bspline.py:182-287 ground kwargs). */
 #define MW_GROUND_NONE        0  /* free space                              */
 #define MW_GROUND_PEC         1  /* perfect image, ground_eps=None          */

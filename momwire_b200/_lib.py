@@ -146,6 +146,7 @@ _SIGS = {
     "mw_profile_enable": (None, [i32]),
     "mw_profile_read": (i32, [i32, C.POINTER(i64), C.POINTER(f64), C.POINTER(f64), C.POINTER(f64)]),
     "mw_selftest_wait_timeout": (i32, [i32, i64, vp, vp]),
+    "mw_selftest_math": (i32, [i32, i64, vp, vp, vp]),
     "mw_set_mixed_pivoting": (i32, [i32]),
     "mw_last_mixed_pivoting": (i32, []),
     "mw_last_mixed_growth": (f64, []),

@@ -147,34 +147,6 @@ __device__ __forceinline__ cd csub_mul(cd c, cd a, cd b) {  // c - a b
     return c;
 }
 
-// 1 / z with one reciprocal: z is first scaled by the power of two that
-// brings its larger part into [1, 2) (exact), so |z|^2 neither overflows nor
-// loses bits.  recip_special: zero, subnormal, infinite and NaN z, which take
-// the plain division instead.
-__device__ __forceinline__ int recip_exp(cd z) {
-    return (int)((__double_as_longlong(fmax(fabs(z.re), fabs(z.im))) >> 52) & 0x7ff);
-}
-__device__ __forceinline__ bool recip_special(cd z) {
-    const int ex = recip_exp(z);
-    return ex < 2 || ex > 2044;
-}
-// (the reciprocal by Newton's iteration from the single-precision one: |z|^2
-// is in [1, 8), two steps reach the last bits, and nothing branches)
-__device__ __forceinline__ cd recip_fast(cd z) {
-    const int ex = min(max(recip_exp(z), 2), 2044);
-    const double s = __longlong_as_double((long long)(2046 - ex) << 52);  // 2^(1023 - ex)
-    const double x = z.re * s, y = z.im * s;
-    const double d = fma(x, x, y * y);
-    float r0;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"((float)d));
-    double r = (double)r0;
-    r = fma(r, fma(-d, r, 1.0), r);
-    r = fma(r, fma(-d, r, 1.0), r);
-    const double t = s * r;
-    return cd{x * t, -(y * t)};
-}
-__device__ __forceinline__ cd crecip(cd z) { return recip_special(z) ? cdiv(cd{1.0, 0.0}, z) : recip_fast(z); }
-
 // Warp-wide best of (value bits hi:lo, larger wins; then smaller pos); lanes
 // without a candidate have pos = kNone.  Returns the lane that holds it (a
 // lane without a candidate if all do).  Values are non-negative doubles,

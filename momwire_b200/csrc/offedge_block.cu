@@ -163,8 +163,7 @@ __device__ __forceinline__ void ob_samples(const double* xi, const double* xj, i
         const double dx = x0 - p[0], dy = x1 - p[1], dz = x2 - p[2];
         const double R2 = fma(dz, dz, fma(dy, dy, dx * dx)) + a2;
         *iR = rsqrt_pos(R2);
-        const double R = R2 * *iR;
-        return fma(0.5 * *iR, fma(-R, R, R2), R);  // Newton's step for the square root
+        return sqrt_pos(R2, *iR);
     };
     double iR, s, c;
     const double kR0 = __dmul_rn(k, distance(xi[0], xi[1], xi[2], 0, &iR));

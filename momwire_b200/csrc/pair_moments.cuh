@@ -128,6 +128,13 @@ __device__ __forceinline__ double rsqrt_pos(double x) {
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+// sqrt(x) from y = rsqrt_pos(x): x y and one step of Newton's iteration on its
+// residual, which is exact, so that the result is rounded (almost always) once.
+__device__ __forceinline__ double sqrt_pos(double x, double y) {
+    const double r = x * y;
+    return fma(0.5 * y, fma(-r, r, x), r);
+}
+
 struct Node {
     double x, y, z, w[3];
 };

@@ -1,3 +1,6 @@
+// mw_selftest_math: the kernels' own elementary functions on given arguments,
+// for a test to hold against the correctly rounded values.
+//
 // mw_selftest_wait_timeout: makes one of the library's bounded device waits
 // run out on purpose, with a short spin limit, so that a test can check
 // that the wait ends, records MW_ERR_TIMEOUT and leaves the context usable.
@@ -12,6 +15,7 @@
 //              cluster waiting for rows that neither sends.
 #include "common.cuh"
 #include "lu_cluster.cuh"
+#include "pair_moments.cuh"
 #include "tc_common.cuh"
 #include "waits.cuh"
 
@@ -34,8 +38,42 @@ __global__ void mbar_wait_selftest_kernel(int* err, long long limit) {
     __syncthreads();
 }
 
+__global__ void math_selftest_kernel(int which, int64_t n, const double2* in, double2* out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double2 x = in[i];
+    double a, b;
+    if (which == 0) {
+        a = rsqrt_pos(x.x);
+        b = sqrt_pos(x.x, a);
+    } else if (which == 1) {
+        const cd z = crecip(cd{x.x, x.y});
+        a = z.re;
+        b = z.im;
+    } else if (which == 2) {
+        phase_step<kPhaseModeShort>(x.x, &a, &b);
+    } else if (which == 3) {
+        phase_step<kPhaseModeLong>(x.x, &a, &b);
+    } else {
+        phase_step<kPhaseModeAny>(x.x, &a, &b);
+    }
+    out[i] = make_double2(a, b);
+}
+
 }  // namespace
 }  // namespace mw
+
+extern "C" mw_status mw_selftest_math(int32_t which, int64_t n, const double* in, double* out, void* stream) {
+    using namespace mw;
+    MW_REQUIRE(which >= 0 && which <= 4, "which must lie in [0, 4], got %d", which);
+    MW_REQUIRE(n >= 0 && n < (int64_t(1) << 31) && in && out, "bad arguments");
+    if (n == 0) return MW_OK;
+    math_selftest_kernel<<<(unsigned)((n + 127) / 128), 128, 0, as_stream(stream)>>>(
+        which, n, reinterpret_cast<const double2*>(in), reinterpret_cast<double2*>(out));
+    MW_CHECK_CUDA(cudaGetLastError());
+    count_launch();
+    return MW_OK;
+}
 
 extern "C" mw_status mw_selftest_wait_timeout(int32_t which, int64_t spin_limit, void* workspace, void* stream) {
     using namespace mw;
