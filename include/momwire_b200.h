@@ -383,7 +383,8 @@ mw_status mw_zgetrs(int64_t n, int64_t nrhs, const double* LU, int64_t lda,
  * its factors, ipiv and info as mw_zgetrf (info: 2 int32, info[1] a device
  * wait's MW_ERR_TIMEOUT, else 0), B (n x nrhs, leading dimension ldb) by X.
  * The right-hand sides ride through the factorisation, so only the back
- * substitution follows it.  Workspace: mw_getrf_workspace_size(n).
+ * substitution follows it.  A and B 16-byte aligned.  Workspace:
+ * mw_getrf_workspace_size(n).
  */
 mw_status mw_zgesv(int64_t n, int64_t nrhs, double* A, int64_t lda, int32_t* ipiv, int32_t* info,
                    double* B, int64_t ldb, void* workspace, size_t workspace_bytes,
@@ -392,7 +393,8 @@ mw_status mw_zgesv(int64_t n, int64_t nrhs, double* A, int64_t lda, int32_t* ipi
 /*
  * mw_zgesv on `batch` systems of one order: matrix b at A + 2 b a_stride,
  * its right-hand sides at B + 2 b b_stride (strides in complex elements),
- * its pivots at ipiv + b n, its two status words at info + 2 b.  Replaces
+ * its pivots at ipiv + b n, its two status words at info + 2 b; A and B
+ * 16-byte aligned.  Replaces
  * the stacked numpy.linalg.solve of a swept solve (bspline.py:4181-4440).
  * Workspace: mw_getrf_workspace_size(n).  Given `cancel`, systems that share
  * a launch (order 640; 1,696 from eight systems on) are launched as many at a

@@ -148,6 +148,32 @@ struct ProfileScope {
 // by Newton iteration on P_n (cached).  Returns pointers to host arrays.
 void gauss_legendre01(int n, const double** t, const double** w);
 
+// Whether p lies on a boundary of `bytes` (a power of two; null does).
+inline bool aligned_to(const void* p, uintptr_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+
+// A complex entry at p, as one access where the caller's array is aligned to
+// the pair (`wide`), else as two: the C interface takes arrays of double and
+// float at their own alignment.
+__device__ __forceinline__ double2 load_pair(const double* p, bool wide) {
+    return wide ? *reinterpret_cast<const double2*>(p) : make_double2(p[0], p[1]);
+}
+__device__ __forceinline__ void store_pair(double* p, bool wide, double x, double y) {
+    if (wide) {
+        *reinterpret_cast<double2*>(p) = make_double2(x, y);
+    } else {
+        p[0] = x;
+        p[1] = y;
+    }
+}
+__device__ __forceinline__ void store_pair(float* p, bool wide, float x, float y) {
+    if (wide) {
+        *reinterpret_cast<float2*>(p) = make_float2(x, y);
+    } else {
+        p[0] = x;
+        p[1] = y;
+    }
+}
+
 // Upper-triangle tile pair of block b: tc(tc+1)/2 <= b < (tc+1)(tc+2)/2,
 // tr = b - tc(tc+1)/2 <= tc.
 __device__ __forceinline__ void tri_pair(int64_t b, int& tr, int& tc) {

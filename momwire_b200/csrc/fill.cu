@@ -372,10 +372,10 @@ __device__ __forceinline__ bool fill_tile(const FillArgs& A, const GLParams& gl,
             if (same_edge) {
                 const int e = s_edge_r[li];
                 const int64_t row = A.e_off[e] + (s_pos_c[lj] - s_pos_r[li]) + A.e_n[e] - 1;
-                const double2* src = reinterpret_cast<const double2*>(table) + row * NMM;
+                const double* src = table + 2 * row * NMM;
 #pragma unroll
                 for (int x = 0; x < NMM; ++x) {
-                    const double2 v = src[x];
+                    const double2 v = load_pair(src + 2 * x, A.wide);
                     dst[x] = cd{v.x, v.y};
                 }
             }
@@ -413,14 +413,14 @@ __device__ __forceinline__ bool fill_tile(const FillArgs& A, const GLParams& gl,
     const double inv_weps = 1.0 / (omz * A.eps0);
     // into Z[m, n]: the value, or under a ground what the image term leaves
     auto put = [&](int64_t m, int64_t n, double zre, double zim) {
-        double2* zp = reinterpret_cast<double2*>(Zb + m * 2 + n * A.ldz * 2);
+        double* zp = Zb + m * 2 + n * A.ldz * 2;
         if (IMAGE) {
-            const double2 z = *zp;
+            const double2 z = load_pair(zp, A.wide);
             zre = z.x - zre;
             zim = z.y - zim;
         }
-        *zp = make_double2(zre, zim);
-        if (Z32b) *reinterpret_cast<float2*>(Z32b + m * 2 + n * A.ldz32 * 2) = make_float2((float)zre, (float)zim);
+        store_pair(zp, A.wide, zre, zim);
+        if (Z32b) store_pair(Z32b + m * 2 + n * A.ldz32 * 2, A.wide, (float)zre, (float)zim);
     };
     for (int n0 = 0; n0 < nb_c; n0 += kFillCols) {
         const int nc = min(kFillCols, nb_c - n0);
@@ -554,7 +554,8 @@ static double fill_flops(int D, int nq, double n_seg, double n_basis) {
 constexpr size_t kFillSmemSM = 227 * 1024;
 
 template <int D, bool IMAGE, bool EK>
-static mw_status launch_fill(const FillArgs& A, const GLParams& gl, cudaStream_t st) {
+static mw_status launch_fill(FillArgs A, const GLParams& gl, cudaStream_t st) {
+    A.wide = aligned_to(A.Z, 16) && aligned_to(A.table, 16) && aligned_to(A.Z32, 8);
     // A single system with a complex64 copy is about to be solved through
     // complex64 factors.  Single coefficients of a large one follow the
     // copy's roundings to 6e-8 (16 x 16 array, 10,496 unknowns), and this

@@ -31,6 +31,7 @@ struct FillArgs {
     const double* omegab;
     int64_t table_stride, z_stride, z32_stride;
     int nbatch;
+    bool wide;  // table, Z and Z32 are aligned to their complex entries
 };
 
 // Z and its complex64 copy for one frequency, each sum in a fixed order

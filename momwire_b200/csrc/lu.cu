@@ -1331,7 +1331,9 @@ mw_status zgemm_launch(bool ta, bool tb, int64_t m, int64_t n, int64_t k, cd alp
                        const cd* B, int64_t ldb, cd beta, cd* C, int64_t ldc, cudaStream_t st, int max_ctas,
                        void* split_ws, size_t split_ws_bytes) {
     if (m <= 0 || n <= 0) return MW_OK;
-    if (k < 128) return zgemm_launch_simt(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st);
+    // (the DMMA kernel's copies take 16 bytes at a time)
+    if (k < 128 || !aligned_to(A, 16) || !aligned_to(B, 16))
+        return zgemm_launch_simt(ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st);
     if (k <= kDmShortK && !split_ws) {
         if (!ta) return tb ? dmma_launch<false, true, 64>(m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, st, max_ctas,
                                                           nullptr, 0)
@@ -2307,7 +2309,10 @@ static mw_status zgetrf_any(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_
         set_error("factorisation cancelled");
         return MW_ERR_CANCELLED;
     }
-    if (n <= zlu_full_max()) {
+    // (the cluster kernels take 16 bytes at a time; the cooperative panels do
+    // not)
+    const bool wide = aligned_to(A, 16);
+    if (wide && n <= zlu_full_max()) {
         MW_CHECK_CUDA(cudaMemsetAsync(info, 0, 2 * sizeof(int32_t), st));
         if (n == 0) return MW_OK;
         const bool in_kernel = back && nrhs <= 64;  // (beyond, the block solves' products win)
@@ -2325,7 +2330,7 @@ static mw_status zgetrf_any(int64_t n, cd* A, int64_t lda, int32_t* ipiv, int32_
         if (s != MW_OK || in_kernel || !back || nrhs == 0) return s;
         return zlu_upper(n, A, lda, B, ldb, nrhs, st);
     }
-    if (n <= zlu_cluster_max_rows()) {
+    if (wide && n <= zlu_cluster_max_rows()) {
         MW_CHECK_CUDA(cudaMemsetAsync(info, 0, 2 * sizeof(int32_t), st));
         mw_status s = zlu_blocked(n, A, lda, ipiv, info, B, ldb, nrhs,
                                   reinterpret_cast<int32_t*>(static_cast<char*>(workspace) + panel_ws_bytes()), cancel,
@@ -2357,6 +2362,7 @@ extern "C" mw_status mw_zgesv(int64_t n, int64_t nrhs, double* Ad, int64_t lda, 
                               const volatile int32_t* cancel, void* stream) {
     MW_REQUIRE(n >= 0 && nrhs >= 0 && lda >= (n > 0 ? n : 1) && ldb >= (n > 0 ? n : 1), "bad sizes");
     MW_REQUIRE(Ad && ipiv && info && workspace && (nrhs == 0 || Bd), "NULL argument");
+    MW_REQUIRE(aligned_to(Ad, 16) && aligned_to(Bd, 16), "A and B must be 16-byte aligned");
     MW_REQUIRE(workspace_bytes >= mw_getrf_workspace_size(n), "workspace too small");
     ProfileScope ps(PC_FACTOR, as_stream(stream), 8.0 / 3.0 * (double)n * n * n + 8.0 * (double)n * n * nrhs, 0.0);
     return zgetrf_any(n, reinterpret_cast<cd*>(Ad), lda, ipiv, info, workspace, reinterpret_cast<cd*>(Bd), ldb, nrhs,
@@ -2377,6 +2383,7 @@ extern "C" mw_status mw_zgesv_batched(int64_t n, int64_t nrhs, int32_t batch, do
     MW_REQUIRE(n >= 1 && nrhs >= 1 && batch >= 1 && lda >= n && ldb >= n, "bad sizes");
     MW_REQUIRE(a_stride >= lda * n && b_stride >= ldb * nrhs, "strides overlap");
     MW_REQUIRE(Ad && ipiv && info && Bd && workspace, "NULL argument");
+    MW_REQUIRE(aligned_to(Ad, 16) && aligned_to(Bd, 16), "A and B must be 16-byte aligned");
     MW_REQUIRE(workspace_bytes >= mw_getrf_workspace_size(n), "workspace too small");
     cudaStream_t st = as_stream(stream);
     cd* A = reinterpret_cast<cd*>(Ad);

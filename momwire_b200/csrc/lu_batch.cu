@@ -381,7 +381,7 @@ constexpr int kGsAhead = 32;  // entries of a row in registers ahead of time
 constexpr size_t kGsSmemMax = 200 * 1024;
 template <int C>
 __global__ void __launch_bounds__(kGsThreads, 2) getrs_batched_kernel(const cf* LU, int64_t lda, int64_t stride, int n,
-                                                                      const int32_t* ipiv, cf* B, int nr) {
+                                                                      const int32_t* ipiv, cf* B, int nr, bool wide) {
     extern __shared__ __align__(16) unsigned char gs_smem[];
     cf* sT = reinterpret_cast<cf*>(gs_smem);  // [2][64][64], sT[k * 64 + i] = T(i, k)
     cf* sX = sT + 2 * kBSB * kBSB;            // [C][n]
@@ -399,10 +399,15 @@ __global__ void __launch_bounds__(kGsThreads, 2) getrs_batched_kernel(const cf* 
         const cf* src = LU + j0 + (int64_t)j0 * lda;
         for (int q = tid; q < kBSB * kBSB; q += kGsThreads) {
             const int i = q % kBSB, k = q / kBSB;
-            if (i < jb && k < jb)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * q),
-                             "l"(src + i + (int64_t)k * lda)
+            if (i >= jb || k >= jb) continue;
+            const cf* from = src + i + (int64_t)k * lda;
+            if (wide) {
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + 8u * q), "l"(from) : "memory");
+            } else {  // factors aligned to their floats only
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 8u * q), "l"(&from->re) : "memory");
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 8u * q + 4u), "l"(&from->im)
                              : "memory");
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -710,7 +715,7 @@ static mw_status getrs_launch(int n, int nr, int batch, const cf* LU, int64_t ld
     }
     const size_t smem = sizeof(cf) * ((size_t)2 * kBSB * kBSB + (size_t)C * n);
     getrs_batched_kernel<C><<<dim3((unsigned)((nr + C - 1) / C), (unsigned)batch), kGsThreads, smem, st>>>(
-        LU, lda, stride, n, ipiv, B, nr);
+        LU, lda, stride, n, ipiv, B, nr, aligned_to(LU, 8));
     count_launch();
     MW_CHECK_CUDA(cudaGetLastError());
     return MW_OK;

@@ -67,6 +67,7 @@ struct ObArgs {
     double a_ek;  // > 0: extended kernel on eligible pairs
     double* Z;
     int64_t ldz;
+    bool wide;  // Z is aligned to its complex entries
 };
 
 // Lists of a CTA, then (in the kernel) what depends on the rule's order.
@@ -369,8 +370,8 @@ __global__ void __launch_bounds__(kObThreads, 3) offedge_block_kernel(ObArgs A) 
             for (int h = 0; h < 2; ++h) {
                 const int e = tid + h * kObThreads, m = e / kObTile, n = e % kObTile;  // the column basis fastest
                 if (m >= nm || n >= nn) continue;
-                double2* out = reinterpret_cast<double2*>(A.Z + 2 * ((int64_t)(m0 + m) * A.ldz + n0 + n));
-                *out = make_double2(-om_mu * zA[h].im + zP[h].im * inv_om_eps, om_mu * zA[h].re - zP[h].re * inv_om_eps);
+                store_pair(A.Z + 2 * ((int64_t)(m0 + m) * A.ldz + n0 + n), A.wide,
+                           -om_mu * zA[h].im + zP[h].im * inv_om_eps, om_mu * zA[h].re - zP[h].re * inv_om_eps);
             }
         }
     }
@@ -442,6 +443,7 @@ extern "C" mw_status mw_offedge_block(int32_t degree, const mw_block_side* I, co
     A.a_ek = a_ek;
     A.Z = Z;
     A.ldz = ldz;
+    A.wide = aligned_to(Z, 16);
     MW_REQUIRE((int64_t)A.nI * A.nJ / 8 < (1ll << 31), "block too large");
     const bool ek = a_ek > 0.0 && A.I.group != nullptr && A.J.group != nullptr;
     cudaStream_t st = as_stream(stream);

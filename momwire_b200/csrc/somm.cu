@@ -130,6 +130,7 @@ struct QArgs {
     int64_t ldz;
     float* Z32;
     int64_t ldz32;
+    bool wide;  // Z and Z32 are aligned to their complex entries
 };
 
 // per staged segment: nq nodes (3 each), W[p][q] ((d+1) x nq), tangent (3),
@@ -300,11 +301,11 @@ __global__ void __launch_bounds__(kQThreads, 2) somm_q_kernel(QArgs A) {
     }
     __syncthreads();
     auto subtract = [&](int64_t m, int64_t n, cd Q) {
-        double2* zp = reinterpret_cast<double2*>(A.Z + 2 * (m + n * A.ldz));
-        const double2 z = *zp;
+        double* zp = A.Z + 2 * (m + n * A.ldz);
+        const double2 z = load_pair(zp, A.wide);
         const double zr = z.x - Q.re, zi = z.y - Q.im;
-        *zp = make_double2(zr, zi);
-        if (A.Z32) *reinterpret_cast<float2*>(A.Z32 + 2 * (m + n * A.ldz32)) = make_float2((float)zr, (float)zi);
+        store_pair(zp, A.wide, zr, zi);
+        if (A.Z32) store_pair(A.Z32 + 2 * (m + n * A.ldz32), A.wide, (float)zr, (float)zi);
     };
     for (int pp = tid; pp < TB * TB; pp += kQThreads) {
         const int mi = pp % TB, ni = pp / TB;
@@ -477,6 +478,7 @@ extern "C" mw_status mw_somm_remainder_q(const mw_segments* seg, const mw_basis*
     A.ldz = ldz;
     A.Z32 = Z32;
     A.ldz32 = ldz32;
+    A.wide = aligned_to(Z, 16) && aligned_to(Z32, 8);
     const int d = basis->degree;
     const int smax = basis->max_tile_seg, tb = basis->max_tile_basis;
     const size_t smem = d == 1 ? QSmem<1>(n_qp, smax, tb).bytes : QSmem<2>(n_qp, smax, tb).bytes;
