@@ -627,10 +627,11 @@ class BSplineSolver:
 
     def _port_plan(self) -> _PortPlan:
         """The packed port tables, built again only when the ports have
-        changed: they depend on the geometry and on these settings, not on
+        changed: they depend on the geometry and on these settings (the
+        ground's height among them: a port must not be grounded), not on
         the frequency, and building them took longer than a small solve."""
         key = (tuple(map(tuple, self.feeds)), self.feed_model, self.feed_smoothing_factor, self.n_qp_source,
-               tuple(map(tuple, self.junction_ports)), tuple(map(tuple, self.node_gaps)))
+               tuple(map(tuple, self.junction_ports)), tuple(map(tuple, self.node_gaps)), self.ground_z)
         if self._cached_ports is None or self._cached_ports[0] != key:
             self._cached_ports = (key, _PortPlan(self))
         return self._cached_ports[1]
