@@ -52,9 +52,10 @@ def read_back(torch, stream, tensors):
 
 class _Bounce(threading.local):
     """Two page-locked slots and their events, per host thread and given back
-    with it."""
+    with it.  21 MB took 711 us through slots of 2 MB, 715 of 4, 599 of 8, 594
+    of 16 (390 to page-locked memory): a slice costs 30 us beside its copies."""
 
-    SLOT = 4 << 20  # bytes
+    SLOT = 8 << 20  # bytes
     slots = events = None
 
     def get(self, torch):
@@ -72,19 +73,29 @@ class _Bounce(threading.local):
 
 
 _bounce = _Bounce()
+_SMALL = 1 << 17  # bytes: up to here one thread copies as fast as several (960 KB: 234 us a call against 176)
+_NUMPY = {"torch.complex128": np.complex128, "torch.complex64": np.complex64, "torch.float64": np.float64,
+          "torch.float32": np.float32, "torch.int32": np.int32}
 
 
 def to_host(torch, stream, t):
     """An ordinary array with a contiguous device tensor's values: slice by
     slice through the thread's page-locked slots, one on its way from the
-    device while the other is copied out."""
-    out = np.empty(tuple(t.shape), dtype=torch.empty(0, dtype=t.dtype).numpy().dtype)
+    device while the other is copied out (a small result, a row of a block
+    say, in one piece)."""
+    out = np.empty(tuple(t.shape), dtype=_NUMPY[str(t.dtype)])
     if out.size == 0:
         return out
     slots, S = _bounce.get(torch), _bounce.SLOT
     with torch.inference_mode():  # (no version counters, no autograd)
-        src, dst = t.view(-1).view(torch.uint8), torch.from_numpy(out.reshape(-1).view(np.uint8))
-        n = dst.numel()
+        src, n = t.view(-1).view(torch.uint8), out.nbytes
+        dst = out.reshape(-1).view(np.uint8)
+        if n <= _SMALL:
+            slots[0][:n].copy_(src, non_blocking=True)
+            stream.synchronize()
+            dst[:] = slots[0].numpy()[:n]
+            return out
+        dst = torch.from_numpy(dst)
         cuts = [(o, min(o + S, n)) for o in range(0, n, S)]
 
         def fetch(i):

@@ -10,11 +10,11 @@ complex128 result, computed by ``mw_offedge_block`` on the current CUDA
 device, so a maintainer can route those calls here (INTEGRATION.md shows
 how).  Inputs are host arrays, as the reference takes them; they are
 uploaded in one copy, the block is filled on the device and comes back as an
-ordinary array, through a page-locked buffer of 8 MB per host thread: an
+ordinary array, through page-locked buffers of 16 MB per host thread: an
 H-matrix host keeps its blocks, and page-locked results would lock all of
 its compressed matrix (and a new page-locked 21 MB costs 15 ms).
 A 1025 x 1311 block measured 5.6 ms through pageable copies, most of it the
-21 MB on their way back, and 1.1 ms so, 2.5 with every block kept.
+21 MB on their way back, and 1.0 ms so, 1.9 with every block kept.
 """
 
 from __future__ import annotations

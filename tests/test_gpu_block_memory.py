@@ -35,13 +35,13 @@ def test_blocks_are_ordinary_arrays(cuda_device):
     assert np.array_equal(_block(a), kept)
 
 
-@pytest.mark.parametrize("count", [0, 1, (1 << 18) - 1, 1 << 18, (1 << 18) + 1, (2 << 18) + 7, 5 << 18])
-def test_sizes_around_the_slots(count, cuda_device):
+@pytest.mark.parametrize("slots,more", [(0, 0), (0, 1), (0, 1 << 13), (0, (1 << 13) + 1), (1, -1), (1, 0), (1, 1), (2, 7), (5, 0)])
+def test_sizes_around_the_slots(slots, more, cuda_device):
     import torch
 
     from momwire_b200 import _staging
 
-    assert _staging._Bounce.SLOT == 16 << 18
+    count = slots * _staging._Bounce.SLOT // 16 + more
     x = torch.randn(count, dtype=torch.complex128, device=cuda_device)
     got = _staging.to_host(torch, torch.cuda.current_stream(cuda_device), x)
     assert got.dtype == np.complex128 and np.array_equal(got, x.cpu().numpy())
@@ -58,7 +58,7 @@ def test_threads_do_not_share_slots(cuda_device):
         stream = torch.cuda.Stream(cuda_device)
         with torch.cuda.stream(stream):
             for i in range(8):
-                x = torch.full((300_000 + 1000 * seed,), float(100 * seed + i), dtype=torch.float64, device=cuda_device)
+                x = torch.full((1_200_000 + 1000 * seed,), float(100 * seed + i), dtype=torch.float64, device=cuda_device)
                 if not np.all(_staging.to_host(torch, stream, x) == 100 * seed + i):
                     bad.append(seed)
 
