@@ -41,9 +41,9 @@ WORKLOAD = "dipole_array_16x16_300MHz_41seg_d2_256port"
 # algorithmic byte of the tensor-core update (C read and written plus the
 # hi / lo operand planes), measured on three consecutive launches of the
 # 12x12 array's factorisation (a next-block, a trailing and a right-hand-side
-# update of one panel: 158.8 MB against 219.3 MB); the bench line scales it
+# update of one panel: 159.3 MB against 219.3 MB); the bench line scales it
 # by the step's algorithmic bytes per launch
-TC_TRAFFIC_PER_ALG_BYTE = 158.8 / 219.3
+TC_TRAFFIC_PER_ALG_BYTE = 159.3 / 219.3
 
 
 def parse():

@@ -14,7 +14,7 @@ ordinary array, through page-locked buffers of 16 MB per host thread: an
 H-matrix host keeps its blocks, and page-locked results would lock all of
 its compressed matrix (and a new page-locked 21 MB costs 15 ms).
 A 1025 x 1311 block measured 5.6 ms through pageable copies, most of it the
-21 MB on their way back, and 1.0 ms so, 1.9 with every block kept.
+21 MB on their way back, and 0.95 ms so, 2.2 with every block kept.
 """
 
 from __future__ import annotations

@@ -459,7 +459,8 @@ __device__ __forceinline__ bool fill_tile(const FillArgs& A, const GLParams& gl,
             // j w mu zA + zP / (j w eps)
             const double zre = -wmu * zA.im + inv_weps * zP.im, zim = wmu * zA.re - inv_weps * zP.re;
             put(fb_r + mi, fb_c + n0 + nl, zre, zim);
-            // the transposed block: 128-byte runs of the column bases
+            // the transposed block: a warp holds two column bases, so 32-byte
+            // pieces of sixteen columns of Z, which L2 puts together
             if (mirror) put(fb_c + n0 + nl, fb_r + mi, zre, zim);
         }
         if (n0 + kFillCols < nb_c) __syncthreads();

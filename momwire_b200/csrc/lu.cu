@@ -2230,7 +2230,11 @@ static mw_status getrs(int64_t n, int64_t nrhs, const T* LU, int64_t lda, const 
 // 1.60 ms at 641 by blocks.
 static int64_t zlu_full_max() { return 640; }
 // A batch fills the device with clusters up to the order its back
-// substitution holds; a few matrices alone follow the rule of one.
+// substitution holds; a few matrices alone follow the rule of one.  Measured
+// on B200 with 4 right-hand sides, one launch against one system after the
+// other: 2.7 against 12.6 ms for 8 systems of 650, 5.9 / 20.1 for 8 of 1,000,
+// 10.1 / 27.5 for 8 of 1,300, 18.8 / 37.6 for 8 of 1,696, 224 / 942 for 200
+// of 1,696.
 static int64_t zlu_batch_max(int32_t batch) { return batch >= 8 ? 1696 : zlu_full_max(); }
 
 static size_t panel_ws_bytes() {

@@ -31,10 +31,12 @@
 // reciprocal root, were off by 1.1e-13 of the block's norm (1025 x 1311,
 // degree 2) and 1.7e-13 (103 x 150, degree 1); this is off by 3.4e-14 and
 // 2.5e-14, as a warp per entry was.
-// What bounds it is the FP64 pipe.  Measured on B200, a 1025 x 1311 block at
-// degree 2: 4.83 ms with one warp per entry, which evaluated every segment
-// pair's samples up to nine times, 0.25 ms now (0.24 with moments).  Output
-// row-major, Z[m * ldz + n], like the reference's (nI, nJ) array.
+// What bounds it is latency: the samples' dependent FP64 operations and the two
+// barriers of a stripe, with twelve warps an SM (issue 45 %, FP64 pipe 36 %).
+// Measured on B200, a 1025 x 1311 block at degree 2: 4.83 ms with one warp per
+// entry, which evaluated every segment pair's samples up to nine times, 0.25
+// ms now (0.24 with moments).  Output row-major, Z[m * ldz + n], like the
+// reference's (nI, nJ) array.
 #include "common.cuh"
 #include "ground_weights.cuh"
 #include "pair_moments.cuh"

@@ -24,8 +24,10 @@
 // polynomials in two stages (source side, observer side) and Q subtracted
 // from Z (and its complex64 copy).  The grid tables are read through the
 // read-only cache: a node's four surfaces are one 64-byte line.  What bounds
-// it is the field evaluation (square roots, an arc tangent, sine and cosine,
-// 64 grid loads).  One thread per segment pair and every ordered tile pair
+// it is the latency of the field evaluation (square roots, an arc tangent, sine
+// and cosine, 64 grid loads: the FP64 pipe at 22 %), with one block an SM at
+// the usual order 3 on 18-segment tiles (118 KB; two where a tile is smaller or
+// the order 2).  One thread per segment pair and every ordered tile pair
 // left three quarters of the threads idle on short wires: the remainder of a
 // 20-cell plate (1,690 segments) took 6.55 ms on B200, 1.1 ms now.
 #include <vector>
