@@ -88,3 +88,19 @@ def test_nodes_off_the_segments(lo, hi, cuda_device):
     got = accel.bspline_assemble_offedge_block(*args, 2, t, 0.5 * w)
     want = BO.offedge_block(*args, t, 0.5 * w, group=None, a_ek=0.0, refl=None)
     assert rel_err(got, want) < 1e-12
+
+
+@pytest.mark.parametrize("n_i,n_j,degree,nq,scattered", [(20, 33, 2, 2, False), (33, 20, 2, 5, False), (18, 35, 1, 6, True),
+                                                         (35, 17, 2, 7, True), (4, 60, 1, 5, False)])
+def test_every_order_of_the_rule(n_i, n_j, degree, nq, scattered, cuda_device):
+    """Stripes of eight observer segments to order 4, of four beyond, with as
+    many as the pairs of a round allow.  Tolerance as for the tiles."""
+    rng = np.random.default_rng(nq)
+    I, J = _side(rng, n_i, degree, 6.0, scattered), _side(rng, n_j, degree, 1.0, scattered)
+    t, w = np.polynomial.legendre.leggauss(nq)
+    t, w = 0.5 * (t + 1.0), 0.5 * w
+    k = 2.0
+    args = (*I[:5], *J[:5], 1e-5, k, k * 3e8, 8.85e-12, 1.2566e-6)
+    got = accel.bspline_assemble_offedge_block_ek(*args, degree, t, w, I[5], J[5], 2e-3)
+    want = BO.offedge_block(*args, t, w, group=(I[5], J[5]), a_ek=2e-3, refl=None)
+    assert rel_err(got, want) < 1e-12
